@@ -75,6 +75,18 @@ __device__ __forceinline__ uint32_t atom_add_acq_rel_cta(uint32_t* p, uint32_t v
   return old;
 }
 
+// ---- programmatic dependent launch
+// Lets the next kernel of the stream start its CTAs while this one runs; it waits in
+// grid_dependency_wait before it touches anything this one reads or writes.
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Waits until the kernels this one depends on have finished and their writes are visible (at
+// once for a kernel launched without the attribute).
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---- ordering between CTAs of one grid (gpu scope)
 // Counter add with acquire-release semantics at gpu scope. Returns the previous value.
 __device__ __forceinline__ uint32_t atom_add_acq_rel_gpu(uint32_t* p, uint32_t v) {

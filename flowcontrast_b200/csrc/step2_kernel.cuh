@@ -600,6 +600,8 @@ __global__ void __launch_bounds__(Step2Tile<D1, TY, TE>::THREADS, TY == 16 ? 2 :
                        const __grid_constant__ CUtensorMap tmap_uvw, const Step2Geom g,
                        const StepConst<float> k) {
   extern __shared__ __align__(128) unsigned char smem[];
+  grid_launch_dependents();
+  grid_dependency_wait();
   if (threadIdx.x == 0 && blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
   // centre pairs carried for FP32 storage (FP16 storage measured 3 % slower with them)
   step2_march<D1, TY, PK, TE, std::is_same<TE, float>::value>(&tmap_p, &tmap_uvw, g, k, blockIdx.x % g.ntiles,

@@ -104,6 +104,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(TS) == 8 ? 1 : 2)
   const int zb = chunk * g.chunk, ze = min(zb + g.chunk, g.L);
   const int t0 = zb - R, t1 = ze + R;
 
+  grid_launch_dependents();
+  grid_dependency_wait();
   if (tid == 0) {
     if (blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
     for (int s = 0; s < S; ++s) mbar_init(&bar[s], 1);
