@@ -204,9 +204,9 @@ struct fslbm_solve {
   CUtensorMap maps[2];
   // FP32 column-pair kernel (even d1): tile height, persistent grid, two maps per buffer
   bool use2 = false;
-  int ty2 = 32, grid2 = 0, packed2 = 1;
+  int ty2 = 32, grid2 = 0;
   std::vector<int> tile_warps[3];  // per column-pair tile: warps holding fluid, [shape] 32 x 2, 16 x 4, 8 x 8
-  CUtensorMap maps2p[2], maps2u[2];
+  CUtensorMap maps2p[2], maps2u[2], maps2o[2];
   DevCounters* d_counters = nullptr;
   fslbm_monitor* d_log = nullptr;
   int log_cap = 4096;
@@ -269,7 +269,7 @@ static int validate_params(const fslbm_params* p, int dtype) {
 }
 
 // Tensor maps of the column-pair kernel with tile height ty over the solve's two state buffers:
-// the p box (one-cell halo) and the u,v,w box (the corrector's halo).
+// the p box (one-cell halo) and the u,v,w box (the corrector's halo) of the loads.
 static int encode_pair_maps(const fslbm_solve* s, int ty, CUtensorMap mp[2], CUtensorMap mu[2]) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return fslbm_set_error(FSLBM_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
@@ -299,8 +299,32 @@ static int encode_pair_maps(const fslbm_solve* s, int ty, CUtensorMap mp[2], CUt
   return FSLBM_OK;
 }
 
+// Tensor maps of the column-pair kernel's stores into the two state buffers: the four fields of
+// one warp's cells in warp shape `shape` (32 x 2, 16 x 4 or 8 x 8).
+static int encode_store_maps(const fslbm_solve* s, int shape, CUtensorMap mo[2]) {
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return fslbm_set_error(FSLBM_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
+  const CUtensorMapDataType dt = s->dtype == FSLBM_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  cuuint64_t dims[4] = {cuuint64_t(s->lxp), cuuint64_t(s->ly), cuuint64_t(s->L), 4};
+  cuuint64_t strides[3] = {cuuint64_t(s->lxp) * s->es, cuuint64_t(s->lxp) * s->ly * s->es,
+                           cuuint64_t(field_stride(s)) * s->es};
+  cuuint32_t estr[4] = {1, 1, 1, 1}, box[4] = {cuuint32_t(32 >> shape), cuuint32_t(2 << shape), 1, 4};
+  for (int b = 0; b < 2; ++b) {
+    const CUresult r = enc(&mo[b], dt, 4, s->state[b], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+      return fslbm_set_error(FSLBM_ERR_CUDA, "cuTensorMapEncodeTiled (pair kernel store) failed (%d)", int(r));
+  }
+  return FSLBM_OK;
+}
+
 static int build_tensor_maps(fslbm_solve* s) {
-  if (s->use2) return encode_pair_maps(s, s->ty2, s->maps2p, s->maps2u);
+  if (s->use2) {
+    if (s->dtype != FSLBM_F64)
+      if (int r = encode_store_maps(s, 0, s->maps2o)) return r;
+    return encode_pair_maps(s, s->ty2, s->maps2p, s->maps2u);
+  }
   EncodeTiledFn enc = encode_fn();
   if (!enc) return fslbm_set_error(FSLBM_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
   const CUtensorMapDataType dt = s->dtype == FSLBM_F64   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
@@ -362,9 +386,55 @@ static void tile_warp_counts(const fslbm_solve* s, const std::vector<int2>& tile
 
 static void choose_chunks(fslbm_solve* s);
 
+// How a solve's step is split over the SMs: tile height and streamwise chunks.
+struct Split {
+  int ty = 0, nch = 0;
+  double us = 1e300;               // modelled time of one step
+  std::vector<int2> tiles;
+};
+
+// Modelled time of one step of `ntiles` tiles of 32 x ty cells in nch chunks, with `per_sm` CTAs
+// resident per SM: each wave of CTAs costs a launch and pipeline fill and then a time per march
+// iteration, measured on B200 (circular pipes from 32 x 24 x 24 to 512 x 128 x 128, every split).
+// FP32 and FP16 storage march two planes per iteration, two iterations before the first output;
+// FP64 one plane, and its eight planes of fill cost as much as 4.8 output planes. An SM's time per
+// iteration grows with its resident warps (32 x 8 tiles have 4, 32 x 16 have 8, 32 x 32 have 16):
+// 1.35 us for one 32 x 8 tile of FP32 against 2.85 us for a 32 x 32 tile, so few cells per SM want
+// small tiles (latency) and many cells the large one (fewer halo cells, more warps).
+static double split_us(int dtype, int ty, int per_sm, int sms, int L, int ntiles, int nch) {
+  static const double f32[3][3] = {{1.35, 1.8, 2.45}, {1.7, 0, 0}, {2.85, 0, 0}};
+  static const double f16[3][3] = {{1.93, 2.37, 3.2}, {2.45, 4.05, 0}, {3.94, 0, 0}};
+  const int planes = (L + nch - 1) / nch;
+  const int64_t ctas = int64_t(ntiles) * nch, waves = (ctas + int64_t(sms) * per_sm - 1) / (int64_t(sms) * per_sm);
+  if (dtype == FSLBM_F64) return double(waves) * 1.3 * (planes + 4.8);
+  const double tau = (dtype == FSLBM_F16 ? f16 : f32)[ty == 8 ? 0 : (ty == 16 ? 1 : 2)][per_sm - 1];
+  return double(waves) * (2.0 + tau * ((planes + 1) / 2 + 2));
+}
+
+// The split with the least modelled time over the tile heights of the solve's kernel (or
+// `only_ty`), CTAs per SM and one to four waves of CTAs.
+static Split choose_split(const fslbm_solve* s, int only_ty) {
+  Split best;
+  const int sms = s->ctx->sm_count, max_nch = s->dtype == FSLBM_F64 ? s->L : (s->L + 1) / 2;
+  for (int ty : {32, 16, 8}) {
+    int box[5];
+    if ((only_ty && ty != only_ty) || !step2_box(s->dtype, s->prm.d1, ty, box, box + 1, box + 2, box + 3, box + 4))
+      continue;
+    const std::vector<int2> tiles = fluid_tiles(s, ty);
+    const int nt = int(tiles.size());
+    for (int per_sm = 1; per_sm <= step2_occupancy(s->dtype, s->prm.d1, ty); ++per_sm)
+      for (int waves = 1; waves <= 4; ++waves) {
+        const int nch = std::max(1, std::min(int(int64_t(sms) * per_sm * waves / nt), max_nch));
+        const double us = split_us(s->dtype, ty, per_sm, sms, s->L, nt, nch);
+        if (us < best.us) best = Split{ty, nch, us, tiles};
+      }
+  }
+  return best;
+}
+
 // Selects the step kernel for the current dtype and d1, uploads its tile list, builds its
 // tensor maps and sizes its grid. FSLBM_STEP_KERNEL=1 forces the one-column kernel and
-// FSLBM_PACKED=0 uses scalar pair arithmetic and FSLBM_TILE_Y=16|32 picks the column-pair kernel's tile height (for comparisons).
+// FSLBM_TILE_Y=8|16|32 picks the column-pair kernel's tile height (for comparisons).
 static int configure_kernel(fslbm_solve* s) {
   const char* ek = std::getenv("FSLBM_STEP_KERNEL");
   const char* et = std::getenv("FSLBM_TILE_Y");
@@ -373,11 +443,12 @@ static int configure_kernel(fslbm_solve* s) {
   // FP16 storage exists only in the column-pair kernel, which has the 2-tap corrector
   s->use2 = step2_supported(s->dtype, s->prm.d1) && s->K == 2 && s->planes == 1 &&
             (s->dtype == FSLBM_F16 || !(ek && std::atoi(ek) == 1));
-  // FP64 runs the column kernel on 32 x 16 tiles
-  s->ty2 = (s->dtype == FSLBM_F64 || (et && std::atoi(et) == 16)) ? 16 : 32;
-  const char* ep = std::getenv("FSLBM_PACKED");
-  s->packed2 = (ep && std::atoi(ep) == 0) ? 0 : 1;
-  const std::vector<int2> tiles = fluid_tiles(s, s->use2 ? s->ty2 : kTY);
+  const int ety = et && s->dtype != FSLBM_F64 ? std::atoi(et) : 0;
+  Split split;
+  if (s->use2) split = choose_split(s, ety == 8 || ety == 16 || ety == 32 ? ety : 0);
+  else split.tiles = fluid_tiles(s, kTY);
+  const std::vector<int2>& tiles = split.tiles;
+  s->ty2 = split.ty;
   for (auto& v : s->tile_warps) v.clear();
   if (s->use2) tile_warp_counts(s, tiles, s->ty2, s->tile_warps);
   if (s->d_tiles) {
@@ -392,13 +463,7 @@ static int configure_kernel(fslbm_solve* s) {
                            cudaMemcpyHostToDevice, s->ctx->stream));
   if (s->use2) {
     CUDA_TRY(step2_prepare(s->dtype, s->prm.d1, s->ty2));
-    // tiles x streamwise chunks, at most one CTA per SM slot and chunks of at least 2R planes
-    // (chunk counts weighted by each tile's fluid warps measured no faster: a tile with wall in
-    // it is not proportionally faster per plane)
-    const int slots = s->ctx->sm_count * step2_occupancy(s->dtype, s->prm.d1, s->ty2);
-    int nch = std::max(1, slots / s->ntiles);
-    nch = std::min(nch, std::max(1, s->L / (4 * s->prm.d1)));
-    s->grid2 = s->ntiles * nch;
+    s->grid2 = s->ntiles * split.nch;
   } else {
     CUDA_TRY(step_prepare(s->dtype, s->prm.d1, s->K));
     choose_chunks(s);
@@ -942,7 +1007,7 @@ static int enqueue_steps(fslbm_solve* s, int64_t nsteps) {
       CUDA_TRY(cudaEventRecord(s->tev[s->tev_used], st));
     }
     if (s->use2) {
-      Step2Launch b2{s->prm.d1, s->ty2, s->packed2, &s->maps2p[s->cur], &s->maps2u[s->cur], s->grid2};
+      Step2Launch b2{s->prm.d1, s->ty2, &s->maps2p[s->cur], &s->maps2u[s->cur], &s->maps2o[1 - s->cur], s->grid2};
       CUDA_TRY(launch_step2(a, b2, st));
     } else {
       CUDA_TRY(launch_step(a, st));
@@ -1299,17 +1364,18 @@ struct fslbm_batch {
   std::vector<BatchMon> h_mons;
   std::vector<int2> h_items;
   std::vector<int2> item_shape;    // per member: (tiles, chunks) the item table was built for
-  int nitems = 0, grid = 0, packed = 1;
+  int nitems = 0, grid = 0;
   // the batch's own column-pair tiling of every member (32 x ty tiles, one height for the whole
   // batch): tile list, fluid warps per tile for the two warp shapes, tensor maps of both buffers.
   // 32 x 16 tiles, two 256-thread CTAs per SM: on the 64-pipe ensemble (cross-sections 24..96)
   // +1.0 % against 32 x 32 tiles; the members' own single-pipe tiling is not affected
-  int ty = 16;
+  int ty = 32;
   struct Tiling {
     int ntiles = 0;
     int2* d_tiles = nullptr;
     std::vector<int> warps[3];
-    CUtensorMap mp[2], mu[2];
+    CUtensorMap mp[2], mu[2], mo[2];
+    int mo_shape = -1;               // warp shape mo was built for
   };
   std::vector<Tiling> mt;
   // per member tiling: streamwise planes per work item and warp shape (0: 32 x 2, 1: 16 x 4,
@@ -1399,7 +1465,11 @@ static int batch_upload(fslbm_batch* b) {
   }
   for (int i = 0; i < n; ++i) {
     fslbm_solve* s = b->members[i];
-    const fslbm_batch::Tiling& tl = b->mt[i];
+    fslbm_batch::Tiling& tl = b->mt[i];
+    if (tl.mo_shape != b->m_shape[i]) {
+      if (int r = encode_store_maps(s, b->m_shape[i], tl.mo)) return r;
+      tl.mo_shape = b->m_shape[i];
+    }
     StepLaunch a{};
     a.dtype = s->dtype; a.d1 = s->prm.d1;
     a.lxp = s->lxp; a.ly = s->ly; a.L = s->L; a.ntiles = tl.ntiles;
@@ -1409,7 +1479,7 @@ static int batch_upload(fslbm_batch* b) {
     fill_constants(s, a);
     const int nch = member_chunks(s, eff_chunk(i));
     const long long stop_at = b->stop[i] >= 0 ? (long long)b->stop[i] : LLONG_MAX;
-    CUDA_TRY(fill_batch_member(b->h_members.data() + mbytes * i, tl.mp, tl.mu, a,
+    CUDA_TRY(fill_batch_member(b->h_members.data() + mbytes * i, tl.mp, tl.mu, tl.mo, a,
                                s->state[0], s->state[1], s->d_gauge, &s->d_counters->steps,
                                stop_at, s->prm.monitor_every, s->cur, nch, b->m_shape[i]));
     if (build_items) {
@@ -1467,7 +1537,7 @@ static int batch_upload(fslbm_batch* b) {
 // One chained launch of `nsteps` steps for every member (each starting at its buffer cur0).
 static cudaError_t batch_enqueue(fslbm_batch* b, int nsteps, cudaStream_t st) {
   return launch_batch_steps(b->members[0]->dtype, b->ty, b->d_members, b->d_mons, b->d_items, b->nitems,
-                            nsteps, b->grid, b->packed, b->d_sync, int(b->members.size()),
+                            nsteps, b->grid, b->d_sync, int(b->members.size()),
                             b->d_tickets + 2, st);
 }
 
@@ -1576,10 +1646,6 @@ extern "C" int fslbm_batch_create(fslbm_ctx* ctx, fslbm_solve* const* solves, in
   default_tiling(b);
   if (const char* ec = std::getenv("FSLBM_BATCH_CHUNK"))
     for (int& c : b->m_chunk) c = std::max(8, std::atoi(ec));
-  // packed FP32x2 pair arithmetic, as the single-pipe kernel (FSLBM_BATCH_PACKED=0 selects the
-  // scalar form, for comparisons; both give the same bits)
-  const char* ebp = std::getenv("FSLBM_BATCH_PACKED");
-  b->packed = (ebp && std::atoi(ebp) == 0) ? 0 : 1;
   cudaError_t e = cudaSetDevice(ctx->device);
   // tile height of the batch's tiles (FSLBM_BATCH_TILE_Y=16|32 overrides the default)
   if (const char* ety = std::getenv("FSLBM_BATCH_TILE_Y")) b->ty = std::atoi(ety) == 16 ? 16 : 32;

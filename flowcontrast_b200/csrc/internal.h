@@ -63,10 +63,10 @@ cudaError_t launch_step(const StepLaunch& a, cudaStream_t st);
 // tiles): two tensor maps per input state (p box with a one-cell halo, u,v,w box with the
 // corrector halo).
 struct Step2Launch {
-  int d1, ty;                // corrective stride, tile height (16 or 32)
-  int packed;                // FP32x2 packed arithmetic (1) or scalar pairs (0)
+  int d1, ty;                // corrective stride, tile height (8, 16 or 32)
   const CUtensorMap* map_p;
   const CUtensorMap* map_uvw;
+  const CUtensorMap* map_out;  // output state, box of one warp's cells (not the FP64 kernel)
   int grid;
 };
 bool step2_supported(int dtype, int d1);
@@ -105,7 +105,7 @@ struct BatchMon {
 cudaError_t batch_prepare(int dtype, int ty);
 size_t batch_member_bytes();
 // Writes one member descriptor (layout private to the kernels) into host memory at dst.
-cudaError_t fill_batch_member(void* dst, const CUtensorMap* map_p, const CUtensorMap* map_u,
+cudaError_t fill_batch_member(void* dst, const CUtensorMap* map_p, const CUtensorMap* map_u, const CUtensorMap* map_o,
                               const StepLaunch& a, void* state0, void* state1,
                               const double* gauge_slot, const long long* steps, long long stop_at,
                               int monitor_every, int cur0, int nchunks, int shape);
@@ -116,8 +116,8 @@ cudaError_t fill_batch_member(void* dst, const CUtensorMap* map_p, const CUtenso
 // reads buffer cur0 ^ (s & 1) of each member.
 size_t batch_sync_words(int nmembers);
 cudaError_t launch_batch_steps(int dtype, int ty, const void* members, const BatchMon* mons,
-                               const int2* items, int nitems, int nsteps, int grid, int packed,
-                               unsigned* sync, int nmembers, unsigned* err, cudaStream_t st);
+                               const int2* items, int nitems, int nsteps, int grid, unsigned* sync,
+                               int nmembers, unsigned* err, cudaStream_t st);
 
 // Seeded Poiseuille start written into a pitched state (walls and pad columns zero).
 cudaError_t launch_init_poiseuille(int dtype, void* state, const uint8_t* mask, int planes, int lxp,

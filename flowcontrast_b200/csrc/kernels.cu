@@ -127,51 +127,42 @@ bool step2_supported(int dtype, int d1) {
   return (dtype == FSLBM_F32 || dtype == FSLBM_F16 || dtype == FSLBM_F64) && d1 == 2;
 }
 
-template <int TY, class TE> static void box2(int* sw, int* ph, int* uh, int* hx, int* hy) {
-  using Tl = Step2Tile<2, TY, TE>;
-  *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
+// Calls fn.template operator()<TY, TE>() for the column-pair tile of (dtype, ty).
+template <class F> static cudaError_t with_step2(int dtype, int ty, F&& fn) {
+  if (dtype == FSLBM_F32) {
+    if (ty == 32) return fn.template operator()<32, float>();
+    if (ty == 16) return fn.template operator()<16, float>();
+    if (ty == 8) return fn.template operator()<8, float>();
+  } else if (dtype == FSLBM_F16) {
+    if (ty == 32) return fn.template operator()<32, __half>();
+    if (ty == 16) return fn.template operator()<16, __half>();
+    if (ty == 8) return fn.template operator()<8, __half>();
+  }
+  return cudaErrorInvalidValue;
 }
 
 bool step2_box(int dtype, int d1, int ty, int* sw, int* ph, int* uh, int* hx, int* hy) {
-  if (d1 != 2 || (ty != 32 && ty != 16)) return false;
+  if (d1 != 2) return false;
   if (dtype == FSLBM_F64) {          // the FP64 column kernel: 32 x 16 tiles only
     using Tl = ColTile<2, 16>;
     if (ty != 16) return false;
     *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
     return true;
   }
-  if (dtype == FSLBM_F32) {
-    if (ty == 32) box2<32, float>(sw, ph, uh, hx, hy);
-    else box2<16, float>(sw, ph, uh, hx, hy);
-    return true;
-  }
-  if (dtype == FSLBM_F16) {
-    if (ty == 32) box2<32, __half>(sw, ph, uh, hx, hy);
-    else box2<16, __half>(sw, ph, uh, hx, hy);
-    return true;
-  }
-  return false;
+  return with_step2(dtype, ty, [&]<int TY, class TE>() {
+           using Tl = Step2Tile<TY, TE>;
+           *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
+           return cudaSuccess;
+         }) == cudaSuccess;
 }
 
-int step2_occupancy(int dtype, int, int ty) { return dtype != FSLBM_F64 && ty == 16 ? 2 : 1; }
-
-template <int TY, bool PK, class TE> static cudaError_t prep2() {
-  return cudaFuncSetAttribute(fslbm_step2_kernel<2, TY, PK, TE>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              int(Step2Tile<2, TY, TE>::SMEM_BYTES));
-}
-
-template <class TE> static cudaError_t prep2_all(int ty) {
-  cudaError_t e;
-  if (ty == 32) {
-    if ((e = prep2<32, true, TE>())) return e;
-    return prep2<32, false, TE>();
-  }
-  if (ty == 16) {
-    if ((e = prep2<16, true, TE>())) return e;
-    return prep2<16, false, TE>();
-  }
-  return cudaErrorInvalidValue;
+int step2_occupancy(int dtype, int, int ty) {
+  int n = 1;
+  (void)with_step2(dtype, ty, [&]<int TY, class TE>() {
+    n = Step2Tile<TY, TE>::CTAS;
+    return cudaSuccess;
+  });
+  return n;
 }
 
 cudaError_t step2_prepare(int dtype, int d1, int ty) {
@@ -180,23 +171,10 @@ cudaError_t step2_prepare(int dtype, int d1, int ty) {
     return ty != 16 ? cudaErrorInvalidValue
                     : cudaFuncSetAttribute(fslbm_col_kernel<2, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            int(ColTile<2, 16>::SMEM_BYTES));
-  if (dtype == FSLBM_F32) return prep2_all<float>(ty);
-  if (dtype == FSLBM_F16) return prep2_all<__half>(ty);
-  return cudaErrorInvalidValue;
-}
-
-template <class TE>
-static cudaError_t launch_step2_t(const Step2Launch& b, const Step2Geom& g,
-                                  const StepConst<float>& k, cudaStream_t st) {
-#define FSLBM_L2(TY, PK)                                                                  \
-  launch_chained(fslbm_step2_kernel<2, TY, PK, TE>, b.grid, Step2Tile<2, TY, TE>::THREADS, \
-                 Step2Tile<2, TY, TE>::SMEM_BYTES, st, *b.map_p, *b.map_uvw, g, k)
-  if (b.ty == 32 && b.packed) return FSLBM_L2(32, true);
-  if (b.ty == 32) return FSLBM_L2(32, false);
-  if (b.ty == 16 && b.packed) return FSLBM_L2(16, true);
-  if (b.ty == 16) return FSLBM_L2(16, false);
-#undef FSLBM_L2
-  return cudaErrorInvalidValue;
+  return with_step2(dtype, ty, [&]<int TY, class TE>() {
+    return cudaFuncSetAttribute(fslbm_step2_kernel<TY, TE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(Step2Tile<TY, TE>::SMEM_BYTES));
+  });
 }
 
 cudaError_t launch_step2(const StepLaunch& a, const Step2Launch& b, cudaStream_t st) {
@@ -221,9 +199,11 @@ cudaError_t launch_step2(const StepLaunch& a, const Step2Launch& b, cudaStream_t
     return launch_chained(fslbm_col_kernel<2, 16>, b.grid, ColTile<2, 16>::THREADS,
                           ColTile<2, 16>::SMEM_BYTES, st, *b.map_p, *b.map_uvw, g, kd);
   }
-  if (a.dtype == FSLBM_F32) return launch_step2_t<float>(b, g, k, st);
-  if (a.dtype == FSLBM_F16) return launch_step2_t<__half>(b, g, k, st);
-  return cudaErrorInvalidValue;
+  return with_step2(a.dtype, b.ty, [&]<int TY, class TE>() {
+    using Tl = Step2Tile<TY, TE>;
+    return launch_chained(fslbm_step2_kernel<TY, TE>, b.grid, Tl::THREADS, Tl::SMEM_BYTES, st, *b.map_p,
+                          *b.map_uvw, *b.map_out, g, k);
+  });
 }
 
 // ------------------------------------------------------------------------------------------
@@ -326,7 +306,6 @@ __device__ void monitor_body(const MonitorLaunch& a, double* sh) {
 template <class TS>
 __global__ void monitor_kernel(MonitorLaunch a) {
   __shared__ double sh[3 * 32];
-  grid_launch_dependents();
   grid_dependency_wait();
   monitor_body<TS>(a, sh);
 }
@@ -337,7 +316,7 @@ __global__ void monitor_kernel(MonitorLaunch a) {
 // One member of a batched ensemble: its tensor maps for both state buffers, its step geometry
 // and constants, and where its step count stops.
 struct alignas(64) BatchMember {
-  CUtensorMap map_p[2], map_u[2];
+  CUtensorMap map_p[2], map_u[2], map_o[2];
   Step2Geom g;                 // g.out is replaced by the buffer the step writes
   StepConst<float> k;
   void* state[2];
@@ -414,11 +393,12 @@ __device__ __forceinline__ bool batch_item_begin(const BatchMember& mb, int memb
 // the barrier). The CTA whose count completes a member's step books it (step counter, monitor)
 // and releases it before marching on. Counting there rather than right after the march keeps
 // the march free of register spills.
-template <int D1, int TY, bool PK, class TE>
-__global__ void __launch_bounds__(Step2Tile<D1, TY, TE>::THREADS, TY == 16 ? 2 : 1)
+template <int TY, class TE>
+__global__ void __launch_bounds__(Step2Tile<TY, TE>::THREADS, Step2Tile<TY, TE>::CTAS)
     fslbm_step2_batch_kernel(const BatchMember* __restrict__ members,
                              const BatchMon* __restrict__ mons, const int2* __restrict__ items,
                              int nitems, int nsteps, unsigned* sync, unsigned* err) {
+  using Tl = Step2Tile<TY, TE>;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ unsigned s_ticket;
   __shared__ long long s_done;
@@ -428,11 +408,15 @@ __global__ void __launch_bounds__(Step2Tile<D1, TY, TE>::THREADS, TY == 16 ? 2 :
   // kernel reads them from the parameter bank); kept in registers through the march they spill
   __shared__ StepConst<float> s_k;
   __shared__ Step2Geom s_g;
-  bool first = true;
+  uint32_t* tm_base = reinterpret_cast<uint32_t*>(smem + Tl::REL_OFFSET) + Tl::SU;
+  if (threadIdx.x < 32) tm_alloc<Tl::TM_COLS>(tm_base);
+  __syncthreads();
+  const uint32_t tmem = *tm_base;
+  bool first = true, ok = true;
   unsigned prev = ~0u;             // the CTA's previous ticket, counted at the next claim
   for (;;) {
     if (threadIdx.x == 0) s_ticket = atomicAdd(&sync[0], 1u);
-    __syncthreads();               // every thread has finished the previous item
+    if (__syncthreads_or(!ok)) break;   // every thread has finished the previous item (or one gave up)
     const unsigned t = s_ticket;
     if (threadIdx.x == 0) {
       s_book = -1;
@@ -451,54 +435,44 @@ __global__ void __launch_bounds__(Step2Tile<D1, TY, TE>::THREADS, TY == 16 ? 2 :
       const unsigned pt = unsigned(s_book);
       const int pm = items[pt % unsigned(nitems)].x;
       const int ps = int(pt / unsigned(nitems));
-      batch_book<Step2Tile<D1, TY, TE>::THREADS>(mons[pm], (ps & 1) ^ 1, s_sh, &s_due);
+      batch_book<Tl::THREADS>(mons[pm], (ps & 1) ^ 1, s_sh, &s_due);
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) st_release_gpu(sync + 5 + 2 * pm, unsigned(ps + 1));
     }
-    if (t >= unsigned(nitems) * unsigned(nsteps)) return;
+    if (t >= unsigned(nitems) * unsigned(nsteps)) break;
     const int step = int(t / unsigned(nitems));
     const int2 it = items[t % unsigned(nitems)];
     const BatchMember& mb = members[it.x];
     if (threadIdx.x == 0)          // every thread has left the previous item (ticket barriers)
       s_go = batch_item_begin(mb, it.x, step, sync, err, &s_g, &s_k, &s_done);
     __syncthreads();
-    if (!s_go) return;
+    if (!s_go) break;
     prev = t;
     if (s_done < mb.stop_at) {
       const int cur = mb.cur0 ^ (step & 1);
       const int ntiles = mb.g.ntiles;
-      const bool ok = step2_march<D1, TY, PK, TE>(&mb.map_p[cur], &mb.map_u[cur], s_g, s_k,
-                                                  it.y % ntiles, it.y / ntiles, smem, !first,
-                                                  mb.shape);
-      if (!ok) return;
+      ok = step2_march<TY, TE>(&mb.map_p[cur], &mb.map_u[cur], &mb.map_o[1 - cur], tmem, s_g, s_k,
+                               it.y % ntiles, it.y / ntiles, smem, !first, mb.shape);
       first = false;
     }
   }
-}
-
-template <int TY, bool PK, class TE> static cudaError_t batch_prep() {
-  return cudaFuncSetAttribute(fslbm_step2_batch_kernel<2, TY, PK, TE>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              int(Step2Tile<2, TY, TE>::SMEM_BYTES));
-}
-
-template <int TY, class TE> static cudaError_t batch_prep_all() {
-  cudaError_t e;
-  if ((e = batch_prep<TY, true, TE>())) return e;
-  return batch_prep<TY, false, TE>();
+  __syncthreads();
+  if (threadIdx.x < 32) tm_free<Tl::TM_COLS>(tmem);
 }
 
 cudaError_t batch_prepare(int dtype, int ty) {
-  if (ty != 16 && ty != 32) return cudaErrorInvalidValue;
-  if (dtype == FSLBM_F32) return ty == 16 ? batch_prep_all<16, float>() : batch_prep_all<32, float>();
-  if (dtype == FSLBM_F16) return ty == 16 ? batch_prep_all<16, __half>() : batch_prep_all<32, __half>();
-  return cudaErrorInvalidValue;
+  return with_step2(dtype, ty, [&]<int TY, class TE>() {
+    if constexpr (TY == 8) return cudaErrorInvalidValue;
+    else
+      return cudaFuncSetAttribute(fslbm_step2_batch_kernel<TY, TE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(Step2Tile<TY, TE>::SMEM_BYTES));
+  });
 }
 
 size_t batch_member_bytes() { return sizeof(BatchMember); }
 
-cudaError_t fill_batch_member(void* dst, const CUtensorMap* mp, const CUtensorMap* mu,
+cudaError_t fill_batch_member(void* dst, const CUtensorMap* mp, const CUtensorMap* mu, const CUtensorMap* mo,
                               const StepLaunch& a, void* state0, void* state1,
                               const double* gauge_slot, const long long* steps, long long stop_at,
                               int monitor_every, int cur0, int nchunks, int shape) {
@@ -506,6 +480,7 @@ cudaError_t fill_batch_member(void* dst, const CUtensorMap* mp, const CUtensorMa
   std::memset(&m, 0, sizeof m);
   m.map_p[0] = mp[0]; m.map_p[1] = mp[1];
   m.map_u[0] = mu[0]; m.map_u[1] = mu[1];
+  m.map_o[0] = mo[0]; m.map_o[1] = mo[1];
   m.g.lxp = a.lxp; m.g.ly = a.ly; m.g.L = a.L; m.g.ntiles = a.ntiles; m.g.nchunks = nchunks;
   m.g.tiles = a.tiles; m.g.mask = a.mask; m.g.colcoef = a.colcoef; m.g.out = nullptr;
   m.g.gauge = nullptr; m.g.err = a.err; m.g.step_counter = nullptr; m.g.step_no = 0;
@@ -520,34 +495,25 @@ cudaError_t fill_batch_member(void* dst, const CUtensorMap* mp, const CUtensorMa
   return cudaSuccess;
 }
 
-template <int TY, class TE>
-static void launch_batch_t(const BatchMember* mb, const BatchMon* mons, const int2* items,
-                           int nitems, int nsteps, int grid, int packed, unsigned* sync,
-                           unsigned* err, cudaStream_t st) {
-  using Tl = Step2Tile<2, TY, TE>;
-  if (packed)
-    fslbm_step2_batch_kernel<2, TY, true, TE><<<grid, Tl::THREADS, Tl::SMEM_BYTES, st>>>(
-        mb, mons, items, nitems, nsteps, sync, err);
-  else
-    fslbm_step2_batch_kernel<2, TY, false, TE><<<grid, Tl::THREADS, Tl::SMEM_BYTES, st>>>(
-        mb, mons, items, nitems, nsteps, sync, err);
-}
-
 size_t batch_sync_words(int nmembers) { return 4 + 2 * size_t(nmembers); }
 
 cudaError_t launch_batch_steps(int dtype, int ty, const void* members, const BatchMon* mons,
-                               const int2* items, int nitems, int nsteps, int grid, int packed,
-                               unsigned* sync, int nmembers, unsigned* err, cudaStream_t st) {
+                               const int2* items, int nitems, int nsteps, int grid, unsigned* sync,
+                               int nmembers, unsigned* err, cudaStream_t st) {
   if (nsteps < 1) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(sync, 0, batch_sync_words(nmembers) * sizeof(unsigned), st);
   if (e) return e;
   const BatchMember* mb = reinterpret_cast<const BatchMember*>(members);
-  if (ty == 32 && dtype == FSLBM_F32) launch_batch_t<32, float>(mb, mons, items, nitems, nsteps, grid, packed, sync, err, st);
-  else if (ty == 32 && dtype == FSLBM_F16) launch_batch_t<32, __half>(mb, mons, items, nitems, nsteps, grid, packed, sync, err, st);
-  else if (ty == 16 && dtype == FSLBM_F32) launch_batch_t<16, float>(mb, mons, items, nitems, nsteps, grid, packed, sync, err, st);
-  else if (ty == 16 && dtype == FSLBM_F16) launch_batch_t<16, __half>(mb, mons, items, nitems, nsteps, grid, packed, sync, err, st);
-  else return cudaErrorInvalidValue;
-  return cudaGetLastError();
+  return with_step2(dtype, ty, [&]<int TY, class TE>() {
+    if constexpr (TY == 8) {
+      return cudaErrorInvalidValue;
+    } else {
+      using Tl = Step2Tile<TY, TE>;
+      fslbm_step2_batch_kernel<TY, TE><<<grid, Tl::THREADS, Tl::SMEM_BYTES, st>>>(mb, mons, items, nitems, nsteps,
+                                                                                 sync, err);
+      return cudaGetLastError();
+    }
+  });
 }
 
 cudaError_t launch_monitor(const MonitorLaunch& a, cudaStream_t st) {
@@ -596,7 +562,6 @@ cudaError_t launch_init_poiseuille(int dtype, void* state, const uint8_t* mask, 
 // ------------------------------------------------------------------------------------------
 template <class TS>
 __global__ void fill_ghosts_kernel(TS* s, const int2* pairs, int n, size_t plane, int L) {
-  grid_launch_dependents();
   grid_dependency_wait();
   const size_t FS = plane * L;
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < size_t(n) * L;

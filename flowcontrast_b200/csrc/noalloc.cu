@@ -12,7 +12,6 @@
 #include <mutex>
 
 #include "internal.h"
-#include "step2_kernel.cuh"
 
 int fslbm_set_error(int code, const char* fmt, ...);
 
@@ -173,7 +172,8 @@ extern "C" int fslbm_step_f32_noalloc(const float* state_in, float* state_out,
   cuuint32_t boxp[4] = {cuuint32_t(sw), cuuint32_t(ph), 1, 1};
   cuuint32_t boxu[4] = {cuuint32_t(sw), cuuint32_t(uh), 1, 3};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUtensorMap mp, mu;
+  cuuint32_t boxo[4] = {32, 2, 1, 4};      // one warp's cells, four fields
+  CUtensorMap mp, mu, mo;
   CUresult r1 = g_encode(&mp, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(state_in),
                          dims, strides, boxp, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -182,7 +182,10 @@ extern "C" int fslbm_step_f32_noalloc(const float* state_in, float* state_out,
                          dims, strides, boxu, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r1 != CUDA_SUCCESS || r2 != CUDA_SUCCESS)
+  CUresult r3 = g_encode(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, state_out, dims, strides, boxo, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r1 != CUDA_SUCCESS || r2 != CUDA_SUCCESS || r3 != CUDA_SUCCESS)
     return fslbm_set_error(FSLBM_ERR_CUDA, "step_f32_noalloc: tensor map encoding failed");
 
   // step constants formed as the reference forms them in FP32 (FSLBM.cu:231, 269, 599, 624)
@@ -207,10 +210,11 @@ extern "C" int fslbm_step_f32_noalloc(const float* state_in, float* state_out,
   a.c1 = 1.0f + 0.3333333333f * blend;
   a.c2 = -0.0833333333f * blend;
   a.fx = float(prm->force[0]); a.fy = float(prm->force[1]); a.fz = float(prm->force[2]);
+  // one CTA per SM, at least a pair of planes each
   int nch = g_sm_count[dev] / a.ntiles;
+  if (nch > (lz + 1) / 2) nch = (lz + 1) / 2;
   if (nch < 1) nch = 1;
-  if (nch > lz / (4 * prm->d1)) nch = lz / (4 * prm->d1) > 0 ? lz / (4 * prm->d1) : 1;
-  Step2Launch b{2, kNoallocTY, 1, &mp, &mu, a.ntiles * nch};
+  Step2Launch b{2, kNoallocTY, &mp, &mu, &mo, a.ntiles * nch};
   if ((e = launch_step2(a, b, st)) != cudaSuccess)
     return fslbm_set_error(FSLBM_ERR_CUDA, "step_f32_noalloc: step launch: %s", cudaGetErrorString(e));
 

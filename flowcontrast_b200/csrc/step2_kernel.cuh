@@ -1,22 +1,26 @@
-// FSLBM time step, FP32 column-pair kernel for sm_100a (even corrective strides).
+// FSLBM time step, FP32 arithmetic, pairs of planes, for sm_100a (corrective stride 2, FP32 or FP16
+// storage).
 //
 // Same step as step_kernel.cuh (predictor factored by neighbour plane, coarse corrector,
 // periodic +-pin seam, walls, gauge, body force), organised for throughput:
-//  - every thread owns two adjacent columns (x, x+1) and computes both with packed FP32x2
-//    arithmetic (__ffma2_rn / __fadd2_rn / __fmul2_rn); neighbour pairs come from 64-bit
+//  - a thread owns N rows of one column and marches along the pipe two planes at a time; the two
+//    planes are the halves of packed FP32x2 operations (add2 / mul2 / fma2). Packing along the
+//    march needs no register moves: the corrector's streamwise taps are an even number of planes
+//    away, so its pairs are the window's pairs, and x and y neighbours of a pair are pairs too;
+//  - the predictor's x sums of a row (RowSums) are formed once per row and serve the rows above
+//    and below it within the thread;
+//  - a 32 x TY tile per CTA; p is staged with a one-cell halo, u,v,w with the corrector's 2*d1
+//    halo, by TMA into a window of SU pairs of planes (u,v,w) and SU - 2 pairs (p);
+//  - the own columns of the last four pairs (centre and the four streamwise taps behind and at
+//    the predictor's pair) live in tensor memory, written once by the predictor and read back
+//    with tcgen05.ld: 24 N words per thread that would otherwise be registers (spills) or
 //    shared-memory loads;
-//  - a 32 x TY tile per CTA, 16 warps per SM either way (TY = 32: one 512-thread CTA per SM;
-//    TY = 16: two 256-thread CTAs, which suit small cross-sections); p is staged with a one-cell
-//    halo, u,v,w with the corrector's 2*d1 halo, as two TMA boxes per plane into a window of 8
-//    planes for TY = 32 (output plane .. 3 planes ahead for d1 = 2), 7 for TY = 16;
-//  - no block-wide barrier in the march and no producer thread: per-slot "full" mbarriers count
-//    TMA completion, each warp releases the slots of a pair of planes after its last read of
-//    them, and the last warp to release a pair refills both slots, so warps drift within the
-//    window and none waits for a free slot;
-//  - the streamwise corrector taps behind the output plane come from a 2*d1 register history
-//    of the thread's own columns, the taps ahead from the window; in the FP32 single-pipe
-//    kernel the output plane's own centre pairs come from the predictor's centre row of the
-//    same plane, read one iteration earlier;
+//  - results leave through a shared staging block per warp and one TMA store per plane, which
+//    needs no per-store address or bounds arithmetic;
+//  - no block-wide barrier in the march and no producer thread: per-pair "full" mbarriers count
+//    TMA completion, each warp releases a pair after its last read of it, and the last warp to
+//    release a pair refills its slot, so warps drift within the window and none waits for a
+//    free slot;
 //  - grid = tiles x streamwise chunks in chunk-major order, so concurrent CTAs work at nearby
 //    planes and halos hit L2; odd chunks march downwards, so the planes two neighbouring
 //    chunks share are read by both at the same time;
@@ -35,41 +39,52 @@ namespace fslbm {
 
 // TE is the storage type of the state (float, or __half for FP16 storage); arithmetic is FP32
 // either way. Halo widths and paddings keep every TMA box start and destination on 16 bytes.
-template <int D1, int TY, class TE = float> struct Step2Tile {
-  static_assert(D1 % 2 == 0, "pair loads of the corrector taps need an even stride");
+template <int TY, class TE = float> struct Step2Tile {
+  static constexpr int D1 = 2;                          // corrective stride
+  static constexpr int N = 2;                           // rows per thread
   static constexpr int ES = int(sizeof(TE));
   static constexpr int A16 = 16 / ES;                   // elements per 16 bytes
   static constexpr int TX = 32;
-  static constexpr int THREADS = TX / 2 * TY;
-  static constexpr int WARPS = THREADS / 32;
+  static constexpr int WARPS = TY / N;                  // a warp owns 32 N cells (see the warp shapes)
+  static constexpr int THREADS = 32 * WARPS;
   static constexpr int R = 2 * D1;                      // farthest corrector tap
   static constexpr int HX = (R + A16 - 1) / A16 * A16;  // x halo, TMA-aligned (16 bytes)
   static constexpr int HY = R;
   static constexpr int SW = TX + 2 * HX;                // row length of both boxes
   static constexpr int PH = TY + 2;                     // p rows (halo 1)
   static constexpr int UH = TY + 2 * HY;                // u,v,w rows
-  static constexpr int PPLANE = (SW * PH * ES + 127) / 128 * 128 / ES;   // 128-byte aligned
-  static constexpr int UPLANE = SW * UH;
-  static constexpr int SLOT = PPLANE + 3 * UPLANE;
-  // window slots: 8 for 32 x 32 tiles (one 512-thread CTA per SM), 7 for 32 x 16 tiles, so that
-  // two 256-thread CTAs fit an SM's shared memory
-  static constexpr int S = TY == 16 ? 7 : 8;
-  static constexpr int AHEAD = S - R - 1;               // planes loaded beyond the current one
-  static_assert(AHEAD >= 1, "window too small for the corrector reach");
-  static constexpr uint32_t TX_BYTES = uint32_t((SW * PH + 3 * UPLANE) * ES);
-  static constexpr size_t RING_BYTES = size_t(S) * SLOT * ES;
-  static constexpr size_t BAR_OFFSET = RING_BYTES;
-  // FP16 storage: the tile's base of w (FP32) for columns org.x-2 .. org.x+TX+1 and rows
-  // org.y-1 .. org.y+TY, after the barriers and counters
-  static constexpr int BW = TX + 4, BH = TY + 2;
-  static constexpr size_t BASE_OFFSET = (BAR_OFFSET + S * sizeof(uint64_t) + S * sizeof(uint32_t) + 15) / 16 * 16;
+  static constexpr int PPL = (SW * PH * ES + 127) / 128 * 128 / ES;   // p plane, 128-byte aligned
+  static constexpr int UPL = SW * UH;                                 // u, v or w plane
+  static constexpr int VPL = (3 * UPL * ES + 127) / 128 * 128 / ES;   // u,v,w of one plane
+  // Window, in pairs of planes. In use: the output pair, the predictor's pair and the one after
+  // it; one more is in flight. p is read by the predictor only.
+  static constexpr int SU = 4, SP = SU - 2;
+  static constexpr uint32_t U_BYTES = uint32_t(3 * UPL * ES), P_BYTES = uint32_t(SW * PH * ES);
+  static constexpr size_t P_OFFSET = size_t(SU) * 2 * VPL * ES;
+  // staging of a warp's output pair: [plane][field][row][column] of the warp's cells
+  static constexpr int STG = 2 * 4 * N * 32;
+  static constexpr size_t STG_OFFSET = P_OFFSET + size_t(SP) * 2 * PPL * ES;
+  static constexpr size_t BAR_OFFSET = STG_OFFSET + size_t(WARPS) * STG * ES;   // a "full" mbarrier per slot
+  static constexpr size_t REL_OFFSET = BAR_OFFSET + SU * sizeof(uint64_t);       // release counters, tensor memory base
+  // FP16 storage: the tile's base of w (FP32) for columns org.x-1 .. org.x+TX and rows
+  // org.y-1 .. org.y+TY
+  static constexpr int BW = TX + 2, BH = TY + 2;
+  static constexpr size_t BASE_OFFSET = (REL_OFFSET + (SU + 1) * sizeof(unsigned) + 15) / 16 * 16;
   static constexpr size_t BASE_BYTES = std::is_same<TE, __half>::value ? size_t(BW) * BH * sizeof(float) : 0;
-  // a "full" mbarrier per slot, then a release counter per slot
-  static constexpr size_t SMEM_BYTES = BASE_BYTES ? BASE_OFFSET + BASE_BYTES
-                                                  : BAR_OFFSET + S * sizeof(uint64_t) + S * sizeof(uint32_t);
-  static_assert((PPLANE * ES) % 128 == 0 && (UPLANE * ES) % 16 == 0 && (SLOT * ES) % 128 == 0,
-                "TMA destinations must stay aligned");
+  static constexpr size_t SMEM_BYTES = BASE_OFFSET + BASE_BYTES;
+  // tensor memory: a ring of 4 pairs of a warp's own columns of u, v, w; warps w, w + 4, ... share
+  // the 32 lanes of subpartition w % 4
+  static constexpr int TM_SLOT = 6 * N, TM_WARP = 4 * TM_SLOT;
+  static constexpr int TM_NEED = TM_WARP * ((WARPS + 3) / 4);
+  static constexpr int TM_COLS = TM_NEED <= 32 ? 32 : TM_NEED <= 64 ? 64 : TM_NEED <= 128 ? 128 : 256;
+  // CTAs per SM (shared memory; 128 registers a thread at 16 warps per SM)
+  static constexpr int CTAS = TY == 32 ? 1 : TY == 16 ? (ES == 2 ? 2 : 1) : 3;
+  static_assert(TM_NEED <= TM_COLS && TM_COLS * CTAS <= 512, "tensor memory columns");
+  static_assert((PPL * ES) % 128 == 0 && (VPL * ES) % 128 == 0 && (STG * ES) % 128 == 0,
+                "TMA addresses must stay aligned");
   static_assert((HX * ES) % 16 == 0, "TMA box x start must be 16-byte aligned");
+  static_assert(SMEM_BYTES <= 227 * 1024, "window exceeds a CTA's shared memory");
+  static_assert(TY % 8 == 0, "warp shapes within a 32-wide tile");
 };
 
 struct Step2Geom {
@@ -90,10 +105,8 @@ struct Step2Geom {
 };
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 lds2(const float* p) { return *reinterpret_cast<const float2*>(p); }
-__device__ __forceinline__ float2 lds2(const __half* p) {
-  return __half22float2(*reinterpret_cast<const __half2*>(p));
-}
+__device__ __forceinline__ float lds1(const float* p) { return *p; }
+__device__ __forceinline__ float lds1(const __half* p) { return __half2float(*p); }
 
 // 32-bit integer hash (the "lowbias32" finaliser of C. Wellons' hash-prospector, public domain).
 __device__ __forceinline__ uint32_t hash32(uint32_t x) {
@@ -115,151 +128,158 @@ __device__ __forceinline__ __half sr_half(float x, uint32_t r) {
   return __float2half_rz(x + copysignf(noise, x));
 }
 
-// Stores of one column pair's four fields. FP32 storage stores the values; FP16 storage rounds
-// stochastically with noise from (pair index, field, time step) only, so a pipe's result does
-// not depend on which other work shares the launch.
-template <class TE> struct PairStore;
-template <> struct PairStore<float> {
-  static __device__ __forceinline__ void put(float* o, size_t fs, float2 p, float2 u, float2 v,
-                                             float2 w, const float*, uint32_t) {
-    *reinterpret_cast<float2*>(o) = p;
-    *reinterpret_cast<float2*>(o + fs) = u;
-    *reinterpret_cast<float2*>(o + 2 * fs) = v;
-    *reinterpret_cast<float2*>(o + 3 * fs) = w;
-  }
-};
-template <> struct PairStore<__half> {
-  static __device__ __forceinline__ __half2 sr2(float2 a, uint32_t r) {
-    return __halves2half2(sr_half(a.x, r), sr_half(a.y, r >> 16));
-  }
-  static __device__ __forceinline__ void put(__half* o, size_t fs, float2 p, float2 u, float2 v,
-                                             float2 w, const __half* base, uint32_t seed) {
-    const uint32_t key = uint32_t(o - base) << 2;
-    *reinterpret_cast<__half2*>(o) = sr2(p, hash32(key ^ seed));
-    *reinterpret_cast<__half2*>(o + fs) = sr2(u, hash32((key | 1u) ^ seed));
-    *reinterpret_cast<__half2*>(o + 2 * fs) = sr2(v, hash32((key | 2u) ^ seed));
-    *reinterpret_cast<__half2*>(o + 3 * fs) = sr2(w, hash32((key | 3u) ^ seed));
-  }
-};
+// Arithmetic on a pair of planes (.x the march-earlier plane, .y the later one): packed FP32x2
+// instructions, each half rounded as the scalar operation.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// Column-pair arithmetic: packed FP32x2 instructions (PK = true) or two scalar ones.
-template <bool PK> struct Pair;
-template <> struct Pair<true> {
-  static __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-  static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-  static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+// x sums of one row at one column (two planes). With weights {4,1,1} over cx = 0, +1, -1 (R) or
+// the difference +1 minus -1 (D), of the terms of the brackets as polynomials of cy:
+//   0: q + 3 cx u + 4.5 cx^2 u^2        (P0 at cy = 0)
+//   1: v (1 + 3 cx u)                   (P0 = 0 + 3 cy 1 + 4.5 cy^2 2)
+//   2: v^2
+//   z: w (1 + 3 cx u)                   (P1/3 = z + 3 cy m)
+//   m: v w
+//   w: w^2                              (P2/4.5)
+struct RowSums {
+  float2 R0, D0, R1, D1, R2, D2, Rz, Dz, Rm, Dm, Rw, Dw;
 };
-template <> struct Pair<false> {
-  static __device__ __forceinline__ float2 add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-  static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
-  static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) {
-    return make_float2(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y));
-  }
-};
+__device__ __forceinline__ float2 rsum(float2 l, float2 c, float2 r) { return fma2(f2(4.0f), c, add2(l, r)); }
 
-// Predictor brackets of one in-plane neighbour (cx, cy), see step_kernel.cuh:
-// P0 = q + a(3 + 4.5a), P1' = w(1 + 3a) (= P1/3), P2' = w^2 (= P2/4.5), a = cx u + cy v.
-template <bool PK, int CX, int CY>
-__device__ __forceinline__ void brackets(float2 Q, float2 U, float2 V, float2 W, float2& P0,
-                                         float2& P1, float2& P2) {
-  using F = Pair<PK>;
-  P2 = F::mul(W, W);
-  if (CX == 0 && CY == 0) {
-    P0 = Q;
-    P1 = W;
-  } else if (CY == 0 || CX == 0) {
-    // a = s*B, s = +-1: a(3 + 4.5a) = B(3s + 4.5B), 1 + 3a = 1 + 3sB
-    const float2 B = CY == 0 ? U : V;
-    constexpr float s = float(CX + CY);
-    P0 = F::fma(B, F::fma(B, f2(4.5f), f2(3.0f * s)), Q);
-    P1 = F::mul(W, F::fma(B, f2(3.0f * s), f2(1.0f)));
-  } else {
-    // a = CX (U + CX*CY V) = CX a': a(3 + 4.5a) = a'(3 CX + 4.5 a'), 1 + 3a = 1 + 3 CX a'
-    const float2 a1 = F::fma(V, f2(float(CX * CY)), U);
-    P0 = F::fma(a1, F::fma(a1, f2(4.5f), f2(3.0f * CX)), Q);
-    P1 = F::mul(W, F::fma(a1, f2(3.0f * CX), f2(1.0f)));
+__device__ __forceinline__ RowSums row_sums(const float2 (&p)[3], const float2 (&u)[3], const float2 (&v)[3],
+                                            const float2 (&w)[3]) {
+  float2 P[3], V[3], V2[3], W[3], M[3], W2[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    V2[j] = mul2(v[j], v[j]);
+    W2[j] = mul2(w[j], w[j]);
+    M[j] = mul2(v[j], w[j]);
+    const float2 s = add2(V2[j], W2[j]);
+    if (j == 1) {
+      P[j] = fma2(f2(-1.5f), fma2(u[j], u[j], s), p[j]);
+      V[j] = v[j];
+      W[j] = w[j];
+    } else {
+      const float sg = j == 2 ? 3.0f : -3.0f;
+      const float2 a = fma2(u[j], f2(sg), f2(1.0f));
+      // q + 3 cx u + 4.5 u^2 = p - 1.5 (v^2 + w^2) + u (3 u + 3 cx)
+      P[j] = fma2(u[j], fma2(u[j], f2(3.0f), f2(sg)), fma2(f2(-1.5f), s, p[j]));
+      V[j] = mul2(v[j], a);
+      W[j] = mul2(w[j], a);
+    }
   }
+  RowSums o;
+  o.R0 = rsum(P[0], P[1], P[2]);   o.D0 = sub2(P[2], P[0]);
+  o.R1 = rsum(V[0], V[1], V[2]);   o.D1 = sub2(V[2], V[0]);
+  o.R2 = rsum(V2[0], V2[1], V2[2]); o.D2 = sub2(V2[2], V2[0]);
+  o.Rz = rsum(W[0], W[1], W[2]);   o.Dz = sub2(W[2], W[0]);
+  o.Rm = rsum(M[0], M[1], M[2]);   o.Dm = sub2(M[2], M[0]);
+  o.Rw = rsum(W2[0], W2[1], W2[2]); o.Dw = sub2(W2[2], W2[0]);
+  return o;
 }
 
-template <bool PK>
-__device__ __forceinline__ float2 qof(float2 P, float2 U, float2 V, float2 W) {
-  using F = Pair<PK>;
-  return F::fma(f2(-1.5f), F::fma(U, U, F::fma(V, V, F::mul(W, W))), P);
+// A row's contribution to the output row one above (cy = -1) or below (cy = +1) it.
+struct RowSide {
+  float2 R0, D0, Rz, Dz, Rw, Dw;
+};
+template <int CY> __device__ __forceinline__ RowSide row_side(const RowSums& o) {
+  RowSide s;
+  s.R0 = fma2(f2(3.0f * CY), o.R1, fma2(f2(4.5f), o.R2, o.R0));
+  s.D0 = fma2(f2(3.0f * CY), o.D1, fma2(f2(4.5f), o.D2, o.D0));
+  s.Rz = fma2(f2(3.0f * CY), o.Rm, o.Rz);
+  s.Dz = fma2(f2(3.0f * CY), o.Dm, o.Dz);
+  s.Rw = o.Rw;
+  s.Dw = o.Dw;
+  return s;
+}
+
+// Tensor memory accesses of a warp: thread i reads and writes lane i of the warp's subpartition.
+__device__ __forceinline__ void tm_store(uint32_t a, float2 v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void tm_load(float2 (&v)[2], uint32_t a) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void tm_wait_stores() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// Completes the loads into v0 .. v3: their uses cannot move before the wait.
+__device__ __forceinline__ void tm_wait_loads(float2 (&v0)[2], float2 (&v1)[2], float2 (&v2)[2], float2 (&v3)[2]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(v0[0].x), "+f"(v0[0].y), "+f"(v0[1].x), "+f"(v0[1].y), "+f"(v1[0].x), "+f"(v1[0].y),
+                 "+f"(v1[1].x), "+f"(v1[1].y), "+f"(v2[0].x), "+f"(v2[0].y), "+f"(v2[1].x), "+f"(v2[1].y),
+                 "+f"(v3[0].x), "+f"(v3[0].y), "+f"(v3[1].x), "+f"(v3[1].y)
+               :: "memory");
+}
+// Allocation of a kernel's tensor memory by its first warp (whole warp); `slot` in shared memory
+// receives the base address. Freed by the same warp before the kernel ends, on every path.
+template <int COLS> __device__ __forceinline__ void tm_alloc(uint32_t* slot) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "n"(COLS)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+template <int COLS> __device__ __forceinline__ void tm_free(uint32_t base) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(COLS) : "memory");
 }
 
 // Marches one (tile, chunk) work item of one pipe: the step of every cell of the tile's columns
-// in the chunk's planes. `reinit` re-arms the CTA's mbarriers when the CTA has marched an item
-// before (persistent grids). Returns false when a bounded wait gave up (error flag set).
-// Freed window slots are refilled by the last warp to release them (no warp waits for a free
-// slot); measured +2 % on the single pipe and +1.7 % on the batched ensemble against thread 0
-// waiting on per-slot "empty" mbarriers and refilling.
-// The warp shape (below) is a runtime argument: it only places each thread in the tile, and a
-// kernel that inlines one march for every shape (the batched kernel, whose members choose their
-// shape) keeps one copy of the march instead of one per shape, which ended its register spills.
-// kCarry: the output plane's centre pairs come from the predictor's centre row of the same plane
-// (one iteration earlier, 8 registers held) instead of 4 shared loads per plane: +1.0 % on the
-// single FP32 pipe, -9 % in the batched kernel and -3 % with FP16 storage, which therefore do
-// not use it.
-template <int D1, int TY, bool PK, class TE, bool kCarry = false>
+// in the chunk's planes. `tmem` is the CTA's tensor memory, `reinit` re-arms the CTA's mbarriers
+// when the CTA has marched an item before (persistent grids). Returns false when a bounded wait
+// gave up (error flag set). The results are complete (visible to this thread) on return.
+// The warp shape is a runtime argument: it only places each thread in the tile. 0: 32 columns x
+// 2 rows; 1: 16 columns x 4 rows; 2: 8 columns x 8 rows (a thread's two rows are adjacent in all
+// of them). The smaller shapes let warps over wall skip at a finer grain, which pays for small
+// cross-sections. With the 160-byte FP32 row stride the shapes 0 and 1 read shared memory without
+// bank conflicts (rows 2 apart are 16 banks apart), shape 2 two-way. The map changes no thread's
+// arithmetic.
+template <int TY, class TE>
 __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUtensorMap* tmap_uvw,
-                                            const Step2Geom& g, const StepConst<float>& k,
-                                            int tile, int chunk, unsigned char* smem, bool reinit,
-                                            int shape = 0) {
-  using Tl = Step2Tile<D1, TY, TE>;
-  using F = Pair<PK>;
-  static_assert(D1 == 2, "the march prologue below is written for d1 = 2 (R = 4)");
-  constexpr int R = Tl::R, HX = Tl::HX, HY = Tl::HY, SW = Tl::SW, S = Tl::S;
-  constexpr int PPL = Tl::PPLANE, UPL = Tl::UPLANE, SLOT = Tl::SLOT;
-
-  // window slot of march plane m and the parity of its fill (m >= 0)
-  auto slot_of = [](int m) { return int(unsigned(m) % unsigned(S)); };
-  auto phase_of = [](int m) { return uint32_t((unsigned(m) / unsigned(S)) & 1u); };
-  TE* ring = reinterpret_cast<TE*>(smem);
+                                            const CUtensorMap* tmap_out, uint32_t tmem, const Step2Geom& g,
+                                            const StepConst<float>& k, int tile, int chunk,
+                                            unsigned char* smem, bool reinit, int shape) {
+  using Tl = Step2Tile<TY, TE>;
+  constexpr int N = Tl::N, R = Tl::R, D1 = Tl::D1, HX = Tl::HX, HY = Tl::HY, SW = Tl::SW, SU = Tl::SU, SP = Tl::SP;
+  constexpr int PPL = Tl::PPL, UPL = Tl::UPL, VPL = Tl::VPL;
+  TE* uring = reinterpret_cast<TE*>(smem);
+  TE* pring = reinterpret_cast<TE*>(smem + Tl::P_OFFSET);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + Tl::BAR_OFFSET);
-  // per slot: warp releases, counted to elect the refilling warp
-  unsigned* released = reinterpret_cast<unsigned*>(full + S);
+  unsigned* released = reinterpret_cast<unsigned*>(smem + Tl::REL_OFFSET);
 
-  // Warp shape. 0: 32 columns x 2 rows (each half-warp reads one contiguous row); 1: 16 columns
-  // (8 pairs) x 4 rows; 2: 8 columns (4 pairs) x 8 rows. The smaller shapes let warps over wall
-  // skip at a finer grain, which pays for small cross-sections (16 x 4: measured +6 % on the
-  // mixed-size ensemble, -2 % on the 128 x 128 pipe). 16 x 4: lanes 0-15 take rows 0 and 2 of
-  // the warp, lanes 16-31 rows 1 and 3; 8 x 8: lanes 4r .. 4r+3 take row r. With the 160-byte
-  // FP32 row stride each half-warp's 64-bit shared loads fall on distinct banks in every shape
-  // (FP16 rows of 96 bytes: conflict-free for 32 x 2 and 16 x 4, two-way for 8 x 8). The map
-  // changes no thread's arithmetic.
-  static_assert(Tl::TX == 32 && TY % 8 == 0, "warp shapes within a 32-wide tile");
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int tp = tid % (Tl::TX / 2), ty = tid / (Tl::TX / 2);
-  if (shape == 1) {
-    tp = (warp & 1) * 8 + (lane & 7);
-    ty = (warp >> 1) * 4 + ((lane >> 3) & 1) * 2 + (lane >> 4);
-  } else if (shape == 2) {
-    tp = (warp & 3) * 4 + (lane & 3);
-    ty = (warp >> 2) * 8 + (lane >> 2);
-  }
+  // position in the tile: the warp's cells start at (wx, wy), the thread's two rows at ty
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int wcols = 32 >> shape, wx = (warp & ((1 << shape) - 1)) * wcols, wy = (warp >> shape) * (N << shape);
+  const int lrow = (lane >> (5 - shape)) * N, lcol = lane & (wcols - 1);
+  const int tx = wx + lcol, ty = wy + lrow;
 
   // ---- work: one (tile, chunk); odd chunks march towards -z
   const int zb = int((long long)g.L * chunk / g.nchunks);
-  const int ze = int((long long)g.L * (chunk + 1) / g.nchunks);
+  const int nout = int((long long)g.L * (chunk + 1) / g.nchunks) - zb;
   const int dir = (chunk & 1) ? -1 : 1;
-  const int nout = ze - zb, niter = nout + 2 * R;
-  const int start = dir > 0 ? zb - R : ze - 1 + R;      // real plane of march index 0
+  const int nstage = (nout + 1) / 2 + R;                // pairs of planes: the outputs and 2 R planes
+  const int start = dir > 0 ? zb - R : zb + nout - 1 + R;   // real plane of march index 0
   const int2 org = g.tiles[tile];
-  const int xa = org.x + 2 * tp, y = org.y + ty;
-  const bool inside = xa < g.lxp && y < g.ly;
+  const int x = org.x + tx, y0 = org.y + ty;
 
-  float2 ws0 = f2(0.f), wsx = f2(0.f), wsy = f2(0.f), fl = f2(0.f);
-  if (inside) {
-    const ColCoef<float>* cp = reinterpret_cast<const ColCoef<float>*>(g.colcoef) + size_t(y) * g.lxp + xa;
-    const ColCoef<float> ca = cp[0], cb = cp[1];
-    ws0 = make_float2(ca.ws0, cb.ws0); wsx = make_float2(ca.wsx, cb.wsx);
-    wsy = make_float2(ca.wsy, cb.wsy); fl = make_float2(ca.fluid, cb.fluid);
+  // warps that compute (some fluid) and warps over fluid away from walls (no wall sums)
+  const ColCoef<float>* ccol = reinterpret_cast<const ColCoef<float>*>(g.colcoef) + ((long long)y0 * g.lxp + x);
+  auto coef = [&](int r) {             // outside the cross-section: nothing
+    return x < g.lxp && y0 + r < g.ly ? ccol[r * g.lxp] : ColCoef<float>{0.f, 0.f, 0.f, 0.f};
+  };
+  bool some = false, every = true;
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    const ColCoef<float> c = coef(r);
+    some |= c.fluid != 0.0f;
+    every &= c.fluid != 0.0f && c.ws0 == 0.0f && c.wsx == 0.0f && c.wsy == 0.0f;
   }
-  const bool warp_on = __any_sync(0xffffffffu, fl.x != 0.f || fl.y != 0.f);
+  const bool warp_on = __any_sync(0xffffffffu, some);
+  const bool plain = __all_sync(0xffffffffu, every);
 
   __syncthreads();   // a previous item (persistent grids) is fully consumed
   if (tid == 0) {
-    for (int s = 0; s < S; ++s) {
+    for (int s = 0; s < SU; ++s) {
       if (reinit) mbar_inval(&full[s]);
       mbar_init(&full[s], 1);
       released[s] = 0u;
@@ -271,341 +291,334 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   float* wbs = reinterpret_cast<float*>(smem + Tl::BASE_OFFSET);
   if (kBase && g.wb)
     for (int i = tid; i < Tl::BW * Tl::BH; i += Tl::THREADS) {
-      const int gx = org.x - 2 + i % Tl::BW, gy = org.y - 1 + i / Tl::BW;
+      const int gx = org.x - 1 + i % Tl::BW, gy = org.y - 1 + i / Tl::BW;
       wbs[i] = (gx >= 0 && gy >= 0 && gx < g.lxp && gy < g.ly) ? g.wb[size_t(gy) * g.lxp + gx] : 0.0f;
     }
   __syncthreads();
 
-  auto issue = [&](int m) {            // load march plane m into slot m % S
-    const int slot = slot_of(m);
-    int zz = (start + dir * m) % g.L;
-    if (zz < 0) zz += g.L;
-    TE* dst = ring + slot * SLOT;
-    mbar_arrive_expect_tx(&full[slot], Tl::TX_BYTES);
-    tma_load_4d(dst, tmap_p, &full[slot], org.x - HX, org.y - 1, zz, 0);
-    tma_load_4d(dst + PPL, tmap_uvw, &full[slot], org.x - HX, org.y - HY, zz, 1);
+  // stage j: u,v,w of the plane pair j (march planes 2j, 2j + 1) and p of the pair j - 1, which
+  // the predictor reads in the iteration that waits for this stage
+  auto plane_of = [&](int m) {
+    int zz = start + dir * m;
+    if (zz < 0 || zz >= g.L) zz %= g.L;
+    return zz < 0 ? zz + g.L : zz;
   };
-  if (tid == 0) {                      // the whole ring up front
+  auto issue = [&](int j) {
+    uint64_t* bar = &full[unsigned(j) % unsigned(SU)];
+    const bool with_p = j >= 2;
+    mbar_arrive_expect_tx(bar, 2 * Tl::U_BYTES + (with_p ? 2 * Tl::P_BYTES : 0u));
+    TE* du = uring + unsigned(j) % unsigned(SU) * (2 * VPL);
+    tma_load_4d(du, tmap_uvw, bar, org.x - HX, org.y - HY, plane_of(2 * j), 1);
+    tma_load_4d(du + VPL, tmap_uvw, bar, org.x - HX, org.y - HY, plane_of(2 * j + 1), 1);
+    if (with_p) {
+      TE* dp = pring + unsigned(j - 1) % unsigned(SP) * (2 * PPL);
+      tma_load_4d(dp, tmap_p, bar, org.x - HX, org.y - 1, plane_of(2 * j - 2), 0);
+      tma_load_4d(dp + PPL, tmap_p, bar, org.x - HX, org.y - 1, plane_of(2 * j - 1), 0);
+    }
+  };
+  if (tid == 0) {                      // the whole window up front
     prefetch_tensormap(tmap_p);
     prefetch_tensormap(tmap_uvw);
-    for (int m = 0; m < S && m < niter; ++m) issue(m);
+    for (int j = 0; j < SU && j < nstage; ++j) issue(j);
   }
-  // failure path: any warp may have issued loads up to S planes ahead; let them land (bounded)
-  auto drain = [&](int from) {
-    if (lane == 0)
-      for (int q = from; q < niter && q < from + S; ++q)
-        mbar_wait_bounded(&full[slot_of(q)], phase_of(q), kWaitLimitNs / 8);
-  };
-  // wait for march plane m; false after flagging a failure (the caller returns)
-  auto arrive_wait = [&](int m) -> bool {
-    if (mbar_wait_bounded(&full[slot_of(m)], phase_of(m), kWaitLimitNs)) return true;
-    if (lane == 0) atomicOr(g.err, 1u);
-    drain(m + 1);
+  // Wait for stage j; false after flagging a failure (the caller returns). Then any warp may have
+  // issued loads up to SU stages ahead: let them land (bounded).
+  auto arrive_wait = [&](int j) -> bool {
+    auto wait = [&](int q, uint64_t limit) {
+      return mbar_wait_bounded(&full[unsigned(q) % unsigned(SU)], (unsigned(q) / unsigned(SU)) & 1u, limit);
+    };
+    if (wait(j, kWaitLimitNs)) return true;
+    if (lane == 0) {
+      atomicOr(g.err, 1u);
+      for (int q = j + 1; q < nstage && q <= j + SU; ++q) wait(q, kWaitLimitNs / 8);
+    }
     return false;
   };
-  // Plane m - R leaves the window at iteration m (its last reader is output(m - R)). Planes leave
-  // in pairs: at odd p = m - R, planes p - 1 and p, whose slots take planes p - 1 + S and p + S.
-  // __syncwarp orders the warp's shared loads before lane 0's acq_rel add to the pair's counter
-  // (the slot of plane p); the warp whose add completes the count has acquired every warp's loads
-  // and orders them before its TMA writes with a proxy fence. One add per two planes halves the
-  // release cost, which is a fence-like wait (measured: plain step +1.5 %, batched ensemble +9 %).
-  // Plane m fills the slot of plane m - S, so a warp waiting for plane m needs every warp to have
-  // released at iteration m - AHEAD at the latest (instead of m - AHEAD - 1): an earlier
-  // iteration, as AHEAD >= 1, so no wait depends on itself. A counter's next use (2S planes later
-  // for odd S, S for S = 8) comes only after every warp has passed its previous use, so the count
-  // is a multiple of WARPS exactly when a pair is complete.
-  auto release_produce = [&](int m) -> bool {
+  // Pair j leaves the window (u,v,w after it was the output pair, p of pair j + 1 after the
+  // predictor read it, both in iteration j + 1). __syncwarp orders the warp's shared loads before
+  // lane 0's acq_rel add to the slot's counter; the warp whose add completes the count has
+  // acquired every warp's loads, orders them before its TMA writes with a proxy fence and refills
+  // the slot with stage j + SU (p of pair j + SU - 1, into the slot of p of pair j + 1). A warp
+  // waiting for stage q needs every warp to have released pair q - SU, in iteration q - SU + 1,
+  // an earlier one than the waiting iteration q - 1, so no wait depends on itself. A slot's next
+  // count starts only after its refill has landed, so the count is a multiple of WARPS exactly
+  // when a pair is complete.
+  auto release = [&](int j) {
     __syncwarp();
-    if (m >= R && ((m - R) & 1) && lane == 0) {
-      const int slot = slot_of(m - R);
-      const unsigned seen = atom_add_acq_rel_cta(&released[slot], 1u) + 1u;
-      const int mn = m - R + S - 1;
-      if (seen % unsigned(Tl::WARPS) == 0u && mn < niter) {
+    if (lane == 0) {
+      const unsigned seen = atom_add_acq_rel_cta(&released[unsigned(j) % unsigned(SU)], 1u) + 1u;
+      if (seen % unsigned(Tl::WARPS) == 0u && j + SU < nstage) {
         fence_proxy_async_smem();
-        issue(mn);
-        if (mn + 1 < niter) issue(mn + 1);
+        issue(j + SU);
       }
     }
-    return true;
   };
 
+  if (!arrive_wait(0) || !arrive_wait(1)) return false;
   if (!warp_on) {   // all-wall warps keep the pipeline protocol only
-    for (int m = 0; m < niter; ++m)
-      if (!arrive_wait(m) || !release_produce(m)) return false;
+#pragma unroll 1
+    for (int q = 1; q <= nstage - 2; ++q) {
+      if (!arrive_wait(q + 1)) return false;
+      release(q - 1);
+    }
     return true;
   }
 
   // the gauge may have been written by another CTA of the same (chained batched) launch: read
   // it from L2, not from a possibly stale L1 line
   const float gauge = g.gauge ? float(__ldcg(g.gauge)) : 0.0f;
-  const float2 wgt2 = (kBase && g.wgt && inside) ? *reinterpret_cast<const float2*>(g.wgt + size_t(y) * g.lxp + xa)
-                                                 : f2(0.f);
-  const size_t FS = size_t(g.lxp) * g.ly * g.L;
-  const TE* obase = reinterpret_cast<const TE*>(g.out);
-  const uint32_t seed = hash32(g.step_no * 0x9e3779b9u + 0x632be5abu);
-  TE* outp = reinterpret_cast<TE*>(g.out) + (size_t(start + dir * R) * g.ly + y) * g.lxp + xa;
-  const long long ostep = (long long)dir * g.ly * g.lxp;     // output pointer step per plane
-  const int po = (ty + 1) * SW + HX + 2 * tp;                 // p box
-  const int uo = PPL + (ty + HY) * SW + HX + 2 * tp;          // u box (v, w at +UPL, +2 UPL)
-  // seam pressure jump: a wrapped plane adds off to p on its non-wall cells, i.e. off times the
-  // non-wall weight sums (raw units, x36) to the row-factored A0, X0, Y0
-  const float n0[2] = {36.f - 36.f * ws0.x, 36.f - 36.f * ws0.y};
-  const float nx[2] = {-36.f * wsx.x, -36.f * wsx.y};
-  const float ny[2] = {-36.f * wsy.x, -36.f * wsy.y};
+  const int po = (ty + 1) * SW + HX + tx;               // p box
+  const int uo = (ty + HY) * SW + HX + tx;              // u box (v, w at +UPL, +2 UPL)
   const float h6 = float(dir) / 72.0f;
   // folded update: u_new = K1 t1 + K2 t2 + K0 u + tb (u* + F), the corrector's taps t1 / t2 at
   // distance d1 / 2 d1, K0 = tb dtddy m c0 + (1 - tb), K1 = tb dtddy m c1, K2 = tb dtddy m c2
   const float kam = __fmul_rn(__fmul_rn(k.tb, k.dtddy), k.m);
   const float kK0 = __fmaf_rn(kam, k.c0, k.cc), kK1 = __fmul_rn(kam, k.c1), kK2 = __fmul_rn(kam, k.c2);
-  const float ktz = __fmul_rn(float(dir), k.tb);              // the z-moment carries the sign
+  const float ktz = __fmul_rn(float(dir), k.tb);        // the z-moment carries the sign
+  // FP16 storage: the rounding noise of a cell pair is keyed by its first cell, the field and the step
+  const uint32_t seed = hash32(g.step_no * 0x9e3779b9u + 0x632be5abu);
 
-  float2 hu[4], hv[4], hw[4];                                 // own columns of planes jo-4..jo-1
-  // Predictor terms waiting for their output plane: b2 = the march-previous plane's share of the
-  // output being completed, b1 = the same for the next output, s1 = the self-plane moments of
-  // the next output. Each output sums its two neighbour planes' shares first (a commutative
-  // add) and then fuses its own plane's share, so the FP32 result of a cell does not depend on
-  // the march direction and hence not on how the pipe is split into streamwise chunks.
-  float b2[4][2], b1[4][2], s1[3][2];
+  auto ldu = [&](const TE* q) { return make_float2(lds1(q), lds1(q + VPL)); };
+  // ring of the own columns of the last four pairs in tensor memory: pair j in slot j % 4, field f
+  // of row r at column f 2 N + 2 r
+  const uint32_t tm = tmem + (uint32_t(warp & 3) << 21) + uint32_t((warp >> 2) * Tl::TM_WARP);
+  auto tm_slot = [&](int j) { return tm + (unsigned(j) & 3u) * unsigned(Tl::TM_SLOT); };
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    hu[j] = hv[j] = hw[j] = f2(0.f);
-    b2[j][0] = b2[j][1] = b1[j][0] = b1[j][1] = 0.f;
-    if (j < 3) s1[j][0] = s1[j][1] = 0.f;
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+      for (int r = 0; r < N; ++r)
+        tm_store(tm_slot(j) + f * 2 * N + 2 * r, ldu(uring + j * 2 * VPL + uo + f * UPL + r * SW));
+  // staging: the thread's place in the warp's block of wcols x (N << shape) cells
+  TE* stg = reinterpret_cast<TE*>(smem + Tl::STG_OFFSET) + warp * Tl::STG;
+  TE* sto = stg + lrow * wcols + lcol;
+  // Predictor terms carried to the next iteration, per row: cl = the finished sums of the pair's
+  // first plane, sh = the self-plane moments of its second, dl / dh = the shares that the first
+  // and second plane give their march-next planes, pc = p of the pair.
+  float cl[N][4], sh[N][3], dl[N][3], dh[N][3];
+  float2 pc[N];
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    pc[r] = f2(0.f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      cl[r][j] = 0.f;
+      if (j < 3) sh[r][j] = dl[r][j] = dh[r][j] = 0.f;
+    }
   }
-  float2 comp0, comp1, comp2, comp3;
-  float2 cen[4] = {}, cnx[4] = {};   // kCarry: centre pairs p,u,v,w of the output plane / the predictor plane
 
-  // predictor contribution of march plane ma (see step_kernel.cuh for the factorisation)
-  auto predictor = [&](int ma) {
-    const TE* ss = ring + slot_of(ma) * SLOT;
-    const int sp = start + dir * ma;                          // real plane
-    const float off = sp < 0 ? k.pin : (sp >= g.L ? -k.pin : 0.0f);
-    // Row-factored weights w(cx)w(cy) = {4,1,1}x{4,1,1}/36, per column of the pair: per row
-    // R = P(-1)+P(+1)+4P(0), D = P(+1)-P(-1); across rows A = R(-1)+R(+1)+4R(0), X likewise on
-    // D, Y = R(+1)-R(-1). The four cells x-1..x+2 of a row are shared by the two columns, so q
-    // and w^2 are formed once per cell.
-    float A[2][3], X[2][3], Y[2][3];
+  // iteration q: predictor of pair q, which completes the sums of pair q - 1, and from q = 3 on
+  // corrector and update of the output pair q - 1
+#pragma unroll 1
+  for (int q = 1; q <= nstage - 2; ++q) {
+    if (!arrive_wait(q + 1)) {
+      tm_wait_stores();
+      if (lane == 0) bulk_wait_all();
+      return false;
+    }
+    const TE* sp0 = pring + unsigned(q) % unsigned(SP) * (2 * PPL) + po;
+    const TE* su0 = uring + unsigned(q) % unsigned(SU) * (2 * VPL) + uo;          // predictor pair q
+    const TE* sub = uring + unsigned(q - 1) % unsigned(SU) * (2 * VPL) + uo;      // output pair q - 1
+    const TE* sua = uring + unsigned(q + 1) % unsigned(SU) * (2 * VPL) + uo;      // pair q + 1
+    const int zp = start + dir * 2 * q;                                           // real plane of the pair's first
+    float comp[N][4], cfirst[N][4];
+    float2 pcen[N];
+    {
+      RowSide above, here;               // rows r - 1 and r as their lower neighbours see them
+      RowSums mid;
 #pragma unroll
-    for (int cy = -1; cy <= 1; ++cy) {
-      const TE* rp = ss + po + cy * SW;
-      const TE* rq = ss + uo + cy * SW;
-      const float2 pL = lds2(rp - 2), pC = lds2(rp), pR = lds2(rp + 2);
-      if (kCarry && cy == 0) cnx[0] = pC;
-      const float2 uL = lds2(rq - 2), uC = lds2(rq), uR = lds2(rq + 2);
-      const float2 vL = lds2(rq + UPL - 2), vC = lds2(rq + UPL), vR = lds2(rq + UPL + 2);
-      const float2 wL = lds2(rq + 2 * UPL - 2), wC = lds2(rq + 2 * UPL), wR = lds2(rq + 2 * UPL + 2);
-      if (kCarry && cy == 0) { cnx[1] = uC; cnx[2] = vC; cnx[3] = wC; }
-      const float pc4[4] = {pL.y, pC.x, pC.y, pR.x};
-      const float uc4[4] = {uL.y, uC.x, uC.y, uR.x};
-      const float vc4[4] = {vL.y, vC.x, vC.y, vR.x};
-      float wc4[4] = {wL.y, wC.x, wC.y, wR.x};
-      if (kBase && g.wb) {             // w = stored deviation + the column's base
-        const float* br = wbs + (ty + 1 + cy) * Tl::BW + 2 * tp;
-        const float2 bL = *reinterpret_cast<const float2*>(br), bC = *reinterpret_cast<const float2*>(br + 2),
-                     bR = *reinterpret_cast<const float2*>(br + 4);
-        wc4[0] = __fadd_rn(wc4[0], bL.y); wc4[1] = __fadd_rn(wc4[1], bC.x);
-        wc4[2] = __fadd_rn(wc4[2], bC.y); wc4[3] = __fadd_rn(wc4[3], bR.x);
-      }
-      float q4[4], w24[4];
+      for (int j = -1; j <= N; ++j) {
+        float2 p3[3], u3[3], v3[3], w3[3];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        w24[j] = wc4[j] * wc4[j];
-        q4[j] = __fmaf_rn(-1.5f, __fmaf_rn(uc4[j], uc4[j], __fmaf_rn(vc4[j], vc4[j], w24[j])), pc4[j]);
-      }
+        for (int c = 0; c < 3; ++c) {
+          const TE* qp = sp0 + j * SW + c - 1;
+          const TE* qu = su0 + j * SW + c - 1;
+          p3[c] = make_float2(lds1(qp), lds1(qp + PPL));
+          u3[c] = ldu(qu);
+          v3[c] = ldu(qu + UPL);
+          w3[c] = ldu(qu + 2 * UPL);
+        }
+        if (j >= 0 && j < N) {
+          pcen[j] = p3[1];
+          const uint32_t ta = tm_slot(q) + 2 * j;
+          tm_store(ta, u3[1]);
+          tm_store(ta + 2 * N, v3[1]);
+          tm_store(ta + 4 * N, w3[1]);
+        }
+        if (kBase && g.wb)               // w = stored deviation + the column's base
 #pragma unroll
-      for (int col = 0; col < 2; ++col) {
-        float P[3][3];   // [cx+1][k]
-#pragma unroll
-        for (int cx = -1; cx <= 1; ++cx) {
-          const int j = col + 1 + cx;
-          const float u = uc4[j], v = vc4[j], w = wc4[j];
-          float P0, P1;
-          if (cx == 0 && cy == 0) {
-            P0 = q4[j];
-            P1 = w;
-          } else if (cx == 0 || cy == 0) {
-            const float Bv = cy == 0 ? u : v;
-            const float s3 = 3.0f * float(cx + cy);
-            P0 = __fmaf_rn(Bv, __fmaf_rn(Bv, 4.5f, s3), q4[j]);
-            P1 = w * __fmaf_rn(Bv, s3, 1.0f);
-          } else {
-            const float a1 = __fmaf_rn(v, float(cx * cy), u);
-            const float s3 = 3.0f * float(cx);
-            P0 = __fmaf_rn(a1, __fmaf_rn(a1, 4.5f, s3), q4[j]);
-            P1 = w * __fmaf_rn(a1, s3, 1.0f);
+          for (int c = 0; c < 3; ++c) w3[c] = add2(w3[c], f2(wbs[(ty + 1 + j) * Tl::BW + tx + c]));
+        const RowSums row = row_sums(p3, u3, v3, w3);
+        if (j >= 1) {
+          const int r = j - 1;
+          const RowSide below = row_side<1>(row);
+          // row-factored weights w(cx)w(cy) = {4,1,1}x{4,1,1}/36: A, X (cx moment), Y (cy moment)
+          float2 A[3], X[3], Y[3];
+          A[0] = fma2(f2(4.0f), mid.R0, add2(above.R0, below.R0));
+          A[1] = fma2(f2(4.0f), mid.Rz, add2(above.Rz, below.Rz));
+          A[2] = fma2(f2(4.0f), mid.Rw, add2(above.Rw, below.Rw));
+          X[0] = fma2(f2(4.0f), mid.D0, add2(above.D0, below.D0));
+          X[1] = fma2(f2(4.0f), mid.Dz, add2(above.Dz, below.Dz));
+          X[2] = fma2(f2(4.0f), mid.Dw, add2(above.Dw, below.Dw));
+          Y[0] = sub2(below.R0, above.R0);
+          Y[1] = sub2(below.Rz, above.Rz);
+          Y[2] = sub2(below.Rw, above.Rw);
+          if (min(zp, zp + dir) < 0 || max(zp, zp + dir) >= g.L) {
+            // seam planes (CTA-uniform): a wrapped plane adds the pressure jump to p on its
+            // non-wall cells, i.e. the jump times their weight sums (raw units, x36)
+            auto jump = [&](int z) { return z < 0 ? k.pin : (z >= g.L ? -k.pin : 0.0f); };
+            const float2 off = make_float2(jump(zp), jump(zp + dir));
+            const ColCoef<float> c = coef(r);
+            A[0] = fma2(off, f2(__fmaf_rn(-36.f, c.ws0, 36.f)), A[0]);
+            X[0] = fma2(off, f2(-36.f * c.wsx), X[0]);
+            Y[0] = fma2(off, f2(-36.f * c.wsy), Y[0]);
           }
-          P[cx + 1][0] = P0; P[cx + 1][1] = P1; P[cx + 1][2] = w24[j];
-        }
+          // True sums are A0/36, dir A1/12, A2/8. A plane is the march-next neighbour of the plane
+          // before it, itself, and the march-previous neighbour of the plane after: with
+          // e = (A0 + A2)/6 and h = A1/6 the shares are e + h (next), (2/3) A0 (self) and e - h
+          // (previous); for the z-moment h - e (previous), none (self) and e + h (next), times dir.
+          float2 s[3], d[3];
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          const float Rq = __fmaf_rn(4.0f, P[1][q], P[0][q] + P[2][q]);
-          const float Dq = P[2][q] - P[0][q];
-          if (cy == -1) { A[col][q] = Rq; X[col][q] = Dq; Y[col][q] = Rq; }
-          else if (cy == 0) { A[col][q] = __fmaf_rn(4.0f, Rq, A[col][q]); X[col][q] = __fmaf_rn(4.0f, Dq, X[col][q]); }
-          else { A[col][q] += Rq; X[col][q] += Dq; Y[col][q] = Rq - Y[col][q]; }
+          for (int i = 0; i < 3; ++i) {
+            const float2(&m)[3] = i == 0 ? A : (i == 1 ? X : Y);
+            const float2 e = fma2(m[2], f2(1.0f / 48.0f), mul2(m[0], f2(1.0f / 216.0f)));
+            s[i] = fma2(m[1], f2(h6), e);
+            d[i] = fma2(m[1], f2(-h6), e);
+          }
+          // Each cell sums its two neighbour planes' shares first (a commutative add) and then
+          // fuses its own plane's share, so its FP32 result depends neither on the march
+          // direction nor on how the pipe is split into chunks and pairs. That makes batched and
+          // served results equal to a solve stepped alone, bit for bit.
+          const float2 self[3] = {A[0], X[0], Y[0]};
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            cfirst[r][i] = cl[r][i];
+            comp[r][i] = __fmaf_rn(sh[r][i], 1.0f / 54.0f, __fadd_rn(dl[r][i], s[i].x));
+            cl[r][i] = __fmaf_rn(self[i].x, 1.0f / 54.0f, __fadd_rn(dh[r][i], s[i].y));
+          }
+          cfirst[r][3] = cl[r][3];
+          comp[r][3] = __fsub_rn(s[0].x, dl[r][0]);
+          cl[r][3] = __fsub_rn(s[0].y, dh[r][0]);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            sh[r][i] = self[i].y;
+            dl[r][i] = d[i].x;
+            dh[r][i] = d[i].y;
+          }
         }
+        if (j >= 0) above = here;
+        mid = row;
+        here = row_side<-1>(row);
       }
     }
-    // True sums are A0'/36, dir A1'/12, A2'/8 (P1 and P2 were formed as P1/3 and P2/4.5).
-    // Plane ma is the march-next neighbour of output ma-1 (completed here), itself, and the
-    // march-previous neighbour of ma+1: with e = (A0 + A2)/6 and h = A1/6 the shares are
-    // e + h (next), (2/3) A0 (self) and e - h (previous); for the z-moment h - e (previous),
-    // none (self) and e + h (next), times dir.
-    float cmp[4][2];
-    if (sp < 0 || sp >= g.L) {         // seam plane (CTA-uniform): the pressure jump's share
+    if (q >= 3) {
+      tm_wait_stores();
+      const int zo = zp - 2 * dir;                           // real plane of the output pair's first
+      ColCoef<float> cc[N];
 #pragma unroll
-      for (int col = 0; col < 2; ++col) {
-        A[col][0] = __fmaf_rn(off, n0[col], A[col][0]);
-        X[col][0] = __fmaf_rn(off, nx[col], X[col][0]);
-        Y[col][0] = __fmaf_rn(off, ny[col], Y[col][0]);
+      for (int r = 0; r < N; ++r) cc[r] = ColCoef<float>{0.f, 0.f, 0.f, 1.f};
+      if (!plain)
+#pragma unroll
+        for (int r = 0; r < N; ++r) cc[r] = coef(r);
+      float2 wg[N];
+      if (kBase)
+#pragma unroll
+        for (int r = 0; r < N; ++r)
+          wg[r] = f2(g.wgt && x < g.lxp && y0 + r < g.ly ? g.wgt[(y0 + r) * g.lxp + x] : 0.0f);
+      if (lane == 0) bulk_wait_read();                       // the previous pair has left the staging
+      __syncwarp();
+      auto put = [&](int f, int r, float2 val) {
+        val = mul2(val, f2(cc[r].fluid));                    // wall columns get zero
+        TE* o = sto + f * N * 32 + r * wcols;
+        if constexpr (kBase) {
+          // two cells share a hash word: the even column's lane forms the first plane's, the odd
+          // column's the second plane's
+          const bool odd = x & 1;
+          const uint32_t cell = (uint32_t(zo + (odd ? dir : 0)) * uint32_t(g.ly) + uint32_t(y0 + r)) * uint32_t(g.lxp)
+                                + (uint32_t(x) & ~1u);
+          const uint32_t mine = hash32(((cell << 2) | uint32_t(f)) ^ seed);
+          const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
+          o[0] = sr_half(val.x, odd ? other >> 16 : mine);
+          o[4 * N * 32] = sr_half(val.y, odd ? mine >> 16 : other);
+        } else {
+          o[0] = val.x;
+          o[4 * N * 32] = val.y;
+        }
+      };
+#pragma unroll
+      for (int r = 0; r < N; ++r)
+        put(0, r, add2(fma2(pc[r], f2(cc[r].ws0), make_float2(cfirst[r][0], comp[r][0])), f2(-gauge)));
+#pragma unroll
+      for (int f = 0; f < 3; ++f) {
+        const TE* b = sub + f * UPL;
+        float2 za1[N], c0[N], h1[N], h2[N];                  // own columns of pairs q, q - 1, q - 2, q - 3
+        tm_load(za1, tm_slot(q) + f * 2 * N);
+        tm_load(c0, tm_slot(q - 1) + f * 2 * N);
+        tm_load(h1, tm_slot(q - 2) + f * 2 * N);
+        tm_load(h2, tm_slot(q - 3) + f * 2 * N);
+        float2 c[N + 2 * R];                                 // rows -R .. N + R - 1 of the own column
+#pragma unroll
+        for (int j = -R; j < N + R; ++j)
+          if (j < 0 || j >= N) c[j + R] = ldu(b + j * SW);
+        tm_wait_loads(za1, c0, h1, h2);
+#pragma unroll
+        for (int r = 0; r < N; ++r) c[r + R] = c0[r];
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+          const TE* t = b + r * SW;
+          const float2 za2 = ldu(sua + f * UPL + r * SW);
+          const float2 t1 = add2(add2(add2(ldu(t - D1), ldu(t + D1)), add2(c[r + R - D1], c[r + R + D1])),
+                                 add2(h1[r], za1[r]));
+          const float2 t2 = add2(add2(add2(ldu(t - 2 * D1), ldu(t + 2 * D1)),
+                                      add2(c[r + R - 2 * D1], c[r + R + 2 * D1])),
+                                 add2(h2[r], za2));
+          const float2 cm = make_float2(cfirst[r][f == 2 ? 3 : 1 + f], comp[r][f == 2 ? 3 : 1 + f]);
+          const float2 mom = f == 2 ? cm : fma2(pc[r], f2(f == 0 ? cc[r].wsx : cc[r].wsy), cm);
+          // FP16 storage updates the stored deviation of w: the force's term becomes the column's
+          // share of the step of the base (tb fz included), see launch_wgt
+          const float2 tf = kBase && f == 2 && g.wgt ? wg[r] : f2(__fmul_rn(k.tb, f == 0 ? k.fx : (f == 1 ? k.fy : k.fz)));
+          put(1 + f, r, fma2(f2(kK1), t1, fma2(f2(kK2), t2, fma2(f2(kK0), c0[r],
+                         fma2(f2(f == 2 ? ktz : k.tb), mom, tf)))));
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_4d(tmap_out, stg, org.x + wx, org.y + wy, zo, 0);
+        // the chunk's plane count may be odd
+        if (2 * q - 1 - R < nout) tma_store_4d(tmap_out, stg + 4 * N * 32, org.x + wx, org.y + wy, zo + dir, 0);
+        bulk_commit();
       }
     }
 #pragma unroll
-    for (int col = 0; col < 2; ++col) {
-      const float A0 = A[col][0], X0 = X[col][0], Y0 = Y[col][0];
-      const float eA = __fmaf_rn(A[col][2], 1.0f / 48.0f, __fmul_rn(A0, 1.0f / 216.0f));
-      const float eX = __fmaf_rn(X[col][2], 1.0f / 48.0f, __fmul_rn(X0, 1.0f / 216.0f));
-      const float eY = __fmaf_rn(Y[col][2], 1.0f / 48.0f, __fmul_rn(Y0, 1.0f / 216.0f));
-      // e + h and e - h with h = A1 h6, each one fused rounding
-      const float sA = __fmaf_rn(A[col][1], h6, eA), dA = __fmaf_rn(A[col][1], -h6, eA);
-      const float sX = __fmaf_rn(X[col][1], h6, eX), dX = __fmaf_rn(X[col][1], -h6, eX);
-      const float sY = __fmaf_rn(Y[col][1], h6, eY), dY = __fmaf_rn(Y[col][1], -h6, eY);
-      cmp[0][col] = __fmaf_rn(s1[0][col], 1.0f / 54.0f, __fadd_rn(b2[0][col], sA));
-      cmp[1][col] = __fmaf_rn(s1[1][col], 1.0f / 54.0f, __fadd_rn(b2[1][col], sX));
-      cmp[2][col] = __fmaf_rn(s1[2][col], 1.0f / 54.0f, __fadd_rn(b2[2][col], sY));
-      cmp[3][col] = __fadd_rn(b2[3][col], sA);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) b2[q][col] = b1[q][col];
-      b1[0][col] = dA;
-      b1[1][col] = dX;
-      b1[2][col] = dY;
-      b1[3][col] = -dA;
-      s1[0][col] = A0;
-      s1[1][col] = X0;
-      s1[2][col] = Y0;
-    }
-    comp0 = make_float2(cmp[0][0], cmp[0][1]);
-    comp1 = make_float2(cmp[1][0], cmp[1][1]);
-    comp2 = make_float2(cmp[2][0], cmp[2][1]);
-    comp3 = make_float2(cmp[3][0], cmp[3][1]);
-  };
-
-  // own columns of march plane jo (for the history)
-  auto own = [&](int jo, float2& uc, float2& vc, float2& wc) {
-    const TE* so = ring + slot_of(jo) * SLOT;
-    uc = lds2(so + uo); vc = lds2(so + uo + UPL); wc = lds2(so + uo + 2 * UPL);
-  };
-
-  // corrector and update of output march plane jo; hist slot ROT holds plane jo-4 and is then
-  // overwritten with plane jo
-  auto output = [&](int jo, auto rot_c) {
-    constexpr int ROT = decltype(rot_c)::value;
-    const TE* so = ring + slot_of(jo) * SLOT;
-    const TE* sa1 = ring + slot_of(jo + D1) * SLOT;   // march planes ahead
-    const TE* sa2 = ring + slot_of(jo + 2 * D1) * SLOT;
-    float2 pc, uc, vc, wc;
-    if (kCarry) {
-      pc = cen[0]; uc = cen[1]; vc = cen[2]; wc = cen[3];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) cen[q] = cnx[q];
-    } else {
-      pc = lds2(so + po);
-      uc = lds2(so + uo); vc = lds2(so + uo + UPL); wc = lds2(so + uo + 2 * UPL);
-    }
-    // u_new = K1 t1 + K2 t2 + K0 u + tb m* + tb F
-    auto update = [&](int f, float2 c, float2 zb1, float2 zb2, float2 mom, float tm, float2 tf) {
-      const TE* q = so + uo + f * UPL;
-      const float2 za1 = lds2(sa1 + uo + f * UPL), za2 = lds2(sa2 + uo + f * UPL);
-      const float2 t1 = F::add(F::add(F::add(lds2(q - D1), lds2(q + D1)),
-                                      F::add(lds2(q - D1 * SW), lds2(q + D1 * SW))),
-                               F::add(zb1, za1));
-      const float2 t2 = F::add(F::add(F::add(lds2(q - 2 * D1), lds2(q + 2 * D1)),
-                                      F::add(lds2(q - 2 * D1 * SW), lds2(q + 2 * D1 * SW))),
-                               F::add(zb2, za2));
-      return F::fma(f2(kK1), t1, F::fma(f2(kK2), t2, F::fma(f2(kK0), c, F::fma(f2(tm), mom, tf))));
-    };
-    constexpr int H2 = (ROT + 2) & 3;                         // plane jo-2
-    const float2 rho = F::add(F::fma(pc, ws0, comp0), f2(-gauge));
-    const float2 us = F::fma(pc, wsx, comp1), vs = F::fma(pc, wsy, comp2);
-    const float2 un = update(0, uc, hu[H2], hu[ROT], us, k.tb, f2(__fmul_rn(k.tb, k.fx)));
-    const float2 vn = update(1, vc, hv[H2], hv[ROT], vs, k.tb, f2(__fmul_rn(k.tb, k.fy)));
-    // FP16 storage updates the stored deviation of w: the force's term becomes the column's share
-    // of the step of the base (tb fz included), see launch_wgt
-    const float2 wn = update(2, wc, hw[H2], hw[ROT], comp3, ktz,
-                             (kBase && g.wgt) ? wgt2 : f2(__fmul_rn(k.tb, k.fz)));
-    hu[ROT] = uc; hv[ROT] = vc; hw[ROT] = wc;
-    if (inside) {   // wall columns get zero (fl = 0)
-      if (fl.x != 0.f && fl.y != 0.f)
-        PairStore<TE>::put(outp, FS, rho, un, vn, wn, obase, seed);
-      else
-        PairStore<TE>::put(outp, FS, F::mul(rho, fl), F::mul(un, fl), F::mul(vn, fl),
-                           F::mul(wn, fl), obase, seed);
-    }
-    outp += ostep;
-  };
-
-  using I0 = std::integral_constant<int, 0>;
-  using I1 = std::integral_constant<int, 1>;
-  using I2 = std::integral_constant<int, 2>;
-  using I3 = std::integral_constant<int, 3>;
-  // ---- prologue (R = 4): planes 0..3 arrive; 4..5 enter the history; 6..7 also start the
-  // predictor sums of the first output
-#pragma unroll
-  for (int m = 0; m < 2 * R; ++m) {
-    if (!arrive_wait(m)) return false;
-    if (m >= 2 * R - 2) predictor(m - R + 1);
-    if (m >= R) {
-      float2 uc, vc, wc;
-      own(m - R, uc, vc, wc);
-      const int h = (m - R) & 3;
-      if (h == 0) { hu[0] = uc; hv[0] = vc; hw[0] = wc; }
-      else if (h == 1) { hu[1] = uc; hv[1] = vc; hw[1] = wc; }
-      else if (h == 2) { hu[2] = uc; hv[2] = vc; hw[2] = wc; }
-      else { hu[3] = uc; hv[3] = vc; hw[3] = wc; }
-    }
-    if (!release_produce(m)) return false;
+    for (int r = 0; r < N; ++r) pc[r] = pcen[r];
+    release(q - 1);
   }
-  if (kCarry)                          // the first output's centre pairs
-#pragma unroll
-    for (int q = 0; q < 4; ++q) cen[q] = cnx[q];
-  // ---- steady state, four planes per pass (the history period)
-  for (int m = 2 * R; m < niter; m += 4) {
-    if (!arrive_wait(m)) return false;
-    predictor(m - R + 1);
-    output(m - R, I0{});
-    if (!release_produce(m)) return false;
-    if (m + 1 >= niter) break;
-    if (!arrive_wait(m + 1)) return false;
-    predictor(m - R + 2);
-    output(m - R + 1, I1{});
-    if (!release_produce(m + 1)) return false;
-    if (m + 2 >= niter) break;
-    if (!arrive_wait(m + 2)) return false;
-    predictor(m - R + 3);
-    output(m - R + 2, I2{});
-    if (!release_produce(m + 2)) return false;
-    if (m + 3 >= niter) break;
-    if (!arrive_wait(m + 3)) return false;
-    predictor(m - R + 4);
-    output(m - R + 3, I3{});
-    if (!release_produce(m + 3)) return false;
-  }
+  if (lane == 0) bulk_wait_all();
   return true;
 }
 
 // One pipe, one step: CTA b marches (tile b % ntiles, chunk b / ntiles).
-template <int D1, int TY, bool PK, class TE>
-__global__ void __launch_bounds__(Step2Tile<D1, TY, TE>::THREADS, TY == 16 ? 2 : 1)
+template <int TY, class TE>
+__global__ void __launch_bounds__(Step2Tile<TY, TE>::THREADS, Step2Tile<TY, TE>::CTAS)
     fslbm_step2_kernel(const __grid_constant__ CUtensorMap tmap_p,
-                       const __grid_constant__ CUtensorMap tmap_uvw, const Step2Geom g,
+                       const __grid_constant__ CUtensorMap tmap_uvw,
+                       const __grid_constant__ CUtensorMap tmap_out, const Step2Geom g,
                        const StepConst<float> k) {
+  using Tl = Step2Tile<TY, TE>;
   extern __shared__ __align__(128) unsigned char smem[];
-  grid_launch_dependents();
+  uint32_t* tm_base = reinterpret_cast<uint32_t*>(smem + Tl::REL_OFFSET) + Tl::SU;
+  if (threadIdx.x < 32) tm_alloc<Tl::TM_COLS>(tm_base);
   grid_dependency_wait();
   if (threadIdx.x == 0 && blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
-  // centre pairs carried for FP32 storage (FP16 storage measured 3 % slower with them)
-  step2_march<D1, TY, PK, TE, std::is_same<TE, float>::value>(&tmap_p, &tmap_uvw, g, k, blockIdx.x % g.ntiles,
-                                                              blockIdx.x / g.ntiles, smem, false);
+  __syncthreads();
+  const uint32_t tmem = *tm_base;
+  step2_march<TY, TE>(&tmap_p, &tmap_uvw, &tmap_out, tmem, g, k, blockIdx.x % g.ntiles, blockIdx.x / g.ntiles, smem,
+                      false, 0);
+  grid_launch_dependents();   // not earlier: waiting CTAs of the next step would share this one's SMs
+  __syncthreads();
+  if (threadIdx.x < 32) tm_free<Tl::TM_COLS>(tmem);
 }
 
 }  // namespace fslbm

@@ -104,7 +104,6 @@ __global__ void __launch_bounds__(kThreads, sizeof(TS) == 8 ? 1 : 2)
   const int zb = chunk * g.chunk, ze = min(zb + g.chunk, g.L);
   const int t0 = zb - R, t1 = ze + R;
 
-  grid_launch_dependents();
   grid_dependency_wait();
   if (tid == 0) {
     if (blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
@@ -287,6 +286,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(TS) == 8 ? 1 : 2)
       out[3 * FS + o] = TS((wzs + k.dtddy * Lw * k.m + k.fz) * k.tb + wc * k.cc);
     }
   }
+  grid_launch_dependents();
 }
 
 }  // namespace fslbm

@@ -335,10 +335,10 @@ __global__ void __launch_bounds__(ColTile<D1, TY>::THREADS, 1)
                      const __grid_constant__ CUtensorMap tmap_uvw, const Step2Geom g,
                      const StepConst<double> k) {
   extern __shared__ __align__(128) unsigned char smem[];
-  grid_launch_dependents();
   grid_dependency_wait();
   if (threadIdx.x == 0 && blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
   col_march<D1, TY>(&tmap_p, &tmap_uvw, g, k, blockIdx.x % g.ntiles, blockIdx.x / g.ntiles, smem);
+  grid_launch_dependents();
 }
 
 }  // namespace fslbm
