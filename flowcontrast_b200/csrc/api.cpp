@@ -199,13 +199,13 @@ struct fslbm_solve {
   int cur = 0;
   uint8_t* d_mask = nullptr;
   void* d_colcoef = nullptr;
+  uint8_t* d_near = nullptr;       // masks per plane, FP32: code per cell, then per column (see step2_march)
   int2* d_tiles = nullptr;
   int ntiles = 0, chunk = 0, nchunks = 0;
   CUtensorMap maps[2];
   // FP32 column-pair kernel (even d1): tile height, persistent grid, two maps per buffer
   bool use2 = false;
   int ty2 = 32, grid2 = 0;
-  std::vector<int> tile_warps[3];  // per column-pair tile: warps holding fluid, [shape] 32 x 2, 16 x 4, 8 x 8
   CUtensorMap maps2p[2], maps2u[2], maps2o[2];
   DevCounters* d_counters = nullptr;
   fslbm_monitor* d_log = nullptr;
@@ -277,8 +277,8 @@ static int encode_pair_maps(const fslbm_solve* s, int ty, CUtensorMap mp[2], CUt
                                  : s->dtype == FSLBM_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                          : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   int sw2, ph, uh, hx2, hy2;
-  if (!step2_box(s->dtype, s->prm.d1, ty, &sw2, &ph, &uh, &hx2, &hy2))
-    return fslbm_set_error(FSLBM_ERR_ARG, "no column-pair kernel for d1 %d, tile height %d", s->prm.d1, ty);
+  if (!step2_box(s->dtype, s->K, ty, &sw2, &ph, &uh, &hx2, &hy2))
+    return fslbm_set_error(FSLBM_ERR_ARG, "no pair kernel for %d corrector taps, tile height %d", s->K, ty);
   cuuint64_t dims[4] = {cuuint64_t(s->lxp), cuuint64_t(s->ly), cuuint64_t(s->L), 4};
   cuuint64_t strides[3] = {cuuint64_t(s->lxp) * s->es, cuuint64_t(s->lxp) * s->ly * s->es,
                            cuuint64_t(field_stride(s)) * s->es};
@@ -401,14 +401,14 @@ struct Split {
 // iteration grows with its resident warps (32 x 8 tiles have 4, 32 x 16 have 8, 32 x 32 have 16):
 // 1.35 us for one 32 x 8 tile of FP32 against 2.85 us for a 32 x 32 tile, so few cells per SM want
 // small tiles (latency) and many cells the large one (fewer halo cells, more warps).
-static double split_us(int dtype, int ty, int per_sm, int sms, int L, int ntiles, int nch) {
+static double split_us(int dtype, int K, int ty, int per_sm, int sms, int L, int ntiles, int nch) {
   static const double f32[3][3] = {{1.35, 1.8, 2.45}, {1.7, 0, 0}, {2.85, 0, 0}};
   static const double f16[3][3] = {{1.93, 2.37, 3.2}, {2.45, 4.05, 0}, {3.94, 0, 0}};
   const int planes = (L + nch - 1) / nch;
   const int64_t ctas = int64_t(ntiles) * nch, waves = (ctas + int64_t(sms) * per_sm - 1) / (int64_t(sms) * per_sm);
   if (dtype == FSLBM_F64) return double(waves) * 1.3 * (planes + 4.8);
   const double tau = (dtype == FSLBM_F16 ? f16 : f32)[ty == 8 ? 0 : (ty == 16 ? 1 : 2)][per_sm - 1];
-  return double(waves) * (2.0 + tau * ((planes + 1) / 2 + 2));
+  return double(waves) * (2.0 + tau * ((planes + 1) / 2 + K));
 }
 
 // The split with the least modelled time over the tile heights of the solve's kernel (or
@@ -418,14 +418,14 @@ static Split choose_split(const fslbm_solve* s, int only_ty) {
   const int sms = s->ctx->sm_count, max_nch = s->dtype == FSLBM_F64 ? s->L : (s->L + 1) / 2;
   for (int ty : {32, 16, 8}) {
     int box[5];
-    if ((only_ty && ty != only_ty) || !step2_box(s->dtype, s->prm.d1, ty, box, box + 1, box + 2, box + 3, box + 4))
+    if ((only_ty && ty != only_ty) || !step2_box(s->dtype, s->K, ty, box, box + 1, box + 2, box + 3, box + 4))
       continue;
     const std::vector<int2> tiles = fluid_tiles(s, ty);
     const int nt = int(tiles.size());
-    for (int per_sm = 1; per_sm <= step2_occupancy(s->dtype, s->prm.d1, ty); ++per_sm)
+    for (int per_sm = 1; per_sm <= step2_occupancy(s->dtype, s->K, ty); ++per_sm)
       for (int waves = 1; waves <= 4; ++waves) {
         const int nch = std::max(1, std::min(int(int64_t(sms) * per_sm * waves / nt), max_nch));
-        const double us = split_us(s->dtype, ty, per_sm, sms, s->L, nt, nch);
+        const double us = split_us(s->dtype, s->K, ty, per_sm, sms, s->L, nt, nch);
         if (us < best.us) best = Split{ty, nch, us, tiles};
       }
   }
@@ -440,8 +440,8 @@ static int configure_kernel(fslbm_solve* s) {
   const char* et = std::getenv("FSLBM_TILE_Y");
   double cf[9];
   s->K = fd_coefficients(s->prm.fd_order, s->prm.blend, s->dtype != FSLBM_F64, cf);
-  // FP16 storage exists only in the column-pair kernel, which has the 2-tap corrector
-  s->use2 = step2_supported(s->dtype, s->prm.d1) && s->K == 2 && s->planes == 1 &&
+  // FP16 storage exists only in the pair kernel
+  s->use2 = step2_supported(s->dtype, s->prm.d1, s->K, s->planes > 1) &&
             (s->dtype == FSLBM_F16 || !(ek && std::atoi(ek) == 1));
   const int ety = et && s->dtype != FSLBM_F64 ? std::atoi(et) : 0;
   Split split;
@@ -449,8 +449,6 @@ static int configure_kernel(fslbm_solve* s) {
   else split.tiles = fluid_tiles(s, kTY);
   const std::vector<int2>& tiles = split.tiles;
   s->ty2 = split.ty;
-  for (auto& v : s->tile_warps) v.clear();
-  if (s->use2) tile_warp_counts(s, tiles, s->ty2, s->tile_warps);
   if (s->d_tiles) {
     ctx_free(s->ctx, s->d_tiles);
     s->bytes_device -= int64_t(s->ntiles) * sizeof(int2);
@@ -462,7 +460,7 @@ static int configure_kernel(fslbm_solve* s) {
   CUDA_TRY(cudaMemcpyAsync(s->d_tiles, tiles.data(), tiles.size() * sizeof(int2),
                            cudaMemcpyHostToDevice, s->ctx->stream));
   if (s->use2) {
-    CUDA_TRY(step2_prepare(s->dtype, s->prm.d1, s->ty2));
+    CUDA_TRY(step2_prepare(s->dtype, s->K, s->planes > 1, s->ty2));
     s->grid2 = s->ntiles * split.nch;
   } else {
     CUDA_TRY(step_prepare(s->dtype, s->prm.d1, s->K));
@@ -551,7 +549,7 @@ static void choose_chunks(fslbm_solve* s) {
 static void free_solve(fslbm_solve* s) {
   if (!s) return;
   cudaSetDevice(s->ctx->device);
-  void* ptrs[] = {s->state[0], s->state[1], s->d_mask, s->d_colcoef, s->d_tiles, s->d_ghosts, s->d_counters,
+  void* ptrs[] = {s->state[0], s->state[1], s->d_mask, s->d_colcoef, s->d_near, s->d_tiles, s->d_ghosts, s->d_counters,
                   s->d_log, s->d_gauge, s->d_err, s->d_scratch, s->d_stats, s->d_prof,
                   s->d_stage, s->d_plane, s->d_wbase, s->d_wgt};
   for (void* p : ptrs) ctx_free(s->ctx, p);
@@ -725,6 +723,14 @@ extern "C" int fslbm_solve_create(fslbm_ctx* ctx, const fslbm_domain* dom, const
     auto cc = cell_coefs<float>(s);
     if ((e = dalloc(s, &s->d_colcoef, cc.size() * sizeof(cc[0])))) return fail("colcoef");
     e = cudaMemcpyAsync(s->d_colcoef, cc.data(), cc.size() * sizeof(cc[0]), cudaMemcpyHostToDevice, st);
+    std::vector<uint8_t> near(cc.size() + plane, 2);   // per cell, then per column over all planes
+    for (size_t j = 0; j < cc.size(); ++j) {
+      if (s->mask[j] == kWall) continue;
+      near[j] = cc[j].ws0 != 0.0f ? 1 : 0;
+      near[cc.size() + j % plane] = 1;
+    }
+    if (!e) e = dalloc(s, &s->d_near, near.size());
+    if (!e) e = cudaMemcpyAsync(s->d_near, near.data(), near.size(), cudaMemcpyHostToDevice, st);
     if (!e) e = cudaStreamSynchronize(st);
   } else if (dtype == FSLBM_F64) {
     auto cc = column_coefs<double>(s);
@@ -908,8 +914,8 @@ extern "C" int fslbm_solve_footprint(const fslbm_domain* dom, fslbm_dtype dtype,
   const int64_t cc = dtype == FSLBM_F64 ? int64_t(sizeof(ColCoef<double>)) : int64_t(sizeof(ColCoef<float>));
   const int64_t tiles = ((lxp + kTX - 1) / kTX) * ((dom->ly + kTY - 1) / kTY) * int64_t(sizeof(int2));
   const int64_t masks = dom->mask_planes > 1
-                            ? cs * dom->lz * (1 + int64_t(dtype == FSLBM_F64 ? sizeof(CellCoef<double>)
-                                                                                : sizeof(CellCoef<float>)))
+                            ? cs + cs * dom->lz * (1 + int64_t(dtype == FSLBM_F64 ? sizeof(CellCoef<double>)
+                                                                                : sizeof(CellCoef<float>) + 1))
                             : cs + cs * cc;
   const int64_t wtabs = dtype == FSLBM_F16 ? 2 * cs * int64_t(sizeof(float)) : 0;
   *bytes = 2 * 4 * fs * es + masks + tiles + wtabs + int64_t(sizeof(DevCounters)) +
@@ -981,7 +987,7 @@ static int enqueue_steps(fslbm_solve* s, int64_t nsteps) {
   a.ntiles = s->ntiles; a.chunk = s->chunk; a.nchunks = s->nchunks;
   a.tiles = s->d_tiles; a.mask = s->d_mask; a.colcoef = s->d_colcoef;
   a.err = s->d_err; a.counters = s->d_counters; a.mask_planes = s->planes;
-  a.wb = s->d_wbase; a.wgt = s->d_wgt;
+  a.wb = s->d_wbase; a.wgt = s->d_wgt; a.near = s->d_near;
   fill_constants(s, a);
   MonitorLaunch m{};
   m.dtype = s->dtype; m.mask = s->d_mask;
@@ -1007,7 +1013,7 @@ static int enqueue_steps(fslbm_solve* s, int64_t nsteps) {
       CUDA_TRY(cudaEventRecord(s->tev[s->tev_used], st));
     }
     if (s->use2) {
-      Step2Launch b2{s->prm.d1, s->ty2, &s->maps2p[s->cur], &s->maps2u[s->cur], &s->maps2o[1 - s->cur], s->grid2};
+      Step2Launch b2{s->ty2, &s->maps2p[s->cur], &s->maps2u[s->cur], &s->maps2o[1 - s->cur], s->grid2};
       CUDA_TRY(launch_step2(a, b2, st));
     } else {
       CUDA_TRY(launch_step(a, st));
@@ -1412,6 +1418,12 @@ static int64_t item_cost(const fslbm_solve* s, const std::vector<int> (&warps)[3
   return int64_t(nout + 4 * s->prm.d1) * (warps[shape][tile] + 2);
 }
 
+// Whether a member fits the batched kernel: the pair kernel with 2 corrector taps and one
+// cross-section, no ghost refill between steps.
+static bool batchable(const fslbm_solve* s) {
+  return s->use2 && s->K == 2 && s->planes == 1 && s->dtype != FSLBM_F64 && s->nghost == 0;
+}
+
 // Resident CTAs of the batched kernel: one per SM for 32 x 32 tiles, two for 32 x 16 tiles.
 static int batch_slots(const fslbm_batch* b) {
   return b->ctx->sm_count * step2_occupancy(b->members[0]->dtype, 2, b->ty);
@@ -1437,8 +1449,7 @@ static int batch_upload(fslbm_batch* b) {
   // (stride, corrector order or storage type changed) is refused
   for (int i = 0; i < n; ++i) {
     const fslbm_solve* s = b->members[i];
-    if (!(s->use2 && s->prm.d1 == 2 && s->dtype == b->members[0]->dtype && s->dtype != FSLBM_F64 &&
-          s->nghost == 0))
+    if (!(batchable(s) && s->dtype == b->members[0]->dtype))
       return fslbm_set_error(FSLBM_ERR_STATE, "batch_step: member %d was reconfigured and no longer "
                              "fits the batched kernel; create a new batch", i);
   }
@@ -1639,8 +1650,7 @@ extern "C" int fslbm_batch_create(fslbm_ctx* ctx, fslbm_solve* const* solves, in
     b->stop.push_back(-1);
     b->m_chunk.push_back(128);
     b->m_shape.push_back(1);
-    fast = fast && solves[i]->use2 && solves[i]->prm.d1 == 2 && solves[i]->dtype != FSLBM_F64 &&
-           solves[i]->dtype == solves[0]->dtype && solves[i]->nghost == 0;
+    fast = fast && batchable(solves[i]) && solves[i]->dtype == solves[0]->dtype;
   }
   b->fast = fast;
   default_tiling(b);

@@ -48,6 +48,7 @@ struct StepLaunch {
   int mask_planes;           // 0/1: extruded cross-section; L: a mask (and CellCoef) per plane
   const float* wb;           // FP16 storage: per-column base of w and its step share, else null
   const float* wgt;
+  const uint8_t* near;       // masks per plane, FP32: code per cell (0 fluid, 1 beside a wall, 2 wall), else null
   // constants in double; converted to the compute type by the launcher
   double tb, cc, pin, dtddy, m, c0, c1, c2, fx, fy, fz;
   double ch[6];              // corrector coefficients c3..c8
@@ -59,20 +60,20 @@ bool step_supported(int dtype, int d1, int K);
 cudaError_t step_prepare(int dtype, int d1, int K);   // sets the dynamic shared memory attribute
 cudaError_t launch_step(const StepLaunch& a, cudaStream_t st);
 
-// Column-pair kernel (FP32 / FP16 storage, d1 = 2) and FP64 column kernel (d1 = 2, 32 x 16
-// tiles): two tensor maps per input state (p box with a one-cell halo, u,v,w box with the
-// corrector halo).
+// Pair kernel (d1 = 2; FP32 with 2 or 3 corrector taps, one cross-section or one per plane; FP16
+// storage with 2 taps) and FP64 column kernel (d1 = 2, 2 taps, 32 x 16 tiles): two tensor maps per
+// input state (p box with a one-cell halo, u,v,w box with the corrector halo).
 struct Step2Launch {
-  int d1, ty;                // corrective stride, tile height (8, 16 or 32)
+  int ty;                    // tile height (8, 16 or 32)
   const CUtensorMap* map_p;
   const CUtensorMap* map_uvw;
   const CUtensorMap* map_out;  // output state, box of one warp's cells (not the FP64 kernel)
   int grid;
 };
-bool step2_supported(int dtype, int d1);
-bool step2_box(int dtype, int d1, int ty, int* sw, int* ph, int* uh, int* hx, int* hy);
-int step2_occupancy(int dtype, int d1, int ty);   // CTAs per SM the kernel is built for
-cudaError_t step2_prepare(int dtype, int d1, int ty);
+bool step2_supported(int dtype, int d1, int K, bool mp);   // mp: a mask per plane
+bool step2_box(int dtype, int K, int ty, int* sw, int* ph, int* uh, int* hx, int* hy);
+int step2_occupancy(int dtype, int K, int ty);   // CTAs per SM the kernel is built for
+cudaError_t step2_prepare(int dtype, int K, bool mp, int ty);
 cudaError_t launch_step2(const StepLaunch& a, const Step2Launch& b, cudaStream_t st);
 
 struct MonitorLaunch {

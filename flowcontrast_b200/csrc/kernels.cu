@@ -123,57 +123,68 @@ cudaError_t launch_step(const StepLaunch& a, cudaStream_t st) {
 // ------------------------------------------------------------------------------------------
 // column-pair kernel (FP32 / FP16 storage) and FP64 column kernel dispatch
 // ------------------------------------------------------------------------------------------
-bool step2_supported(int dtype, int d1) {
-  return (dtype == FSLBM_F32 || dtype == FSLBM_F16 || dtype == FSLBM_F64) && d1 == 2;
+bool step2_supported(int dtype, int d1, int K, bool mp) {
+  if (d1 != 2) return false;
+  if (dtype == FSLBM_F32) return K == 2 || K == 3;
+  return (dtype == FSLBM_F16 || dtype == FSLBM_F64) && K == 2 && !mp;
 }
 
-// Calls fn.template operator()<TY, TE>() for the column-pair tile of (dtype, ty).
-template <class F> static cudaError_t with_step2(int dtype, int ty, F&& fn) {
-  if (dtype == FSLBM_F32) {
-    if (ty == 32) return fn.template operator()<32, float>();
-    if (ty == 16) return fn.template operator()<16, float>();
-    if (ty == 8) return fn.template operator()<8, float>();
-  } else if (dtype == FSLBM_F16) {
-    if (ty == 32) return fn.template operator()<32, __half>();
-    if (ty == 16) return fn.template operator()<16, __half>();
-    if (ty == 8) return fn.template operator()<8, __half>();
+// Calls fn.template operator()<TY, TE, K, MP>() for the pair kernel of (dtype, K, mask per plane)
+// with tile height ty.
+template <class F> static cudaError_t with_step2(int dtype, int K, bool mp, int ty, F&& fn) {
+  if (dtype == FSLBM_F32 && K == 2 && !mp) {
+    if (ty == 32) return fn.template operator()<32, float, 2, false>();
+    if (ty == 16) return fn.template operator()<16, float, 2, false>();
+    if (ty == 8) return fn.template operator()<8, float, 2, false>();
+  } else if (dtype == FSLBM_F32 && K == 2) {
+    if (ty == 32) return fn.template operator()<32, float, 2, true>();
+    if (ty == 16) return fn.template operator()<16, float, 2, true>();
+    if (ty == 8) return fn.template operator()<8, float, 2, true>();
+  } else if (dtype == FSLBM_F32 && K == 3 && !mp) {     // the window of 32 x 32 tiles exceeds shared memory
+    if (ty == 16) return fn.template operator()<16, float, 3, false>();
+    if (ty == 8) return fn.template operator()<8, float, 3, false>();
+  } else if (dtype == FSLBM_F32 && K == 3) {
+    if (ty == 16) return fn.template operator()<16, float, 3, true>();
+    if (ty == 8) return fn.template operator()<8, float, 3, true>();
+  } else if (dtype == FSLBM_F16 && K == 2 && !mp) {
+    if (ty == 32) return fn.template operator()<32, __half, 2, false>();
+    if (ty == 16) return fn.template operator()<16, __half, 2, false>();
+    if (ty == 8) return fn.template operator()<8, __half, 2, false>();
   }
   return cudaErrorInvalidValue;
 }
 
-bool step2_box(int dtype, int d1, int ty, int* sw, int* ph, int* uh, int* hx, int* hy) {
-  if (d1 != 2) return false;
+bool step2_box(int dtype, int K, int ty, int* sw, int* ph, int* uh, int* hx, int* hy) {
   if (dtype == FSLBM_F64) {          // the FP64 column kernel: 32 x 16 tiles only
     using Tl = ColTile<2, 16>;
     if (ty != 16) return false;
     *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
     return true;
   }
-  return with_step2(dtype, ty, [&]<int TY, class TE>() {
-           using Tl = Step2Tile<TY, TE>;
+  return with_step2(dtype, K, false, ty, [&]<int TY, class TE, int KK, bool MP>() {
+           using Tl = Step2Tile<TY, TE, KK>;
            *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
            return cudaSuccess;
          }) == cudaSuccess;
 }
 
-int step2_occupancy(int dtype, int, int ty) {
+int step2_occupancy(int dtype, int K, int ty) {
   int n = 1;
-  (void)with_step2(dtype, ty, [&]<int TY, class TE>() {
-    n = Step2Tile<TY, TE>::CTAS;
+  (void)with_step2(dtype, K, false, ty, [&]<int TY, class TE, int KK, bool MP>() {
+    n = Step2Tile<TY, TE, KK>::CTAS;
     return cudaSuccess;
   });
   return n;
 }
 
-cudaError_t step2_prepare(int dtype, int d1, int ty) {
-  if (d1 != 2) return cudaErrorInvalidValue;
+cudaError_t step2_prepare(int dtype, int K, bool mp, int ty) {
   if (dtype == FSLBM_F64)
     return ty != 16 ? cudaErrorInvalidValue
                     : cudaFuncSetAttribute(fslbm_col_kernel<2, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            int(ColTile<2, 16>::SMEM_BYTES));
-  return with_step2(dtype, ty, [&]<int TY, class TE>() {
-    return cudaFuncSetAttribute(fslbm_step2_kernel<TY, TE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(Step2Tile<TY, TE>::SMEM_BYTES));
+  return with_step2(dtype, K, mp, ty, [&]<int TY, class TE, int KK, bool MP>() {
+    return cudaFuncSetAttribute(fslbm_step2_kernel<TY, TE, KK, MP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(Step2Tile<TY, TE, KK>::SMEM_BYTES));
   });
 }
 
@@ -182,26 +193,26 @@ cudaError_t launch_step2(const StepLaunch& a, const Step2Launch& b, cudaStream_t
   g.lxp = a.lxp; g.ly = a.ly; g.L = a.L; g.ntiles = a.ntiles; g.nchunks = b.grid / a.ntiles;
   g.tiles = a.tiles; g.mask = a.mask; g.colcoef = a.colcoef; g.out = a.out;
   g.gauge = a.gauge; g.err = a.err;
-  g.wb = a.wb; g.wgt = a.wgt;
+  g.wb = a.wb; g.wgt = a.wgt; g.near = a.near;
   g.step_counter = a.counters ? &a.counters->steps : nullptr;
   g.step_no = unsigned(a.step_no);
-  StepConst<float> k;
+  StepConst<float> k{};
   k.tb = float(a.tb); k.cc = float(a.cc); k.pin = float(a.pin); k.dtddy = float(a.dtddy);
   k.m = float(a.m); k.c0 = float(a.c0); k.c1 = float(a.c1); k.c2 = float(a.c2);
+  for (int j = 0; j < 6; ++j) k.ch[j] = float(a.ch[j]);
   k.fx = float(a.fx); k.fy = float(a.fy); k.fz = float(a.fz);
-  if (b.d1 != 2) return cudaErrorInvalidValue;
+  if (a.d1 != 2) return cudaErrorInvalidValue;
   if (a.dtype == FSLBM_F64) {
     if (b.ty != 16) return cudaErrorInvalidValue;
-    StepConst<double> kd;
+    StepConst<double> kd{};
     kd.tb = a.tb; kd.cc = a.cc; kd.pin = a.pin; kd.dtddy = a.dtddy; kd.m = a.m;
     kd.c0 = a.c0; kd.c1 = a.c1; kd.c2 = a.c2; kd.fx = a.fx; kd.fy = a.fy; kd.fz = a.fz;
-    for (int j = 0; j < 6; ++j) kd.ch[j] = a.ch[j];
     return launch_chained(fslbm_col_kernel<2, 16>, b.grid, ColTile<2, 16>::THREADS,
                           ColTile<2, 16>::SMEM_BYTES, st, *b.map_p, *b.map_uvw, g, kd);
   }
-  return with_step2(a.dtype, b.ty, [&]<int TY, class TE>() {
-    using Tl = Step2Tile<TY, TE>;
-    return launch_chained(fslbm_step2_kernel<TY, TE>, b.grid, Tl::THREADS, Tl::SMEM_BYTES, st, *b.map_p,
+  return with_step2(a.dtype, a.K, a.mask_planes > 1, b.ty, [&]<int TY, class TE, int KK, bool MP>() {
+    using Tl = Step2Tile<TY, TE, KK>;
+    return launch_chained(fslbm_step2_kernel<TY, TE, KK, MP>, b.grid, Tl::THREADS, Tl::SMEM_BYTES, st, *b.map_p,
                           *b.map_uvw, *b.map_out, g, k);
   });
 }
@@ -462,8 +473,8 @@ __global__ void __launch_bounds__(Step2Tile<TY, TE>::THREADS, Step2Tile<TY, TE>:
 }
 
 cudaError_t batch_prepare(int dtype, int ty) {
-  return with_step2(dtype, ty, [&]<int TY, class TE>() {
-    if constexpr (TY == 8) return cudaErrorInvalidValue;
+  return with_step2(dtype, 2, false, ty, [&]<int TY, class TE, int K, bool MP>() {
+    if constexpr (TY == 8 || K != 2 || MP) return cudaErrorInvalidValue;
     else
       return cudaFuncSetAttribute(fslbm_step2_batch_kernel<TY, TE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(Step2Tile<TY, TE>::SMEM_BYTES));
@@ -504,8 +515,8 @@ cudaError_t launch_batch_steps(int dtype, int ty, const void* members, const Bat
   cudaError_t e = cudaMemsetAsync(sync, 0, batch_sync_words(nmembers) * sizeof(unsigned), st);
   if (e) return e;
   const BatchMember* mb = reinterpret_cast<const BatchMember*>(members);
-  return with_step2(dtype, ty, [&]<int TY, class TE>() {
-    if constexpr (TY == 8) {
+  return with_step2(dtype, 2, false, ty, [&]<int TY, class TE, int K, bool MP>() {
+    if constexpr (TY == 8 || K != 2 || MP) {
       return cudaErrorInvalidValue;
     } else {
       using Tl = Step2Tile<TY, TE>;

@@ -98,7 +98,7 @@ int setup_device(int dev) {
   if (e != cudaSuccess)
     return fslbm_set_error(FSLBM_ERR_CUDA, "step_f32_noalloc: cudaGetSymbolAddress: %s",
                            cudaGetErrorString(e));
-  if ((e = step2_prepare(FSLBM_F32, 2, kNoallocTY)) != cudaSuccess)
+  if ((e = step2_prepare(FSLBM_F32, 2, false, kNoallocTY)) != cudaSuccess)
     return fslbm_set_error(FSLBM_ERR_CUDA, "step_f32_noalloc: kernel set-up: %s", cudaGetErrorString(e));
   int sms = 0;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
@@ -190,7 +190,7 @@ extern "C" int fslbm_step_f32_noalloc(const float* state_in, float* state_out,
 
   // step constants formed as the reference forms them in FP32 (FSLBM.cu:231, 269, 599, 624)
   StepLaunch a{};
-  a.dtype = FSLBM_F32; a.d1 = 2;
+  a.dtype = FSLBM_F32; a.d1 = 2; a.K = 2;
   a.lxp = lx_pitch; a.ly = ly; a.L = lz;
   a.ntiles = ntx * nty;
   a.tiles = reinterpret_cast<const int2*>(scratch + kCoefBytes);
@@ -214,7 +214,7 @@ extern "C" int fslbm_step_f32_noalloc(const float* state_in, float* state_out,
   int nch = g_sm_count[dev] / a.ntiles;
   if (nch > (lz + 1) / 2) nch = (lz + 1) / 2;
   if (nch < 1) nch = 1;
-  Step2Launch b{2, kNoallocTY, &mp, &mu, &mo, a.ntiles * nch};
+  Step2Launch b{kNoallocTY, &mp, &mu, &mo, a.ntiles * nch};
   if ((e = launch_step2(a, b, st)) != cudaSuccess)
     return fslbm_set_error(FSLBM_ERR_CUDA, "step_f32_noalloc: step launch: %s", cudaGetErrorString(e));
 

@@ -1,5 +1,5 @@
 // FSLBM time step, FP32 arithmetic, pairs of planes, for sm_100a (corrective stride 2, FP32 or FP16
-// storage).
+// storage; corrector of 2 or 3 taps; one cross-section or one per plane).
 //
 // Same step as step_kernel.cuh (predictor factored by neighbour plane, coarse corrector,
 // periodic +-pin seam, walls, gauge, body force), organised for throughput:
@@ -39,7 +39,9 @@ namespace fslbm {
 
 // TE is the storage type of the state (float, or __half for FP16 storage); arithmetic is FP32
 // either way. Halo widths and paddings keep every TMA box start and destination on 16 bytes.
-template <int TY, class TE = float> struct Step2Tile {
+// K is the number of corrector taps per direction (2: the reference's order 2<->4 blend, 3: its
+// order 4<->6 blend).
+template <int TY, class TE = float, int K = 2> struct Step2Tile {
   static constexpr int D1 = 2;                          // corrective stride
   static constexpr int N = 2;                           // rows per thread
   static constexpr int ES = int(sizeof(TE));
@@ -47,7 +49,7 @@ template <int TY, class TE = float> struct Step2Tile {
   static constexpr int TX = 32;
   static constexpr int WARPS = TY / N;                  // a warp owns 32 N cells (see the warp shapes)
   static constexpr int THREADS = 32 * WARPS;
-  static constexpr int R = 2 * D1;                      // farthest corrector tap
+  static constexpr int R = K * D1;                      // farthest corrector tap: K pairs of planes
   static constexpr int HX = (R + A16 - 1) / A16 * A16;  // x halo, TMA-aligned (16 bytes)
   static constexpr int HY = R;
   static constexpr int SW = TX + 2 * HX;                // row length of both boxes
@@ -56,9 +58,9 @@ template <int TY, class TE = float> struct Step2Tile {
   static constexpr int PPL = (SW * PH * ES + 127) / 128 * 128 / ES;   // p plane, 128-byte aligned
   static constexpr int UPL = SW * UH;                                 // u, v or w plane
   static constexpr int VPL = (3 * UPL * ES + 127) / 128 * 128 / ES;   // u,v,w of one plane
-  // Window, in pairs of planes. In use: the output pair, the predictor's pair and the one after
-  // it; one more is in flight. p is read by the predictor only.
-  static constexpr int SU = 4, SP = SU - 2;
+  // Window, in pairs of planes. In use: the output pair and the K after it, of which the first is
+  // the predictor's; one more is in flight. p is read by the predictor only.
+  static constexpr int SU = K + 2, SP = 2;
   static constexpr uint32_t U_BYTES = uint32_t(3 * UPL * ES), P_BYTES = uint32_t(SW * PH * ES);
   static constexpr size_t P_OFFSET = size_t(SU) * 2 * VPL * ES;
   // staging of a warp's output pair: [plane][field][row][column] of the warp's cells
@@ -72,13 +74,14 @@ template <int TY, class TE = float> struct Step2Tile {
   static constexpr size_t BASE_OFFSET = (REL_OFFSET + (SU + 1) * sizeof(unsigned) + 15) / 16 * 16;
   static constexpr size_t BASE_BYTES = std::is_same<TE, __half>::value ? size_t(BW) * BH * sizeof(float) : 0;
   static constexpr size_t SMEM_BYTES = BASE_OFFSET + BASE_BYTES;
-  // tensor memory: a ring of 4 pairs of a warp's own columns of u, v, w; warps w, w + 4, ... share
-  // the 32 lanes of subpartition w % 4
-  static constexpr int TM_SLOT = 6 * N, TM_WARP = 4 * TM_SLOT;
+  // tensor memory: a ring of a warp's own columns of u, v, w of the predictor's pair and the K + 1
+  // before it; warps w, w + 4, ... share the 32 lanes of subpartition w % 4
+  static constexpr int TM_RING = K == 2 ? 4 : 8;
+  static constexpr int TM_SLOT = 6 * N, TM_WARP = TM_RING * TM_SLOT;
   static constexpr int TM_NEED = TM_WARP * ((WARPS + 3) / 4);
   static constexpr int TM_COLS = TM_NEED <= 32 ? 32 : TM_NEED <= 64 ? 64 : TM_NEED <= 128 ? 128 : 256;
   // CTAs per SM (shared memory; 128 registers a thread at 16 warps per SM)
-  static constexpr int CTAS = TY == 32 ? 1 : TY == 16 ? (ES == 2 ? 2 : 1) : 3;
+  static constexpr int CTAS = K > 2 || TY == 32 ? 1 : TY == 16 ? (ES == 2 ? 2 : 1) : 3;
   static_assert(TM_NEED <= TM_COLS && TM_COLS * CTAS <= 512, "tensor memory columns");
   static_assert((PPL * ES) % 128 == 0 && (VPL * ES) % 128 == 0 && (STG * ES) % 128 == 0,
                 "TMA addresses must stay aligned");
@@ -102,9 +105,11 @@ struct Step2Geom {
   // of the stored w. Null for other storage types.
   const float* wb;
   const float* wgt;
+  const uint8_t* near;     // masks per plane: code per cell (see step2_march), else null
 };
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 f2(float2 a) { return a; }
 __device__ __forceinline__ float lds1(const float* p) { return *p; }
 __device__ __forceinline__ float lds1(const __half* p) { return __half2float(*p); }
 
@@ -131,7 +136,8 @@ __device__ __forceinline__ __half sr_half(float x, uint32_t r) {
 // Arithmetic on a pair of planes (.x the march-earlier plane, .y the later one): packed FP32x2
 // instructions, each half rounded as the scalar operation.
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }   // an operand modifier
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
@@ -158,14 +164,14 @@ __device__ __forceinline__ RowSums row_sums(const float2 (&p)[3], const float2 (
     M[j] = mul2(v[j], w[j]);
     const float2 s = add2(V2[j], W2[j]);
     if (j == 1) {
-      P[j] = fma2(f2(-1.5f), fma2(u[j], u[j], s), p[j]);
+      P[j] = fma2(neg2(fma2(u[j], u[j], s)), f2(1.5f), p[j]);
       V[j] = v[j];
       W[j] = w[j];
     } else {
-      const float sg = j == 2 ? 3.0f : -3.0f;
-      const float2 a = fma2(u[j], f2(sg), f2(1.0f));
-      // q + 3 cx u + 4.5 u^2 = p - 1.5 (v^2 + w^2) + u (3 u + 3 cx)
-      P[j] = fma2(u[j], fma2(u[j], f2(3.0f), f2(sg)), fma2(f2(-1.5f), s, p[j]));
+      const float2 cu = j == 2 ? u[j] : neg2(u[j]);          // cx u
+      const float2 a = fma2(cu, f2(3.0f), f2(1.0f));
+      // q + 3 cx u + 4.5 u^2 = p - 1.5 (v^2 + w^2) + cx u (3 cx u + 3)
+      P[j] = fma2(cu, fma2(cu, f2(3.0f), f2(3.0f)), fma2(neg2(s), f2(1.5f), p[j]));
       V[j] = mul2(v[j], a);
       W[j] = mul2(w[j], a);
     }
@@ -185,11 +191,12 @@ struct RowSide {
   float2 R0, D0, Rz, Dz, Rw, Dw;
 };
 template <int CY> __device__ __forceinline__ RowSide row_side(const RowSums& o) {
+  auto cy = [](float2 a) { return CY > 0 ? a : neg2(a); };
   RowSide s;
-  s.R0 = fma2(f2(3.0f * CY), o.R1, fma2(f2(4.5f), o.R2, o.R0));
-  s.D0 = fma2(f2(3.0f * CY), o.D1, fma2(f2(4.5f), o.D2, o.D0));
-  s.Rz = fma2(f2(3.0f * CY), o.Rm, o.Rz);
-  s.Dz = fma2(f2(3.0f * CY), o.Dm, o.Dz);
+  s.R0 = fma2(cy(o.R1), f2(3.0f), fma2(f2(4.5f), o.R2, o.R0));
+  s.D0 = fma2(cy(o.D1), f2(3.0f), fma2(f2(4.5f), o.D2, o.D0));
+  s.Rz = fma2(cy(o.Rm), f2(3.0f), o.Rz);
+  s.Dz = fma2(cy(o.Dm), f2(3.0f), o.Dz);
   s.Rw = o.Rw;
   s.Dw = o.Dw;
   return s;
@@ -204,14 +211,17 @@ __device__ __forceinline__ void tm_load(float2 (&v)[2], uint32_t a) {
                : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y) : "r"(a) : "memory");
 }
 __device__ __forceinline__ void tm_wait_stores() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// Completes the loads into v0 .. v3: their uses cannot move before the wait.
-__device__ __forceinline__ void tm_wait_loads(float2 (&v0)[2], float2 (&v1)[2], float2 (&v2)[2], float2 (&v3)[2]) {
+// Completes the loads into v: their uses cannot move before the wait.
+#define FSLBM_TM_REGS(i) "+f"(v[i][0].x), "+f"(v[i][0].y), "+f"(v[i][1].x), "+f"(v[i][1].y)
+__device__ __forceinline__ void tm_wait_loads(float2 (&v)[4][2]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+f"(v0[0].x), "+f"(v0[0].y), "+f"(v0[1].x), "+f"(v0[1].y), "+f"(v1[0].x), "+f"(v1[0].y),
-                 "+f"(v1[1].x), "+f"(v1[1].y), "+f"(v2[0].x), "+f"(v2[0].y), "+f"(v2[1].x), "+f"(v2[1].y),
-                 "+f"(v3[0].x), "+f"(v3[0].y), "+f"(v3[1].x), "+f"(v3[1].y)
-               :: "memory");
+               : FSLBM_TM_REGS(0), FSLBM_TM_REGS(1), FSLBM_TM_REGS(2), FSLBM_TM_REGS(3)::"memory");
 }
+__device__ __forceinline__ void tm_wait_loads(float2 (&v)[5][2]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : FSLBM_TM_REGS(0), FSLBM_TM_REGS(1), FSLBM_TM_REGS(2), FSLBM_TM_REGS(3), FSLBM_TM_REGS(4)::"memory");
+}
+#undef FSLBM_TM_REGS
 // Allocation of a kernel's tensor memory by its first warp (whole warp); `slot` in shared memory
 // receives the base address. Freed by the same warp before the kernel ends, on every path.
 template <int COLS> __device__ __forceinline__ void tm_alloc(uint32_t* slot) {
@@ -233,12 +243,12 @@ template <int COLS> __device__ __forceinline__ void tm_free(uint32_t base) {
 // cross-sections. With the 160-byte FP32 row stride the shapes 0 and 1 read shared memory without
 // bank conflicts (rows 2 apart are 16 banks apart), shape 2 two-way. The map changes no thread's
 // arithmetic.
-template <int TY, class TE>
+template <int TY, class TE, int K = 2, bool MP = false>
 __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUtensorMap* tmap_uvw,
                                             const CUtensorMap* tmap_out, uint32_t tmem, const Step2Geom& g,
                                             const StepConst<float>& k, int tile, int chunk,
                                             unsigned char* smem, bool reinit, int shape) {
-  using Tl = Step2Tile<TY, TE>;
+  using Tl = Step2Tile<TY, TE, K>;
   constexpr int N = Tl::N, R = Tl::R, D1 = Tl::D1, HX = Tl::HX, HY = Tl::HY, SW = Tl::SW, SU = Tl::SU, SP = Tl::SP;
   constexpr int PPL = Tl::PPL, UPL = Tl::UPL, VPL = Tl::VPL;
   TE* uring = reinterpret_cast<TE*>(smem);
@@ -257,25 +267,37 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   const int zb = int((long long)g.L * chunk / g.nchunks);
   const int nout = int((long long)g.L * (chunk + 1) / g.nchunks) - zb;
   const int dir = (chunk & 1) ? -1 : 1;
-  const int nstage = (nout + 1) / 2 + R;                // pairs of planes: the outputs and 2 R planes
+  const int nstage = (nout + 1) / 2 + 2 * K;            // pairs of planes: the outputs and K either side
   const int start = dir > 0 ? zb - R : zb + nout - 1 + R;   // real plane of march index 0
   const int2 org = g.tiles[tile];
   const int x = org.x + tx, y0 = org.y + ty;
 
-  // warps that compute (some fluid) and warps over fluid away from walls (no wall sums)
-  const ColCoef<float>* ccol = reinterpret_cast<const ColCoef<float>*>(g.colcoef) + ((long long)y0 * g.lxp + x);
-  auto coef = [&](int r) {             // outside the cross-section: nothing
-    return x < g.lxp && y0 + r < g.ly ? ccol[r * g.lxp] : ColCoef<float>{0.f, 0.f, 0.f, 0.f};
+  // Warps that compute (some fluid) and warps over fluid away from walls (no wall sums). With a
+  // mask per plane (MP) the codes in g.near tell, per cell: 0 fluid without a wall neighbour,
+  // 1 fluid beside a wall, 2 wall; one more plane holds 2 for the columns without any fluid.
+  const size_t cplane = size_t(g.lxp) * g.ly;
+  const long long col = (long long)y0 * g.lxp + x;
+  auto coef = [&](int r) {             // extruded masks; outside the cross-section: nothing
+    return x < g.lxp && y0 + r < g.ly ? reinterpret_cast<const ColCoef<float>*>(g.colcoef)[col + r * g.lxp]
+                                      : ColCoef<float>{0.f, 0.f, 0.f, 0.f};
+  };
+  auto near_code = [&](int r, int z) -> unsigned {
+    return x < g.lxp && y0 + r < g.ly ? g.near[z * cplane + col + r * g.lxp] : 2u;
   };
   bool some = false, every = true;
+  if constexpr (MP) {
 #pragma unroll
-  for (int r = 0; r < N; ++r) {
-    const ColCoef<float> c = coef(r);
-    some |= c.fluid != 0.0f;
-    every &= c.fluid != 0.0f && c.ws0 == 0.0f && c.wsx == 0.0f && c.wsy == 0.0f;
+    for (int r = 0; r < N; ++r) some |= near_code(r, g.L) != 2u;   // over all planes
+  } else {
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+      const ColCoef<float> c = coef(r);
+      some |= c.fluid != 0.0f;
+      every &= c.fluid != 0.0f && c.ws0 == 0.0f && c.wsx == 0.0f && c.wsy == 0.0f;
+    }
   }
   const bool warp_on = __any_sync(0xffffffffu, some);
-  const bool plain = __all_sync(0xffffffffu, every);
+  const bool plain_column = __all_sync(0xffffffffu, every);
 
   __syncthreads();   // a previous item (persistent grids) is fully consumed
   if (tid == 0) {
@@ -296,7 +318,7 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
     }
   __syncthreads();
 
-  // stage j: u,v,w of the plane pair j (march planes 2j, 2j + 1) and p of the pair j - 1, which
+  // stage j: u,v,w of the plane pair j (march planes 2j, 2j + 1) and p of the pair j - K + 1, which
   // the predictor reads in the iteration that waits for this stage
   auto plane_of = [&](int m) {
     int zz = start + dir * m;
@@ -305,15 +327,16 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   };
   auto issue = [&](int j) {
     uint64_t* bar = &full[unsigned(j) % unsigned(SU)];
-    const bool with_p = j >= 2;
+    const bool with_p = j >= 2 * K - 2;
     mbar_arrive_expect_tx(bar, 2 * Tl::U_BYTES + (with_p ? 2 * Tl::P_BYTES : 0u));
     TE* du = uring + unsigned(j) % unsigned(SU) * (2 * VPL);
     tma_load_4d(du, tmap_uvw, bar, org.x - HX, org.y - HY, plane_of(2 * j), 1);
     tma_load_4d(du + VPL, tmap_uvw, bar, org.x - HX, org.y - HY, plane_of(2 * j + 1), 1);
     if (with_p) {
-      TE* dp = pring + unsigned(j - 1) % unsigned(SP) * (2 * PPL);
-      tma_load_4d(dp, tmap_p, bar, org.x - HX, org.y - 1, plane_of(2 * j - 2), 0);
-      tma_load_4d(dp + PPL, tmap_p, bar, org.x - HX, org.y - 1, plane_of(2 * j - 1), 0);
+      const int m = 2 * (j - K + 1);
+      TE* dp = pring + unsigned(j - K + 1) % unsigned(SP) * (2 * PPL);
+      tma_load_4d(dp, tmap_p, bar, org.x - HX, org.y - 1, plane_of(m), 0);
+      tma_load_4d(dp + PPL, tmap_p, bar, org.x - HX, org.y - 1, plane_of(m + 1), 0);
     }
   };
   if (tid == 0) {                      // the whole window up front
@@ -338,9 +361,9 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   // predictor read it, both in iteration j + 1). __syncwarp orders the warp's shared loads before
   // lane 0's acq_rel add to the slot's counter; the warp whose add completes the count has
   // acquired every warp's loads, orders them before its TMA writes with a proxy fence and refills
-  // the slot with stage j + SU (p of pair j + SU - 1, into the slot of p of pair j + 1). A warp
-  // waiting for stage q needs every warp to have released pair q - SU, in iteration q - SU + 1,
-  // an earlier one than the waiting iteration q - 1, so no wait depends on itself. A slot's next
+  // the slot with stage j + SU (and p of pair j + 3 into the slot of p of pair j + 1). A warp that
+  // waits for stage s in iteration s - K + 1 needs every warp to have released pair s - SU, in
+  // iteration s - SU + 1 = s - K - 1 at the latest, so no wait depends on itself. A slot's next
   // count starts only after its refill has landed, so the count is a multiple of WARPS exactly
   // when a pair is complete.
   auto release = [&](int j) {
@@ -354,11 +377,15 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
     }
   };
 
-  if (!arrive_wait(0) || !arrive_wait(1)) return false;
+#pragma unroll
+  for (int j = 0; j < 2 * K - 2; ++j)
+    if (!arrive_wait(j)) return false;
   if (!warp_on) {   // all-wall warps keep the pipeline protocol only
 #pragma unroll 1
-    for (int q = 1; q <= nstage - 2; ++q) {
-      if (!arrive_wait(q + 1)) return false;
+    for (int q = K - 1; q <= nstage - K; ++q) {
+      if (!arrive_wait(q + K - 1)) return false;
+      if (q == K - 1)
+        for (int j = 0; j < K - 2; ++j) release(j);
       release(q - 1);
     }
     return true;
@@ -369,22 +396,28 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   const float gauge = g.gauge ? float(__ldcg(g.gauge)) : 0.0f;
   const int po = (ty + 1) * SW + HX + tx;               // p box
   const int uo = (ty + HY) * SW + HX + tx;              // u box (v, w at +UPL, +2 UPL)
-  const float h6 = float(dir) / 72.0f;
+  const float dir3 = 3.0f * float(dir);
   // folded update: u_new = K1 t1 + K2 t2 + K0 u + tb (u* + F), the corrector's taps t1 / t2 at
   // distance d1 / 2 d1, K0 = tb dtddy m c0 + (1 - tb), K1 = tb dtddy m c1, K2 = tb dtddy m c2
   const float kam = __fmul_rn(__fmul_rn(k.tb, k.dtddy), k.m);
-  const float kK0 = __fmaf_rn(kam, k.c0, k.cc), kK1 = __fmul_rn(kam, k.c1), kK2 = __fmul_rn(kam, k.c2);
-  const float ktz = __fmul_rn(float(dir), k.tb);        // the z-moment carries the sign
+  const float kK0 = __fmaf_rn(kam, k.c0, k.cc);
+  float kKt[K];                                         // K1 .. KK
+  kKt[0] = __fmul_rn(kam, k.c1);
+  kKt[1] = __fmul_rn(kam, k.c2);
+#pragma unroll
+  for (int j = 2; j < K; ++j) kKt[j] = __fmul_rn(kam, k.ch[j - 2]);
+  // the predictor's moments come times 216; the z-moment carries the march direction's sign
+  const float ktb = __fdiv_rn(k.tb, 216.0f), ktz = __fmul_rn(float(dir), ktb);
   // FP16 storage: the rounding noise of a cell pair is keyed by its first cell, the field and the step
   const uint32_t seed = hash32(g.step_no * 0x9e3779b9u + 0x632be5abu);
 
   auto ldu = [&](const TE* q) { return make_float2(lds1(q), lds1(q + VPL)); };
-  // ring of the own columns of the last four pairs in tensor memory: pair j in slot j % 4, field f
-  // of row r at column f 2 N + 2 r
-  const uint32_t tm = tmem + (uint32_t(warp & 3) << 21) + uint32_t((warp >> 2) * Tl::TM_WARP);
-  auto tm_slot = [&](int j) { return tm + (unsigned(j) & 3u) * unsigned(Tl::TM_SLOT); };
+  // ring of the own columns in tensor memory: pair j in slot j % TM_RING, field f of row r at
+  // column f 2 N + 2 r
+  const uint32_t tm = __shfl_sync(0xffffffffu, tmem + (uint32_t(warp & 3) << 21) + uint32_t((warp >> 2) * Tl::TM_WARP), 0);
+  auto tm_slot = [&](int j) { return tm + (unsigned(j) & unsigned(Tl::TM_RING - 1)) * unsigned(Tl::TM_SLOT); };
 #pragma unroll
-  for (int j = 0; j < 2; ++j)
+  for (int j = 0; j < K - 1; ++j)        // pairs the predictor does not visit
 #pragma unroll
     for (int f = 0; f < 3; ++f)
 #pragma unroll
@@ -393,26 +426,34 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   // staging: the thread's place in the warp's block of wcols x (N << shape) cells
   TE* stg = reinterpret_cast<TE*>(smem + Tl::STG_OFFSET) + warp * Tl::STG;
   TE* sto = stg + lrow * wcols + lcol;
-  // Predictor terms carried to the next iteration, per row: cl = the finished sums of the pair's
-  // first plane, sh = the self-plane moments of its second, dl / dh = the shares that the first
-  // and second plane give their march-next planes, pc = p of the pair.
-  float cl[N][4], sh[N][3], dl[N][3], dh[N][3];
-  float2 pc[N];
+  // Predictor terms carried to the next iteration, per row: cp = the sums of the pair (its first
+  // plane's are finished), sh = the self-plane moments of its second plane, dd = the shares that
+  // its planes give their march-next planes, pc = p of the pair.
+  float2 cp[N][4], dd[N][3], pc[N];
+  float sh[N][3];
 #pragma unroll
   for (int r = 0; r < N; ++r) {
     pc[r] = f2(0.f);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      cl[r][j] = 0.f;
-      if (j < 3) sh[r][j] = dl[r][j] = dh[r][j] = 0.f;
+      cp[r][j] = f2(0.f);
+      if (j < 3) {
+        dd[r][j] = f2(0.f);
+        sh[r][j] = 0.f;
+      }
     }
   }
 
-  // iteration q: predictor of pair q, which completes the sums of pair q - 1, and from q = 3 on
+#pragma unroll
+  for (int j = 0; j < K - 2; ++j) release(j);
+  // iteration q: predictor of pair q, which completes the sums of pair q - 1, and from q = K + 1 on
   // corrector and update of the output pair q - 1
-#pragma unroll 1
-  for (int q = 1; q <= nstage - 2; ++q) {
-    if (!arrive_wait(q + 1)) {
+  // Two iterations per pass rename the carried registers instead of moving them (FP32, one
+  // cross-section: 4679 -> 4550 us per 50 steps at 512 x 128 x 128); the others would spill.
+  constexpr int kPass = !MP && !kBase ? 2 : 1;
+#pragma unroll kPass
+  for (int q = K - 1; q <= nstage - K; ++q) {
+    if (!arrive_wait(q + K - 1)) {
       tm_wait_stores();
       if (lane == 0) bulk_wait_all();
       return false;
@@ -420,9 +461,11 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
     const TE* sp0 = pring + unsigned(q) % unsigned(SP) * (2 * PPL) + po;
     const TE* su0 = uring + unsigned(q) % unsigned(SU) * (2 * VPL) + uo;          // predictor pair q
     const TE* sub = uring + unsigned(q - 1) % unsigned(SU) * (2 * VPL) + uo;      // output pair q - 1
-    const TE* sua = uring + unsigned(q + 1) % unsigned(SU) * (2 * VPL) + uo;      // pair q + 1
+    const TE* sua[K - 1];                                                         // pairs q + 1 ..
+#pragma unroll
+    for (int j = 0; j < K - 1; ++j) sua[j] = uring + unsigned(q + 1 + j) % unsigned(SU) * (2 * VPL) + uo;
     const int zp = start + dir * 2 * q;                                           // real plane of the pair's first
-    float comp[N][4], cfirst[N][4];
+    float nfirst[N][4];                  // finished sums of pair q's first plane
     float2 pcen[N];
     {
       RowSide above, here;               // rows r - 1 and r as their lower neighbours see them
@@ -469,22 +512,42 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
             // non-wall cells, i.e. the jump times their weight sums (raw units, x36)
             auto jump = [&](int z) { return z < 0 ? k.pin : (z >= g.L ? -k.pin : 0.0f); };
             const float2 off = make_float2(jump(zp), jump(zp + dir));
-            const ColCoef<float> c = coef(r);
-            A[0] = fma2(off, f2(__fmaf_rn(-36.f, c.ws0, 36.f)), A[0]);
-            X[0] = fma2(off, f2(-36.f * c.wsx), X[0]);
-            Y[0] = fma2(off, f2(-36.f * c.wsy), Y[0]);
+            float2 n0, nx, ny;
+            if constexpr (MP) {
+              float s0[2], sx[2], sy[2];
+              for (int h = 0; h < 2; ++h) {
+                const uint8_t* mz = g.mask + plane_of(2 * q + h) * cplane;
+                s0[h] = sx[h] = sy[h] = 0.f;
+                for (int cy = -1; cy <= 1; ++cy)
+                  for (int cx = -1; cx <= 1; ++cx) {
+                    const int gx = x + cx, gy = y0 + r + cy;
+                    if (gx < 0 || gy < 0 || gx >= g.lxp || gy >= g.ly || mz[gy * g.lxp + gx] == kWall) continue;
+                    const float w = (cx ? 1.f : 4.f) * (cy ? 1.f : 4.f);
+                    s0[h] += w; sx[h] += cx * w; sy[h] += cy * w;
+                  }
+              }
+              n0 = make_float2(s0[0], s0[1]); nx = make_float2(sx[0], sx[1]); ny = make_float2(sy[0], sy[1]);
+            } else {
+              const ColCoef<float> c = coef(r);
+              n0 = f2(__fmaf_rn(-36.f, c.ws0, 36.f)); nx = f2(-36.f * c.wsx); ny = f2(-36.f * c.wsy);
+            }
+            A[0] = fma2(off, n0, A[0]);
+            X[0] = fma2(off, nx, X[0]);
+            Y[0] = fma2(off, ny, Y[0]);
           }
           // True sums are A0/36, dir A1/12, A2/8. A plane is the march-next neighbour of the plane
           // before it, itself, and the march-previous neighbour of the plane after: with
           // e = (A0 + A2)/6 and h = A1/6 the shares are e + h (next), (2/3) A0 (self) and e - h
           // (previous); for the z-moment h - e (previous), none (self) and e + h (next), times dir.
+          // All are carried times 216 (the weights' common denominator): e = A0 + 4.5 A2,
+          // h = 3 dir A1, self = 4 A0.
           float2 s[3], d[3];
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             const float2(&m)[3] = i == 0 ? A : (i == 1 ? X : Y);
-            const float2 e = fma2(m[2], f2(1.0f / 48.0f), mul2(m[0], f2(1.0f / 216.0f)));
-            s[i] = fma2(m[1], f2(h6), e);
-            d[i] = fma2(m[1], f2(-h6), e);
+            const float2 e = fma2(m[2], f2(4.5f), m[0]);
+            s[i] = fma2(m[1], f2(dir3), e);
+            d[i] = fma2(neg2(m[1]), f2(dir3), e);
           }
           // Each cell sums its two neighbour planes' shares first (a commutative add) and then
           // fuses its own plane's share, so its FP32 result depends neither on the march
@@ -493,18 +556,15 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
           const float2 self[3] = {A[0], X[0], Y[0]};
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
-            cfirst[r][i] = cl[r][i];
-            comp[r][i] = __fmaf_rn(sh[r][i], 1.0f / 54.0f, __fadd_rn(dl[r][i], s[i].x));
-            cl[r][i] = __fmaf_rn(self[i].x, 1.0f / 54.0f, __fadd_rn(dh[r][i], s[i].y));
+            cp[r][i].y = __fmaf_rn(sh[r][i], 4.0f, __fadd_rn(dd[r][i].x, s[i].x));
+            nfirst[r][i] = __fmaf_rn(self[i].x, 4.0f, __fadd_rn(dd[r][i].y, s[i].y));
           }
-          cfirst[r][3] = cl[r][3];
-          comp[r][3] = __fsub_rn(s[0].x, dl[r][0]);
-          cl[r][3] = __fsub_rn(s[0].y, dh[r][0]);
+          cp[r][3].y = __fsub_rn(s[0].x, dd[r][0].x);
+          nfirst[r][3] = __fsub_rn(s[0].y, dd[r][0].y);
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             sh[r][i] = self[i].y;
-            dl[r][i] = d[i].x;
-            dh[r][i] = d[i].y;
+            dd[r][i] = d[i];
           }
         }
         if (j >= 0) above = here;
@@ -512,15 +572,54 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
         here = row_side<-1>(row);
       }
     }
-    if (q >= 3) {
+    if (q > K) {
       tm_wait_stores();
       const int zo = zp - 2 * dir;                           // real plane of the output pair's first
-      ColCoef<float> cc[N];
+      const bool second = 2 * (q - 1 - K) + 1 < nout;        // the chunk's plane count may be odd
+      // wall sums (times 216) and fluid flag of the rows: one value for both planes of an extruded mask
+      using Sum = std::conditional_t<MP, float2, float>;
+      auto both = [](float a, float b) {
+        if constexpr (MP) return make_float2(a, b);
+        else return a;
+      };
+      Sum ws0[N], wsx[N], wsy[N], wsz[N], fluid[N];
 #pragma unroll
-      for (int r = 0; r < N; ++r) cc[r] = ColCoef<float>{0.f, 0.f, 0.f, 1.f};
-      if (!plain)
+      for (int r = 0; r < N; ++r) {
+        ws0[r] = wsx[r] = wsy[r] = wsz[r] = both(0.f, 0.f);
+        fluid[r] = both(1.f, 1.f);
+      }
+      if constexpr (MP) {
+        const int z1 = second ? zo + dir : zo;
+        unsigned code[N][2], any = 0;
 #pragma unroll
-        for (int r = 0; r < N; ++r) cc[r] = coef(r);
+        for (int r = 0; r < N; ++r) {
+          code[r][0] = near_code(r, zo);
+          code[r][1] = near_code(r, z1);
+          any |= code[r][0] | code[r][1];
+        }
+        if (__any_sync(0xffffffffu, any != 0u)) {
+          const CellCoef<float>* cells = reinterpret_cast<const CellCoef<float>*>(g.colcoef) + col;
+#pragma unroll
+          for (int r = 0; r < N; ++r)
+            if (x < g.lxp && y0 + r < g.ly) {
+              const CellCoef<float> a = cells[zo * cplane + r * g.lxp], b = cells[z1 * cplane + r * g.lxp];
+              ws0[r] = make_float2(216.f * a.ws0, 216.f * b.ws0);
+              wsx[r] = make_float2(216.f * a.wsx, 216.f * b.wsx);
+              wsy[r] = make_float2(216.f * a.wsy, 216.f * b.wsy);
+              wsz[r] = make_float2(216.f * float(dir) * a.wsz, 216.f * float(dir) * b.wsz);
+            }
+#pragma unroll
+          for (int r = 0; r < N; ++r)
+            fluid[r] = make_float2(code[r][0] == 2u ? 0.f : 1.f, code[r][1] == 2u ? 0.f : 1.f);
+        }
+      } else if (!plain_column) {
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+          const ColCoef<float> c = coef(r);
+          ws0[r] = 216.f * c.ws0; wsx[r] = 216.f * c.wsx; wsy[r] = 216.f * c.wsy;
+          fluid[r] = c.fluid;
+        }
+      }
       float2 wg[N];
       if (kBase)
 #pragma unroll
@@ -529,7 +628,7 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
       if (lane == 0) bulk_wait_read();                       // the previous pair has left the staging
       __syncwarp();
       auto put = [&](int f, int r, float2 val) {
-        val = mul2(val, f2(cc[r].fluid));                    // wall columns get zero
+        val = mul2(val, f2(fluid[r]));                           // walls get zero
         TE* o = sto + f * N * 32 + r * wcols;
         if constexpr (kBase) {
           // two cells share a hash word: the even column's lane forms the first plane's, the odd
@@ -548,51 +647,58 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
       };
 #pragma unroll
       for (int r = 0; r < N; ++r)
-        put(0, r, add2(fma2(pc[r], f2(cc[r].ws0), make_float2(cfirst[r][0], comp[r][0])), f2(-gauge)));
+        put(0, r, fma2(fma2(pc[r], f2(ws0[r]), cp[r][0]), f2(1.0f / 216.0f), f2(-gauge)));
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
         const TE* b = sub + f * UPL;
-        float2 za1[N], c0[N], h1[N], h2[N];                  // own columns of pairs q, q - 1, q - 2, q - 3
-        tm_load(za1, tm_slot(q) + f * 2 * N);
-        tm_load(c0, tm_slot(q - 1) + f * 2 * N);
-        tm_load(h1, tm_slot(q - 2) + f * 2 * N);
-        tm_load(h2, tm_slot(q - 3) + f * 2 * N);
+        float2 ring[K + 2][N];                               // own columns of pairs q, q - 1, ...
+#pragma unroll
+        for (int j = 0; j < K + 2; ++j) tm_load(ring[j], tm_slot(q - j) + f * 2 * N);
         float2 c[N + 2 * R];                                 // rows -R .. N + R - 1 of the own column
 #pragma unroll
         for (int j = -R; j < N + R; ++j)
           if (j < 0 || j >= N) c[j + R] = ldu(b + j * SW);
-        tm_wait_loads(za1, c0, h1, h2);
+        tm_wait_loads(ring);
 #pragma unroll
-        for (int r = 0; r < N; ++r) c[r + R] = c0[r];
+        for (int r = 0; r < N; ++r) c[r + R] = ring[1][r];
 #pragma unroll
         for (int r = 0; r < N; ++r) {
           const TE* t = b + r * SW;
-          const float2 za2 = ldu(sua + f * UPL + r * SW);
-          const float2 t1 = add2(add2(add2(ldu(t - D1), ldu(t + D1)), add2(c[r + R - D1], c[r + R + D1])),
-                                 add2(h1[r], za1[r]));
-          const float2 t2 = add2(add2(add2(ldu(t - 2 * D1), ldu(t + 2 * D1)),
-                                      add2(c[r + R - 2 * D1], c[r + R + 2 * D1])),
-                                 add2(h2[r], za2));
-          const float2 cm = make_float2(cfirst[r][f == 2 ? 3 : 1 + f], comp[r][f == 2 ? 3 : 1 + f]);
-          const float2 mom = f == 2 ? cm : fma2(pc[r], f2(f == 0 ? cc[r].wsx : cc[r].wsy), cm);
+          float2 taps[K];                                    // the six taps at distance 2 (j + 1)
+#pragma unroll
+          for (int j = 0; j < K; ++j) {
+            const int o = D1 * (j + 1);
+            const float2 ahead = j == 0 ? ring[0][r] : ldu(sua[j > 0 ? j - 1 : 0] + f * UPL + r * SW);
+            taps[j] = add2(add2(add2(ldu(t - o), ldu(t + o)), add2(c[r + R - o], c[r + R + o])),
+                           add2(ring[j + 2][r], ahead));
+          }
+          const float2 cm = cp[r][f == 2 ? 3 : 1 + f];
+          const float2 mom = f == 2 && !MP ? cm : fma2(pc[r], f2(f == 0 ? wsx[r] : (f == 1 ? wsy[r] : wsz[r])), cm);
           // FP16 storage updates the stored deviation of w: the force's term becomes the column's
           // share of the step of the base (tb fz included), see launch_wgt
           const float2 tf = kBase && f == 2 && g.wgt ? wg[r] : f2(__fmul_rn(k.tb, f == 0 ? k.fx : (f == 1 ? k.fy : k.fz)));
-          put(1 + f, r, fma2(f2(kK1), t1, fma2(f2(kK2), t2, fma2(f2(kK0), c0[r],
-                         fma2(f2(f == 2 ? ktz : k.tb), mom, tf)))));
+          // the small terms first: only the last operation rounds at the size of u
+          float2 un = fma2(f2(f == 2 ? ktz : ktb), mom, tf);
+#pragma unroll
+          for (int j = K - 1; j >= 0; --j) un = fma2(f2(kKt[j]), taps[j], un);
+          un = fma2(f2(kK0), ring[1][r], un);
+          put(1 + f, r, un);
         }
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
         tma_store_4d(tmap_out, stg, org.x + wx, org.y + wy, zo, 0);
-        // the chunk's plane count may be odd
-        if (2 * q - 1 - R < nout) tma_store_4d(tmap_out, stg + 4 * N * 32, org.x + wx, org.y + wy, zo + dir, 0);
+        if (second) tma_store_4d(tmap_out, stg + 4 * N * 32, org.x + wx, org.y + wy, zo + dir, 0);
         bulk_commit();
       }
     }
 #pragma unroll
-    for (int r = 0; r < N; ++r) pc[r] = pcen[r];
+    for (int r = 0; r < N; ++r) {
+      pc[r] = pcen[r];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) cp[r][i].x = nfirst[r][i];
+    }
     release(q - 1);
   }
   if (lane == 0) bulk_wait_all();
@@ -600,13 +706,13 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
 }
 
 // One pipe, one step: CTA b marches (tile b % ntiles, chunk b / ntiles).
-template <int TY, class TE>
-__global__ void __launch_bounds__(Step2Tile<TY, TE>::THREADS, Step2Tile<TY, TE>::CTAS)
+template <int TY, class TE, int K = 2, bool MP = false>
+__global__ void __launch_bounds__(Step2Tile<TY, TE, K>::THREADS, Step2Tile<TY, TE, K>::CTAS)
     fslbm_step2_kernel(const __grid_constant__ CUtensorMap tmap_p,
                        const __grid_constant__ CUtensorMap tmap_uvw,
                        const __grid_constant__ CUtensorMap tmap_out, const Step2Geom g,
                        const StepConst<float> k) {
-  using Tl = Step2Tile<TY, TE>;
+  using Tl = Step2Tile<TY, TE, K>;
   extern __shared__ __align__(128) unsigned char smem[];
   uint32_t* tm_base = reinterpret_cast<uint32_t*>(smem + Tl::REL_OFFSET) + Tl::SU;
   if (threadIdx.x < 32) tm_alloc<Tl::TM_COLS>(tm_base);
@@ -614,7 +720,7 @@ __global__ void __launch_bounds__(Step2Tile<TY, TE>::THREADS, Step2Tile<TY, TE>:
   if (threadIdx.x == 0 && blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
   __syncthreads();
   const uint32_t tmem = *tm_base;
-  step2_march<TY, TE>(&tmap_p, &tmap_uvw, &tmap_out, tmem, g, k, blockIdx.x % g.ntiles, blockIdx.x / g.ntiles, smem,
+  step2_march<TY, TE, K, MP>(&tmap_p, &tmap_uvw, &tmap_out, tmem, g, k, blockIdx.x % g.ntiles, blockIdx.x / g.ntiles, smem,
                       false, 0);
   grid_launch_dependents();   // not earlier: waiting CTAs of the next step would share this one's SMs
   __syncthreads();

@@ -48,3 +48,35 @@ def test_tile_heights_match_oracle_and_each_other(built, ctx, monkeypatch, L, lx
     got, _ = run_gpu(built, ctx, dom, prm, built.F64, f, steps, monitor_every=3)
     _, eu, eps = errors(got, ref, m2)
     assert eu <= 1e-12 and eps <= 1e-12, (eu, eps)
+
+
+@pytest.mark.parametrize("order,rough", [(6, False), (0, True), (6, True)])
+@pytest.mark.parametrize("L,lx,ly", [(7, 33, 20), (33, 24, 41), (40, 65, 40)])
+def test_three_taps_and_masks_per_plane(built, ctx, monkeypatch, L, lx, ly, order, rough):
+    """The pair kernel's 3-tap corrector and its masks per plane, every tile height it has, with
+    wall bumps that start and end inside a pair of planes and on the seam."""
+    m2, f, prm = case(L, lx, ly)
+    mask = m2
+    if rough:
+        mask = np.repeat(m2[None], L, axis=0)
+        inner = np.argwhere(m2 == 0)
+        for z in (0, 3, L - 1):                   # a few fluid cells of these planes become wall
+            for y, x in inner[z % 5::7]:
+                mask[z, y, x] = 125
+        f = f * (mask == 0)
+    prm = dict(prm, fd_order=order, blend=0.4 if order == 6 else 1.0)
+    dom = built.make_domain(lx, ly, L, mask=mask, radius=min(lx, ly) / 2 - 1, buffer_depth=4)
+    steps = 7
+    ref, _ = O.run_core(mask, L, f, prm, steps, monitor_every=0)
+    outs = []
+    for ty in ("0", "8", "16") + (("32",) if order == 0 else ()):
+        monkeypatch.setenv("FSLBM_TILE_Y", ty)
+        outs.append(run_gpu(built, ctx, dom, prm, built.F32, f, steps, monitor_every=0)[0])
+    for o in outs[1:]:
+        assert np.array_equal(outs[0], o)
+    fluid = (mask == 0) if rough else np.broadcast_to(mask == 0, f[0].shape)
+    d, want = (outs[0] - ref)[:, fluid], ref[:, fluid]
+    scale = np.abs(want[0]) + 1.5 * (want[1:] ** 2).sum(0)
+    assert np.linalg.norm(d[1:]) <= 1e-5 * np.linalg.norm(want[1:])
+    assert np.linalg.norm(d[0]) <= 1e-5 * np.linalg.norm(scale)
+    assert not outs[0][:, ~fluid].any()
