@@ -1278,14 +1278,13 @@ extern "C" int fslbm_stats_get(fslbm_solve* s, double* out, int* cnt, int* cnt2)
   CUDA_TRY(cudaSetDevice(s->ctx->device));
   if (int r = ensure_stats(s)) return r;
   const size_t n = size_t(s->ly) * (s->L + 2 * s->d2);
-  std::vector<double> acc(22 * n);
-  CUDA_TRY(cudaMemcpyAsync(acc.data(), s->d_stats, 22 * n * sizeof(double), cudaMemcpyDeviceToHost,
-                           s->ctx->stream));
+  double* val = nullptr;                            // compensated sums / counts
+  CUDA_TRY(ctx_alloc(s->ctx, reinterpret_cast<void**>(&val), 11 * n * sizeof(double)));
+  cudaError_t e = launch_stats_value(s->d_stats, n, s->cnt, s->cnt2, val, s->ctx->stream);
+  if (!e) e = cudaMemcpyAsync(out, val, 11 * n * sizeof(double), cudaMemcpyDeviceToHost, s->ctx->stream);
+  ctx_free(s->ctx, val);
+  CUDA_TRY(e);
   CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
-  for (size_t k = 0; k < 11 * n; ++k) {
-    const int c = k < 4 * n ? s->cnt : s->cnt2;
-    out[k] = c ? (acc[k] + acc[11 * n + k]) / double(c) : 0.0;   // compensated sum / count
-  }
   if (cnt) *cnt = s->cnt;
   if (cnt2) *cnt2 = s->cnt2;
   return FSLBM_OK;
@@ -1323,18 +1322,18 @@ extern "C" int fslbm_profile_sample(fslbm_solve* s) {
 extern "C" int fslbm_profile_get(fslbm_solve* s, double* sums, int64_t* nsamples) {
   if (!s || !sums) return fslbm_set_error(FSLBM_ERR_ARG, "profile_get: null argument");
   CUDA_TRY(cudaSetDevice(s->ctx->device));
-  const size_t n = size_t(s->lxp) * s->ly;
-  std::vector<double> buf(20 * n, 0.0);
+  const size_t n = size_t(s->lx) * s->ly;
   if (s->d_prof) {
-    CUDA_TRY(cudaMemcpyAsync(buf.data(), s->d_prof, buf.size() * sizeof(double),
-                             cudaMemcpyDeviceToHost, s->ctx->stream));
+    double* val = nullptr;                          // compensated sums, dense rows
+    CUDA_TRY(ctx_alloc(s->ctx, reinterpret_cast<void**>(&val), 10 * n * sizeof(double)));
+    cudaError_t e = launch_profile_value(s->d_prof, s->lx, s->lxp, s->ly, val, s->ctx->stream);
+    if (!e) e = cudaMemcpyAsync(sums, val, 10 * n * sizeof(double), cudaMemcpyDeviceToHost, s->ctx->stream);
+    ctx_free(s->ctx, val);
+    CUDA_TRY(e);
     CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
+  } else {
+    std::fill(sums, sums + 10 * n, 0.0);
   }
-  for (int k = 0; k < 10; ++k)
-    for (int y = 0; y < s->ly; ++y)
-      for (int x = 0; x < s->lx; ++x)
-        sums[(size_t(k) * s->ly + y) * s->lx + x] =
-            buf[(size_t(k) * s->ly + y) * s->lxp + x] + buf[(size_t(10 + k) * s->ly + y) * s->lxp + x];
   if (nsamples) *nsamples = s->prof_n;
   return FSLBM_OK;
 }

@@ -135,6 +135,10 @@ cudaError_t launch_plane_stats(int dtype, const void* state, const uint8_t* mask
                                int do_fluct, double* acc, cudaStream_t st, const float* wb = nullptr);
 cudaError_t launch_profile(int dtype, const void* state, int lxp, int ly, int L, double* acc,
                            cudaStream_t st, const float* wb = nullptr);
+// Values of the compensated accumulators: (sum + compensation) / count of the 11 plane statistics
+// of n values, and sum + compensation of the 10 profiles as dense ly x lx arrays.
+cudaError_t launch_stats_value(const double* acc, size_t n, int cnt, int cnt2, double* out, cudaStream_t st);
+cudaError_t launch_profile_value(const double* acc, int lx, int lxp, int ly, double* out, cudaStream_t st);
 cudaError_t launch_check(int dtype, const void* state, size_t n_per_field, double* out,
                          cudaStream_t st, int lxp = 0, int ly = 0, const float* wb = nullptr);
 // Converts between the storage type and FP32/FP64 staging buffers (dense per field, pitched).
