@@ -348,19 +348,30 @@ static int build_tensor_maps(fslbm_solve* s) {
   return FSLBM_OK;
 }
 
-// Tile list (tiles holding fluid) for a tile of kTX x th cells.
+// Tile list (tiles holding fluid) for a tile of kTX x th cells, by rows of tiles. Every 32-wide
+// column of tiles starts at its own first fluid row (TMA boxes may start at any row), which saves
+// a tile where the fluid rows fit fewer: 30 instead of 32 tiles of 32 x 16 over the 128 x 128
+// pipe, 4 % of the march over the mixed-size ensemble.
 static std::vector<int2> fluid_tiles(const fslbm_solve* s, int th) {
-  std::vector<int2> tiles;
-  for (int y0 = 0; y0 < s->ly; y0 += th)
-    for (int x0 = 0; x0 < s->lxp; x0 += kTX) {
-      bool any = false;
-      for (int z = 0; z < s->planes && !any; ++z)
-        for (int y = y0; y < std::min(y0 + th, s->ly) && !any; ++y)
-          for (int x = x0; x < std::min(x0 + kTX, s->lxp); ++x)
-            if (s->mask[(size_t(z) * s->ly + y) * s->lxp + x] == 0) { any = true; break; }
-      if (any) tiles.push_back(make_int2(x0, y0));
+  std::vector<std::pair<int, int2>> tiles;            // (row of tiles, origin)
+  std::vector<uint8_t> row(s->ly);
+  for (int x0 = 0; x0 < s->lxp; x0 += kTX) {
+    for (int y = 0; y < s->ly; ++y) {
+      row[y] = 0;
+      for (int z = 0; z < s->planes && !row[y]; ++z)
+        for (int x = x0; x < std::min(x0 + kTX, s->lxp); ++x)
+          if (s->mask[(size_t(z) * s->ly + y) * s->lxp + x] == 0) { row[y] = 1; break; }
     }
-  return tiles;
+    int y0 = 0, k = 0;
+    while (y0 < s->ly && !row[y0]) ++y0;
+    for (; y0 < s->ly; y0 += th, ++k)
+      if (std::any_of(row.begin() + y0, row.begin() + std::min(y0 + th, s->ly), [](uint8_t r) { return r; }))
+        tiles.push_back({k, make_int2(x0, y0)});
+  }
+  std::stable_sort(tiles.begin(), tiles.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+  std::vector<int2> out;
+  for (const auto& t : tiles) out.push_back(t.second);
+  return out;
 }
 
 // Warps of each column-pair tile (32 x ty cells) that hold fluid, for the three warp shapes:
@@ -1384,7 +1395,7 @@ struct fslbm_batch {
   };
   std::vector<Tiling> mt;
   // per member tiling: streamwise planes per work item and warp shape (0: 32 x 2, 1: 16 x 4,
-  // 2: 8 x 8), from the tuning table by size class, else 128 (FSLBM_BATCH_CHUNK) and 16 x 4
+  // 2: 8 x 8), from the tuning table by size class, else 256 (FSLBM_BATCH_CHUNK) and 16 x 4
   std::vector<int> m_chunk, m_shape;
   int shrink = 1;                  // chunk divisor for batches with fewer than 2 items per SM
   cudaGraphExec_t exec2 = nullptr;  // one chained launch of `chain` steps
@@ -1564,7 +1575,7 @@ static std::string class_key(const fslbm_solve* s) {
   return buf;
 }
 
-struct Tiling { int chunk = 128, shape = 1; double ms = 0; };
+struct Tiling { int chunk = 256, shape = 1; double ms = 0; };
 using TilingTable = std::map<std::string, Tiling>;
 
 static bool write_tiling(const char* path, const TilingTable& t) {
@@ -1647,7 +1658,7 @@ extern "C" int fslbm_batch_create(fslbm_ctx* ctx, fslbm_solve* const* solves, in
     }
     b->members.push_back(solves[i]);
     b->stop.push_back(-1);
-    b->m_chunk.push_back(128);
+    b->m_chunk.push_back(256);
     b->m_shape.push_back(1);
     fast = fast && batchable(solves[i]) && solves[i]->dtype == solves[0]->dtype;
   }
