@@ -299,16 +299,16 @@ static int encode_pair_maps(const fslbm_solve* s, int ty, CUtensorMap mp[2], CUt
   return FSLBM_OK;
 }
 
-// Tensor maps of the column-pair kernel's stores into the two state buffers: the four fields of
-// one warp's cells in warp shape `shape` (32 x 2, 16 x 4 or 8 x 8).
-static int encode_store_maps(const fslbm_solve* s, int shape, CUtensorMap mo[2]) {
+// Tensor maps of the pair kernel's stores into the two state buffers: the four fields of one
+// warp's cells, 32 >> shape columns and rows << shape rows.
+static int encode_store_maps(const fslbm_solve* s, int rows, int shape, CUtensorMap mo[2]) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return fslbm_set_error(FSLBM_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
   const CUtensorMapDataType dt = s->dtype == FSLBM_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   cuuint64_t dims[4] = {cuuint64_t(s->lxp), cuuint64_t(s->ly), cuuint64_t(s->L), 4};
   cuuint64_t strides[3] = {cuuint64_t(s->lxp) * s->es, cuuint64_t(s->lxp) * s->ly * s->es,
                            cuuint64_t(field_stride(s)) * s->es};
-  cuuint32_t estr[4] = {1, 1, 1, 1}, box[4] = {cuuint32_t(32 >> shape), cuuint32_t(2 << shape), 1, 4};
+  cuuint32_t estr[4] = {1, 1, 1, 1}, box[4] = {cuuint32_t(32 >> shape), cuuint32_t(rows << shape), 1, 4};
   for (int b = 0; b < 2; ++b) {
     const CUresult r = enc(&mo[b], dt, 4, s->state[b], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -322,7 +322,7 @@ static int encode_store_maps(const fslbm_solve* s, int shape, CUtensorMap mo[2])
 static int build_tensor_maps(fslbm_solve* s) {
   if (s->use2) {
     if (s->dtype != FSLBM_F64)
-      if (int r = encode_store_maps(s, 0, s->maps2o)) return r;
+      if (int r = encode_store_maps(s, step2_rows(s->dtype, s->K, s->planes > 1, s->ty2), 0, s->maps2o)) return r;
     return encode_pair_maps(s, s->ty2, s->maps2p, s->maps2u);
   }
   EncodeTiledFn enc = encode_fn();
@@ -409,11 +409,11 @@ struct Split {
 // iteration, measured on B200 (circular pipes from 32 x 24 x 24 to 512 x 128 x 128, every split).
 // FP32 and FP16 storage march two planes per iteration, two iterations before the first output;
 // FP64 one plane, and its eight planes of fill cost as much as 4.8 output planes. An SM's time per
-// iteration grows with its resident warps (32 x 8 tiles have 4, 32 x 16 have 8, 32 x 32 have 16):
-// 1.35 us for one 32 x 8 tile of FP32 against 2.85 us for a 32 x 32 tile, so few cells per SM want
+// iteration grows with its resident rows of cells:
+// 1.35 us for one 32 x 8 tile of FP32 against 2.7 us for a 32 x 32 tile, so few cells per SM want
 // small tiles (latency) and many cells the large one (fewer halo cells, more warps).
 static double split_us(int dtype, int K, int ty, int per_sm, int sms, int L, int ntiles, int nch) {
-  static const double f32[3][3] = {{1.35, 1.8, 2.45}, {1.7, 0, 0}, {2.85, 0, 0}};
+  static const double f32[3][3] = {{1.35, 1.8, 2.45}, {1.7, 0, 0}, {2.7, 0, 0}};
   static const double f16[3][3] = {{1.93, 2.37, 3.2}, {2.45, 4.05, 0}, {3.94, 0, 0}};
   const int planes = (L + nch - 1) / nch;
   const int64_t ctas = int64_t(ntiles) * nch, waves = (ctas + int64_t(sms) * per_sm - 1) / (int64_t(sms) * per_sm);
@@ -1488,7 +1488,7 @@ static int batch_upload(fslbm_batch* b) {
     fslbm_solve* s = b->members[i];
     fslbm_batch::Tiling& tl = b->mt[i];
     if (tl.mo_shape != b->m_shape[i]) {
-      if (int r = encode_store_maps(s, b->m_shape[i], tl.mo)) return r;
+      if (int r = encode_store_maps(s, 2, b->m_shape[i], tl.mo)) return r;
       tl.mo_shape = b->m_shape[i];
     }
     StepLaunch a{};

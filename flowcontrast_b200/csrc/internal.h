@@ -73,6 +73,7 @@ struct Step2Launch {
 bool step2_supported(int dtype, int d1, int K, bool mp);   // mp: a mask per plane
 bool step2_box(int dtype, int K, int ty, int* sw, int* ph, int* uh, int* hx, int* hy);
 int step2_occupancy(int dtype, int K, int ty);   // CTAs per SM the kernel is built for
+int step2_rows(int dtype, int K, bool mp, int ty);   // rows per thread: a warp stores 32 x rows cells
 cudaError_t step2_prepare(int dtype, int K, bool mp, int ty);
 cudaError_t launch_step2(const StepLaunch& a, const Step2Launch& b, cudaStream_t st);
 

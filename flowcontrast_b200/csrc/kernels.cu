@@ -129,27 +129,27 @@ bool step2_supported(int dtype, int d1, int K, bool mp) {
   return (dtype == FSLBM_F16 || dtype == FSLBM_F64) && K == 2 && !mp;
 }
 
-// Calls fn.template operator()<TY, TE, K, MP>() for the pair kernel of (dtype, K, mask per plane)
-// with tile height ty.
+// Calls fn.template operator()<TY, TE, K, MP, rows per thread>() for the pair kernel of (dtype, K,
+// mask per plane) with tile height ty.
 template <class F> static cudaError_t with_step2(int dtype, int K, bool mp, int ty, F&& fn) {
   if (dtype == FSLBM_F32 && K == 2 && !mp) {
-    if (ty == 32) return fn.template operator()<32, float, 2, false>();
-    if (ty == 16) return fn.template operator()<16, float, 2, false>();
-    if (ty == 8) return fn.template operator()<8, float, 2, false>();
+    if (ty == 32) return fn.template operator()<32, float, 2, false, 4>();
+    if (ty == 16) return fn.template operator()<16, float, 2, false, 2>();
+    if (ty == 8) return fn.template operator()<8, float, 2, false, 2>();
   } else if (dtype == FSLBM_F32 && K == 2) {
-    if (ty == 32) return fn.template operator()<32, float, 2, true>();
-    if (ty == 16) return fn.template operator()<16, float, 2, true>();
-    if (ty == 8) return fn.template operator()<8, float, 2, true>();
+    if (ty == 32) return fn.template operator()<32, float, 2, true, 2>();
+    if (ty == 16) return fn.template operator()<16, float, 2, true, 2>();
+    if (ty == 8) return fn.template operator()<8, float, 2, true, 2>();
   } else if (dtype == FSLBM_F32 && K == 3 && !mp) {     // the window of 32 x 32 tiles exceeds shared memory
-    if (ty == 16) return fn.template operator()<16, float, 3, false>();
-    if (ty == 8) return fn.template operator()<8, float, 3, false>();
+    if (ty == 16) return fn.template operator()<16, float, 3, false, 2>();
+    if (ty == 8) return fn.template operator()<8, float, 3, false, 2>();
   } else if (dtype == FSLBM_F32 && K == 3) {
-    if (ty == 16) return fn.template operator()<16, float, 3, true>();
-    if (ty == 8) return fn.template operator()<8, float, 3, true>();
+    if (ty == 16) return fn.template operator()<16, float, 3, true, 2>();
+    if (ty == 8) return fn.template operator()<8, float, 3, true, 2>();
   } else if (dtype == FSLBM_F16 && K == 2 && !mp) {
-    if (ty == 32) return fn.template operator()<32, __half, 2, false>();
-    if (ty == 16) return fn.template operator()<16, __half, 2, false>();
-    if (ty == 8) return fn.template operator()<8, __half, 2, false>();
+    if (ty == 32) return fn.template operator()<32, __half, 2, false, 2>();
+    if (ty == 16) return fn.template operator()<16, __half, 2, false, 2>();
+    if (ty == 8) return fn.template operator()<8, __half, 2, false, 2>();
   }
   return cudaErrorInvalidValue;
 }
@@ -161,8 +161,8 @@ bool step2_box(int dtype, int K, int ty, int* sw, int* ph, int* uh, int* hx, int
     *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
     return true;
   }
-  return with_step2(dtype, K, false, ty, [&]<int TY, class TE, int KK, bool MP>() {
-           using Tl = Step2Tile<TY, TE, KK>;
+  return with_step2(dtype, K, false, ty, [&]<int TY, class TE, int KK, bool MP, int ROWS>() {
+           using Tl = Step2Tile<TY, TE, KK, ROWS>;
            *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
            return cudaSuccess;
          }) == cudaSuccess;
@@ -170,8 +170,17 @@ bool step2_box(int dtype, int K, int ty, int* sw, int* ph, int* uh, int* hx, int
 
 int step2_occupancy(int dtype, int K, int ty) {
   int n = 1;
-  (void)with_step2(dtype, K, false, ty, [&]<int TY, class TE, int KK, bool MP>() {
-    n = Step2Tile<TY, TE, KK>::CTAS;
+  (void)with_step2(dtype, K, false, ty, [&]<int TY, class TE, int KK, bool MP, int ROWS>() {
+    n = Step2Tile<TY, TE, KK, ROWS>::CTAS;
+    return cudaSuccess;
+  });
+  return n;
+}
+
+int step2_rows(int dtype, int K, bool mp, int ty) {
+  int n = 2;
+  (void)with_step2(dtype, K, mp, ty, [&]<int TY, class TE, int KK, bool MP, int ROWS>() {
+    n = ROWS;
     return cudaSuccess;
   });
   return n;
@@ -182,9 +191,10 @@ cudaError_t step2_prepare(int dtype, int K, bool mp, int ty) {
     return ty != 16 ? cudaErrorInvalidValue
                     : cudaFuncSetAttribute(fslbm_col_kernel<2, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            int(ColTile<2, 16>::SMEM_BYTES));
-  return with_step2(dtype, K, mp, ty, [&]<int TY, class TE, int KK, bool MP>() {
-    return cudaFuncSetAttribute(fslbm_step2_kernel<TY, TE, KK, MP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(Step2Tile<TY, TE, KK>::SMEM_BYTES));
+  return with_step2(dtype, K, mp, ty, [&]<int TY, class TE, int KK, bool MP, int ROWS>() {
+    return cudaFuncSetAttribute(fslbm_step2_kernel<TY, TE, KK, MP, ROWS>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(Step2Tile<TY, TE, KK, ROWS>::SMEM_BYTES));
   });
 }
 
@@ -210,9 +220,9 @@ cudaError_t launch_step2(const StepLaunch& a, const Step2Launch& b, cudaStream_t
     return launch_chained(fslbm_col_kernel<2, 16>, b.grid, ColTile<2, 16>::THREADS,
                           ColTile<2, 16>::SMEM_BYTES, st, *b.map_p, *b.map_uvw, g, kd);
   }
-  return with_step2(a.dtype, a.K, a.mask_planes > 1, b.ty, [&]<int TY, class TE, int KK, bool MP>() {
-    using Tl = Step2Tile<TY, TE, KK>;
-    return launch_chained(fslbm_step2_kernel<TY, TE, KK, MP>, b.grid, Tl::THREADS, Tl::SMEM_BYTES, st, *b.map_p,
+  return with_step2(a.dtype, a.K, a.mask_planes > 1, b.ty, [&]<int TY, class TE, int KK, bool MP, int ROWS>() {
+    using Tl = Step2Tile<TY, TE, KK, ROWS>;
+    return launch_chained(fslbm_step2_kernel<TY, TE, KK, MP, ROWS>, b.grid, Tl::THREADS, Tl::SMEM_BYTES, st, *b.map_p,
                           *b.map_uvw, *b.map_out, g, k);
   });
 }
@@ -473,7 +483,7 @@ __global__ void __launch_bounds__(Step2Tile<TY, TE>::THREADS, Step2Tile<TY, TE>:
 }
 
 cudaError_t batch_prepare(int dtype, int ty) {
-  return with_step2(dtype, 2, false, ty, [&]<int TY, class TE, int K, bool MP>() {
+  return with_step2(dtype, 2, false, ty, [&]<int TY, class TE, int K, bool MP, int ROWS>() {
     if constexpr (TY == 8 || K != 2 || MP) return cudaErrorInvalidValue;
     else
       return cudaFuncSetAttribute(fslbm_step2_batch_kernel<TY, TE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -515,7 +525,7 @@ cudaError_t launch_batch_steps(int dtype, int ty, const void* members, const Bat
   cudaError_t e = cudaMemsetAsync(sync, 0, batch_sync_words(nmembers) * sizeof(unsigned), st);
   if (e) return e;
   const BatchMember* mb = reinterpret_cast<const BatchMember*>(members);
-  return with_step2(dtype, 2, false, ty, [&]<int TY, class TE, int K, bool MP>() {
+  return with_step2(dtype, 2, false, ty, [&]<int TY, class TE, int K, bool MP, int ROWS>() {
     if constexpr (TY == 8 || K != 2 || MP) {
       return cudaErrorInvalidValue;
     } else {

@@ -172,7 +172,7 @@ extern "C" int fslbm_step_f32_noalloc(const float* state_in, float* state_out,
   cuuint32_t boxp[4] = {cuuint32_t(sw), cuuint32_t(ph), 1, 1};
   cuuint32_t boxu[4] = {cuuint32_t(sw), cuuint32_t(uh), 1, 3};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  cuuint32_t boxo[4] = {32, 2, 1, 4};      // one warp's cells, four fields
+  cuuint32_t boxo[4] = {32, cuuint32_t(step2_rows(FSLBM_F32, 2, false, kNoallocTY)), 1, 4};   // one warp's cells, four fields
   CUtensorMap mp, mu, mo;
   CUresult r1 = g_encode(&mp, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(state_in),
                          dims, strides, boxp, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -41,9 +41,9 @@ namespace fslbm {
 // either way. Halo widths and paddings keep every TMA box start and destination on 16 bytes.
 // K is the number of corrector taps per direction (2: the reference's order 2<->4 blend, 3: its
 // order 4<->6 blend).
-template <int TY, class TE = float, int K = 2> struct Step2Tile {
+template <int TY, class TE = float, int K = 2, int ROWS = 2> struct Step2Tile {
   static constexpr int D1 = 2;                          // corrective stride
-  static constexpr int N = 2;                           // rows per thread
+  static constexpr int N = ROWS;                        // rows per thread
   static constexpr int ES = int(sizeof(TE));
   static constexpr int A16 = 16 / ES;                   // elements per 16 bytes
   static constexpr int TX = 32;
@@ -211,17 +211,20 @@ __device__ __forceinline__ void tm_load(float2 (&v)[2], uint32_t a) {
                : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y) : "r"(a) : "memory");
 }
 __device__ __forceinline__ void tm_wait_stores() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tm_load(float2 (&v)[4], uint32_t a) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y), "=f"(v[3].x),
+                 "=f"(v[3].y)
+               : "r"(a) : "memory");
+}
 // Completes the loads into v: their uses cannot move before the wait.
-#define FSLBM_TM_REGS(i) "+f"(v[i][0].x), "+f"(v[i][0].y), "+f"(v[i][1].x), "+f"(v[i][1].y)
-__device__ __forceinline__ void tm_wait_loads(float2 (&v)[4][2]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : FSLBM_TM_REGS(0), FSLBM_TM_REGS(1), FSLBM_TM_REGS(2), FSLBM_TM_REGS(3)::"memory");
+template <int M, int N> __device__ __forceinline__ void tm_wait_loads(float2 (&v)[M][N]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < M; ++j)
+#pragma unroll
+    for (int r = 0; r < N; ++r) asm volatile("" : "+f"(v[j][r].x), "+f"(v[j][r].y));
 }
-__device__ __forceinline__ void tm_wait_loads(float2 (&v)[5][2]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : FSLBM_TM_REGS(0), FSLBM_TM_REGS(1), FSLBM_TM_REGS(2), FSLBM_TM_REGS(3), FSLBM_TM_REGS(4)::"memory");
-}
-#undef FSLBM_TM_REGS
 // Allocation of a kernel's tensor memory by its first warp (whole warp); `slot` in shared memory
 // receives the base address. Freed by the same warp before the kernel ends, on every path.
 template <int COLS> __device__ __forceinline__ void tm_alloc(uint32_t* slot) {
@@ -243,12 +246,12 @@ template <int COLS> __device__ __forceinline__ void tm_free(uint32_t base) {
 // cross-sections. With the 160-byte FP32 row stride the shapes 0 and 1 read shared memory without
 // bank conflicts (rows 2 apart are 16 banks apart), shape 2 two-way. The map changes no thread's
 // arithmetic.
-template <int TY, class TE, int K = 2, bool MP = false>
+template <int TY, class TE, int K = 2, bool MP = false, int ROWS = 2>
 __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUtensorMap* tmap_uvw,
                                             const CUtensorMap* tmap_out, uint32_t tmem, const Step2Geom& g,
                                             const StepConst<float>& k, int tile, int chunk,
                                             unsigned char* smem, bool reinit, int shape) {
-  using Tl = Step2Tile<TY, TE, K>;
+  using Tl = Step2Tile<TY, TE, K, ROWS>;
   constexpr int N = Tl::N, R = Tl::R, D1 = Tl::D1, HX = Tl::HX, HY = Tl::HY, SW = Tl::SW, SU = Tl::SU, SP = Tl::SP;
   constexpr int PPL = Tl::PPL, UPL = Tl::UPL, VPL = Tl::VPL;
   TE* uring = reinterpret_cast<TE*>(smem);
@@ -448,9 +451,10 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   for (int j = 0; j < K - 2; ++j) release(j);
   // iteration q: predictor of pair q, which completes the sums of pair q - 1, and from q = K + 1 on
   // corrector and update of the output pair q - 1
-  // Two iterations per pass rename the carried registers instead of moving them (FP32, one
-  // cross-section: 4679 -> 4550 us per 50 steps at 512 x 128 x 128); the others would spill.
-  constexpr int kPass = !MP && !kBase ? 2 : 1;
+  // Two iterations per pass rename the carried registers instead of moving them (FP32, two rows
+  // per thread, one cross-section: -3 %); the other forms would spill or outgrow the instruction
+  // cache (four rows: 4718 against 4415 us per 50 steps at 512 x 128 x 128).
+  constexpr int kPass = !MP && !kBase && N == 2 ? 2 : 1;
 #pragma unroll kPass
   for (int q = K - 1; q <= nstage - K; ++q) {
     if (!arrive_wait(q + K - 1)) {
@@ -648,17 +652,27 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
 #pragma unroll
       for (int r = 0; r < N; ++r)
         put(0, r, fma2(fma2(pc[r], f2(ws0[r]), cp[r][0]), f2(1.0f / 216.0f), f2(-gauge)));
+      // own columns of pairs q, q - 1, ...: with kAhead the next field's arrive while a field is
+      // computed (-1 % on the FP32 32 x 32 tile, -2 % with FP16 storage; in the FP32 batched
+      // kernel the registers spill, +5 %)
+      constexpr bool kAhead = N == 4 || kBase;
+      float2 rings[kAhead ? 2 : 1][K + 2][N];
+      auto load_ring = [&](int f) {
+#pragma unroll
+        for (int j = 0; j < K + 2; ++j) tm_load(rings[kAhead ? f & 1 : 0][j], tm_slot(q - j) + f * 2 * N);
+      };
+      if (kAhead) load_ring(0);
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
         const TE* b = sub + f * UPL;
-        float2 ring[K + 2][N];                               // own columns of pairs q, q - 1, ...
-#pragma unroll
-        for (int j = 0; j < K + 2; ++j) tm_load(ring[j], tm_slot(q - j) + f * 2 * N);
+        float2 (&ring)[K + 2][N] = rings[kAhead ? f & 1 : 0];
+        if (!kAhead) load_ring(f);
         float2 c[N + 2 * R];                                 // rows -R .. N + R - 1 of the own column
 #pragma unroll
         for (int j = -R; j < N + R; ++j)
           if (j < 0 || j >= N) c[j + R] = ldu(b + j * SW);
         tm_wait_loads(ring);
+        if (kAhead && f < 2) load_ring(f + 1);
 #pragma unroll
         for (int r = 0; r < N; ++r) c[r + R] = ring[1][r];
 #pragma unroll
@@ -706,13 +720,13 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
 }
 
 // One pipe, one step: CTA b marches (tile b % ntiles, chunk b / ntiles).
-template <int TY, class TE, int K = 2, bool MP = false>
-__global__ void __launch_bounds__(Step2Tile<TY, TE, K>::THREADS, Step2Tile<TY, TE, K>::CTAS)
+template <int TY, class TE, int K = 2, bool MP = false, int ROWS = 2>
+__global__ void __launch_bounds__(Step2Tile<TY, TE, K, ROWS>::THREADS, Step2Tile<TY, TE, K, ROWS>::CTAS)
     fslbm_step2_kernel(const __grid_constant__ CUtensorMap tmap_p,
                        const __grid_constant__ CUtensorMap tmap_uvw,
                        const __grid_constant__ CUtensorMap tmap_out, const Step2Geom g,
                        const StepConst<float> k) {
-  using Tl = Step2Tile<TY, TE, K>;
+  using Tl = Step2Tile<TY, TE, K, ROWS>;
   extern __shared__ __align__(128) unsigned char smem[];
   uint32_t* tm_base = reinterpret_cast<uint32_t*>(smem + Tl::REL_OFFSET) + Tl::SU;
   if (threadIdx.x < 32) tm_alloc<Tl::TM_COLS>(tm_base);
@@ -720,7 +734,7 @@ __global__ void __launch_bounds__(Step2Tile<TY, TE, K>::THREADS, Step2Tile<TY, T
   if (threadIdx.x == 0 && blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
   __syncthreads();
   const uint32_t tmem = *tm_base;
-  step2_march<TY, TE, K, MP>(&tmap_p, &tmap_uvw, &tmap_out, tmem, g, k, blockIdx.x % g.ntiles, blockIdx.x / g.ntiles, smem,
+  step2_march<TY, TE, K, MP, ROWS>(&tmap_p, &tmap_uvw, &tmap_out, tmem, g, k, blockIdx.x % g.ntiles, blockIdx.x / g.ntiles, smem,
                       false, 0);
   grid_launch_dependents();   // not earlier: waiting CTAs of the next step would share this one's SMs
   __syncthreads();
