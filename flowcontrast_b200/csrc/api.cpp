@@ -199,7 +199,7 @@ struct fslbm_solve {
   int cur = 0;
   uint8_t* d_mask = nullptr;
   void* d_colcoef = nullptr;
-  uint8_t* d_near = nullptr;       // masks per plane, FP32: code per cell, then per column (see step2_march)
+  uint32_t* d_near = nullptr;      // masks per plane, FP32: packed wall sums per cell, then per column (step2_march)
   int2* d_tiles = nullptr;
   int ntiles = 0, chunk = 0, nchunks = 0;
   CUtensorMap maps[2];
@@ -534,6 +534,32 @@ static std::vector<CellCoef<TC>> cell_coefs(const fslbm_solve* s) {
   return cc;
 }
 
+// Packed wall sums of every cell for masks that vary along z (pack_wall_sums), then one value per
+// column: kSolidCell where no plane has fluid, else 0.
+static std::vector<uint32_t> packed_cell_sums(const fslbm_solve* s) {
+  const size_t plane = size_t(s->lxp) * s->ly;
+  std::vector<uint32_t> near(plane * (size_t(s->L) + 1), kSolidCell);
+  for (int z = 0; z < s->L; ++z)
+    for (int y = 0; y < s->ly; ++y)
+      for (int x = 0; x < s->lxp; ++x) {
+        const size_t c = size_t(y) * s->lxp + x;
+        if (s->mask[z * plane + c] == kWall) continue;
+        int a = 0, bx = 0, by = 0, bz = 0;
+        for (int dz = -1; dz <= 1; ++dz)
+          for (int dy = -1; dy <= 1; ++dy)
+            for (int dx = -1; dx <= 1; ++dx) {
+              const int gx = x + dx, gy = y + dy, gz = (z + dz + s->L) % s->L;
+              if (gx >= 0 && gy >= 0 && gx < s->lxp && gy < s->ly && s->mask[gz * plane + size_t(gy) * s->lxp + gx] != kWall)
+                continue;
+              const int w = (dx ? 1 : 4) * (dy ? 1 : 4) * (dz ? 1 : 4);
+              a += w; bx += w * dx; by += w * dy; bz += w * dz;
+            }
+        near[z * plane + c] = pack_wall_sums(a, bx, by, bz);
+        near[plane * s->L + c] = 0;
+      }
+  return near;
+}
+
 // Picks the streamwise chunking: minimises waves * (chunk + 2R) over chunk counts.
 static void choose_chunks(fslbm_solve* s) {
   int occ = 1;
@@ -734,14 +760,9 @@ extern "C" int fslbm_solve_create(fslbm_ctx* ctx, const fslbm_domain* dom, const
     auto cc = cell_coefs<float>(s);
     if ((e = dalloc(s, &s->d_colcoef, cc.size() * sizeof(cc[0])))) return fail("colcoef");
     e = cudaMemcpyAsync(s->d_colcoef, cc.data(), cc.size() * sizeof(cc[0]), cudaMemcpyHostToDevice, st);
-    std::vector<uint8_t> near(cc.size() + plane, 2);   // per cell, then per column over all planes
-    for (size_t j = 0; j < cc.size(); ++j) {
-      if (s->mask[j] == kWall) continue;
-      near[j] = cc[j].ws0 != 0.0f ? 1 : 0;
-      near[cc.size() + j % plane] = 1;
-    }
-    if (!e) e = dalloc(s, &s->d_near, near.size());
-    if (!e) e = cudaMemcpyAsync(s->d_near, near.data(), near.size(), cudaMemcpyHostToDevice, st);
+    const std::vector<uint32_t> near = packed_cell_sums(s);
+    if (!e) e = dalloc(s, &s->d_near, near.size() * sizeof(near[0]));
+    if (!e) e = cudaMemcpyAsync(s->d_near, near.data(), near.size() * sizeof(near[0]), cudaMemcpyHostToDevice, st);
     if (!e) e = cudaStreamSynchronize(st);
   } else if (dtype == FSLBM_F64) {
     auto cc = column_coefs<double>(s);
@@ -925,8 +946,8 @@ extern "C" int fslbm_solve_footprint(const fslbm_domain* dom, fslbm_dtype dtype,
   const int64_t cc = dtype == FSLBM_F64 ? int64_t(sizeof(ColCoef<double>)) : int64_t(sizeof(ColCoef<float>));
   const int64_t tiles = ((lxp + kTX - 1) / kTX) * ((dom->ly + kTY - 1) / kTY) * int64_t(sizeof(int2));
   const int64_t masks = dom->mask_planes > 1
-                            ? cs + cs * dom->lz * (1 + int64_t(dtype == FSLBM_F64 ? sizeof(CellCoef<double>)
-                                                                                : sizeof(CellCoef<float>) + 1))
+                            ? 4 * cs + cs * dom->lz * (1 + int64_t(dtype == FSLBM_F64 ? sizeof(CellCoef<double>)
+                                                                                : sizeof(CellCoef<float>) + 4))
                             : cs + cs * cc;
   const int64_t wtabs = dtype == FSLBM_F16 ? 2 * cs * int64_t(sizeof(float)) : 0;
   *bytes = 2 * 4 * fs * es + masks + tiles + wtabs + int64_t(sizeof(DevCounters)) +

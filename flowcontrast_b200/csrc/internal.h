@@ -48,7 +48,7 @@ struct StepLaunch {
   int mask_planes;           // 0/1: extruded cross-section; L: a mask (and CellCoef) per plane
   const float* wb;           // FP16 storage: per-column base of w and its step share, else null
   const float* wgt;
-  const uint8_t* near;       // masks per plane, FP32: code per cell (0 fluid, 1 beside a wall, 2 wall), else null
+  const uint32_t* near;      // masks per plane, FP32: packed wall sums per cell (pack_wall_sums), else null
   // constants in double; converted to the compute type by the launcher
   double tb, cc, pin, dtddy, m, c0, c1, c2, fx, fy, fz;
   double ch[6];              // corrector coefficients c3..c8

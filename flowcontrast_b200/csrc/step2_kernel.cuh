@@ -105,7 +105,7 @@ struct Step2Geom {
   // of the stored w. Null for other storage types.
   const float* wb;
   const float* wgt;
-  const uint8_t* near;     // masks per plane: code per cell (see step2_march), else null
+  const uint32_t* near;    // masks per plane: packed wall sums per cell (pack_wall_sums), else null
 };
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
@@ -276,21 +276,26 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   const int x = org.x + tx, y0 = org.y + ty;
 
   // Warps that compute (some fluid) and warps over fluid away from walls (no wall sums). With a
-  // mask per plane (MP) the codes in g.near tell, per cell: 0 fluid without a wall neighbour,
-  // 1 fluid beside a wall, 2 wall; one more plane holds 2 for the columns without any fluid.
+  // mask per plane (MP) g.near holds every cell's wall sums; one more plane holds kSolidCell for
+  // the columns without any fluid.
   const size_t cplane = size_t(g.lxp) * g.ly;
   const long long col = (long long)y0 * g.lxp + x;
   auto coef = [&](int r) {             // extruded masks; outside the cross-section: nothing
     return x < g.lxp && y0 + r < g.ly ? reinterpret_cast<const ColCoef<float>*>(g.colcoef)[col + r * g.lxp]
                                       : ColCoef<float>{0.f, 0.f, 0.f, 0.f};
   };
-  auto near_code = [&](int r, int z) -> unsigned {
-    return x < g.lxp && y0 + r < g.ly ? g.near[z * cplane + col + r * g.lxp] : 2u;
+  // The load is volatile and its address always valid, so nothing waits for it before its use a
+  // predictor later; cells outside the cross-section are settled there.
+  auto inside = [&](int r) { return x < g.lxp && y0 + r < g.ly; };
+  auto walls = [&](int r, int z) -> uint32_t {
+    uint32_t m;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(m) : "l"(g.near + (inside(r) ? z * cplane + col + r * g.lxp : 0)));
+    return m;
   };
   bool some = false, every = true;
   if constexpr (MP) {
 #pragma unroll
-    for (int r = 0; r < N; ++r) some |= near_code(r, g.L) != 2u;   // over all planes
+    for (int r = 0; r < N; ++r) some |= inside(r) && walls(r, g.L) != kSolidCell;   // over all planes
   } else {
 #pragma unroll
     for (int r = 0; r < N; ++r) {
@@ -469,6 +474,17 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
 #pragma unroll
     for (int j = 0; j < K - 1; ++j) sua[j] = uring + unsigned(q + 1 + j) % unsigned(SU) * (2 * VPL) + uo;
     const int zp = start + dir * 2 * q;                                           // real plane of the pair's first
+    // the output pair's wall sums (MP), loaded a predictor ahead of their use
+    const bool second = 2 * (q - 1 - K) + 1 < nout;          // the chunk's plane count may be odd
+    uint32_t code[N][2];
+    if constexpr (MP) {
+      const int z0 = q > K ? zp - 2 * dir : zb, z1 = q > K && second ? zp - dir : z0;
+#pragma unroll
+      for (int r = 0; r < N; ++r) {
+        code[r][0] = walls(r, z0);
+        code[r][1] = walls(r, z1);
+      }
+    }
     float nfirst[N][4];                  // finished sums of pair q's first plane
     float2 pcen[N];
     {
@@ -579,7 +595,6 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
     if (q > K) {
       tm_wait_stores();
       const int zo = zp - 2 * dir;                           // real plane of the output pair's first
-      const bool second = 2 * (q - 1 - K) + 1 < nout;        // the chunk's plane count may be odd
       // wall sums (times 216) and fluid flag of the rows: one value for both planes of an extruded mask
       using Sum = std::conditional_t<MP, float2, float>;
       auto both = [](float a, float b) {
@@ -593,28 +608,26 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
         fluid[r] = both(1.f, 1.f);
       }
       if constexpr (MP) {
-        const int z1 = second ? zo + dir : zo;
-        unsigned code[N][2], any = 0;
+        uint32_t any = 0;
 #pragma unroll
         for (int r = 0; r < N; ++r) {
-          code[r][0] = near_code(r, zo);
-          code[r][1] = near_code(r, z1);
+          if (!inside(r)) code[r][0] = code[r][1] = kSolidCell;
           any |= code[r][0] | code[r][1];
         }
         if (__any_sync(0xffffffffu, any != 0u)) {
-          const CellCoef<float>* cells = reinterpret_cast<const CellCoef<float>*>(g.colcoef) + col;
 #pragma unroll
-          for (int r = 0; r < N; ++r)
-            if (x < g.lxp && y0 + r < g.ly) {
-              const CellCoef<float> a = cells[zo * cplane + r * g.lxp], b = cells[z1 * cplane + r * g.lxp];
-              ws0[r] = make_float2(216.f * a.ws0, 216.f * b.ws0);
-              wsx[r] = make_float2(216.f * a.wsx, 216.f * b.wsx);
-              wsy[r] = make_float2(216.f * a.wsy, 216.f * b.wsy);
-              wsz[r] = make_float2(216.f * float(dir) * a.wsz, 216.f * float(dir) * b.wsz);
-            }
-#pragma unroll
-          for (int r = 0; r < N; ++r)
-            fluid[r] = make_float2(code[r][0] == 2u ? 0.f : 1.f, code[r][1] == 2u ? 0.f : 1.f);
+          for (int r = 0; r < N; ++r) {
+            auto sums = [&](uint32_t m, float& s0, float& sx, float& sy, float& sz, float& fl) {
+              auto field = [&](int at) { return float(int(m << (25 - at)) >> 25); };
+              s0 = float(m & 255u);
+              sx = field(8);
+              sy = field(15);
+              sz = float(dir) * field(22);
+              fl = m & kSolidCell ? 0.f : 1.f;
+            };
+            sums(code[r][0], ws0[r].x, wsx[r].x, wsy[r].x, wsz[r].x, fluid[r].x);
+            sums(code[r][1], ws0[r].y, wsx[r].y, wsy[r].y, wsz[r].y, fluid[r].y);
+          }
         }
       } else if (!plain_column) {
 #pragma unroll
