@@ -30,11 +30,55 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
+// Host buffers for the submitted start fields, handed from request to request: a fresh buffer costs
+// a page fault per 4 KB it is filled with, and the allocator returns buffers of this size to the
+// system. Held buffers are bounded (kHold floats) and freed with the server; a buffer serves only
+// requests that fill at least half of it. Not zeroed: every value is copied over.
+class StartBuffers {
+ public:
+  struct Buffer {
+    std::unique_ptr<float[]> data;
+    size_t size = 0;
+  };
+  Buffer take(size_t n) {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      auto best = free_.end();
+      for (auto it = free_.begin(); it != free_.end(); ++it)
+        if (it->size >= n && it->size <= 2 * n && (best == free_.end() || it->size < best->size)) best = it;
+      if (best != free_.end()) {
+        Buffer b = std::move(*best);
+        free_.erase(best);
+        held_ -= b.size;
+        return b;
+      }
+    }
+    return Buffer{std::unique_ptr<float[]>(new float[n]), n};
+  }
+  void give(Buffer b) {
+    if (!b.data) return;
+    std::lock_guard<std::mutex> lk(mu_);
+    if (b.size > kHold) return;
+    while (!free_.empty() && held_ + b.size > kHold) {   // drop the oldest
+      held_ -= free_.front().size;
+      free_.pop_front();
+    }
+    held_ += b.size;
+    free_.push_back(std::move(b));
+  }
+
+ private:
+  static constexpr size_t kHold = size_t(64) << 20;      // 256 MB
+  std::mutex mu_;
+  std::deque<Buffer> free_;
+  size_t held_ = 0;
+};
+
 struct Request {
   int64_t id = 0;
   fslbm_request req{};
   std::vector<uint8_t> mask;      // copy of req.domain.mask
-  std::vector<float> init;        // copy of the host start, 4 * cells, if given
+  StartBuffers::Buffer init;      // copy of the host start, 4 * cells, if given, until the solve has it
   fslbm_result res{};
   fslbm_solve* solve = nullptr;   // worker-owned while running
   int64_t left = 0;
@@ -64,6 +108,7 @@ struct fslbm_server {
   bool stop = false;
   std::deque<ReqPtr> queue;                 // waiting for admission, arrival order
   std::map<int64_t, ReqPtr> table;          // every request not yet released
+  StartBuffers buffers;
   int64_t next_id = 1;
   fslbm_server_stats st{};
   Clock::time_point t0;
@@ -101,10 +146,11 @@ int start_request(fslbm_server* S, const ReqPtr& r) {
   fslbm_solve* s = nullptr;
   int rc = fslbm_solve_create(S->ctx, &dom, &r->req.params, fslbm_dtype(r->req.dtype), &s);
   if (rc) return rc;
-  if (!r->init.empty()) {
+  if (r->init.data) {
     const size_t n = size_t(r->res.cells);
-    const float* f = r->init.data();
+    const float* f = r->init.data.get();
     rc = fslbm_solve_set_fields(s, FSLBM_F32, f, f + n, f + 2 * n, f + 3 * n);
+    S->buffers.give(std::move(r->init));   // a copy from pageable memory has read it on return
   } else {
     const fslbm_init_spec& q = r->req.init_spec;
     rc = fslbm_solve_init_poiseuille(s, q.umax, q.noise, q.modes, q.mode_amp, q.seed);
@@ -395,8 +441,8 @@ extern "C" int fslbm_server_submit(fslbm_server* S, const fslbm_request* req, in
   r->req.domain.mask = nullptr;
   if (all_init) {
     const size_t n = size_t(r->res.cells);
-    r->init.resize(4 * n);
-    for (int f = 0; f < 4; ++f) std::memcpy(r->init.data() + f * n, req->init[f], n * sizeof(float));
+    r->init = S->buffers.take(4 * n);
+    for (int f = 0; f < 4; ++f) std::memcpy(r->init.data.get() + f * n, req->init[f], n * sizeof(float));
     for (int f = 0; f < 4; ++f) r->req.init[f] = nullptr;
   }
   {
