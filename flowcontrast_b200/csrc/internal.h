@@ -69,6 +69,7 @@ struct Step2Launch {
   const CUtensorMap* map_uvw;
   const CUtensorMap* map_out;  // output state, box of one warp's cells (not the FP64 kernel)
   int grid;
+  bool fresh_tables = false;   // the stream's previous kernel writes tiles or colcoef (pair kernel only)
 };
 bool step2_supported(int dtype, int d1, int K, bool mp);   // mp: a mask per plane
 bool step2_box(int dtype, int K, int ty, int* sw, int* ph, int* uh, int* hx, int* hy);

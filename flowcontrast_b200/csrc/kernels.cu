@@ -203,7 +203,7 @@ cudaError_t launch_step2(const StepLaunch& a, const Step2Launch& b, cudaStream_t
   g.lxp = a.lxp; g.ly = a.ly; g.L = a.L; g.ntiles = a.ntiles; g.nchunks = b.grid / a.ntiles;
   g.tiles = a.tiles; g.mask = a.mask; g.colcoef = a.colcoef; g.out = a.out;
   g.gauge = a.gauge; g.err = a.err;
-  g.wb = a.wb; g.wgt = a.wgt; g.near = a.near;
+  g.wb = a.wb; g.wgt = a.wgt; g.near = a.near; g.early = !b.fresh_tables;
   g.step_counter = a.counters ? &a.counters->steps : nullptr;
   g.step_no = unsigned(a.step_no);
   StepConst<float> k{};
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(Step2Tile<TY, TE>::THREADS, Step2Tile<TY, TE>:
       const int cur = mb.cur0 ^ (step & 1);
       const int ntiles = mb.g.ntiles;
       ok = step2_march<TY, TE>(&mb.map_p[cur], &mb.map_u[cur], &mb.map_o[1 - cur], tmem, s_g, s_k,
-                               it.y % ntiles, it.y / ntiles, smem, !first, mb.shape);
+                               it.y % ntiles, it.y / ntiles, smem, !first, mb.shape, false);
       first = false;
     }
   }

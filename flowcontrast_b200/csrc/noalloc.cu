@@ -214,7 +214,7 @@ extern "C" int fslbm_step_f32_noalloc(const float* state_in, float* state_out,
   int nch = g_sm_count[dev] / a.ntiles;
   if (nch > (lz + 1) / 2) nch = (lz + 1) / 2;
   if (nch < 1) nch = 1;
-  Step2Launch b{kNoallocTY, &mp, &mu, &mo, a.ntiles * nch};
+  Step2Launch b{kNoallocTY, &mp, &mu, &mo, a.ntiles * nch, true};
   if ((e = launch_step2(a, b, st)) != cudaSuccess)
     return fslbm_set_error(FSLBM_ERR_CUDA, "step_f32_noalloc: step launch: %s", cudaGetErrorString(e));
 

@@ -105,6 +105,7 @@ struct Step2Geom {
   // of the stored w. Null for other storage types.
   const float* wb;
   const float* wgt;
+  bool early;              // tiles, colcoef and near are older than the previous kernel of the stream
   const uint32_t* near;    // masks per plane: packed wall sums per cell (pack_wall_sums), else null
 };
 
@@ -238,7 +239,8 @@ template <int COLS> __device__ __forceinline__ void tm_free(uint32_t base) {
 
 // Marches one (tile, chunk) work item of one pipe: the step of every cell of the tile's columns
 // in the chunk's planes. `tmem` is the CTA's tensor memory, `reinit` re-arms the CTA's mbarriers
-// when the CTA has marched an item before (persistent grids). Returns false when a bounded wait
+// when the CTA has marched an item before (persistent grids), `chained` waits for the stream's
+// previous kernel before the state is read. Returns false when a bounded wait
 // gave up (error flag set). The results are complete (visible to this thread) on return.
 // The warp shape is a runtime argument: it only places each thread in the tile. 0: 32 columns x
 // 2 rows; 1: 16 columns x 4 rows; 2: 8 columns x 8 rows (a thread's two rows are adjacent in all
@@ -250,7 +252,7 @@ template <int TY, class TE, int K = 2, bool MP = false, int ROWS = 2>
 __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUtensorMap* tmap_uvw,
                                             const CUtensorMap* tmap_out, uint32_t tmem, const Step2Geom& g,
                                             const StepConst<float>& k, int tile, int chunk,
-                                            unsigned char* smem, bool reinit, int shape) {
+                                            unsigned char* smem, bool reinit, int shape, bool chained) {
   using Tl = Step2Tile<TY, TE, K, ROWS>;
   constexpr int N = Tl::N, R = Tl::R, D1 = Tl::D1, HX = Tl::HX, HY = Tl::HY, SW = Tl::SW, SU = Tl::SU, SP = Tl::SP;
   constexpr int PPL = Tl::PPL, UPL = Tl::UPL, VPL = Tl::VPL;
@@ -275,6 +277,42 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   const int2 org = g.tiles[tile];
   const int x = org.x + tx, y0 = org.y + ty;
 
+  __syncthreads();   // a previous item (persistent grids) is fully consumed
+  if (tid == 0) {
+    for (int s = 0; s < SU; ++s) {
+      if (reinit) mbar_inval(&full[s]);
+      mbar_init(&full[s], 1);
+      released[s] = 0u;
+    }
+    mbar_init_fence();
+  }
+  // stage j: u,v,w of the plane pair j (march planes 2j, 2j + 1) and p of the pair j - K + 1, which
+  // the predictor reads in the iteration that waits for this stage
+  auto plane_of = [&](int m) {
+    int zz = start + dir * m;
+    if (zz < 0 || zz >= g.L) zz %= g.L;
+    return zz < 0 ? zz + g.L : zz;
+  };
+  auto issue = [&](int j) {
+    uint64_t* bar = &full[unsigned(j) % unsigned(SU)];
+    const bool with_p = j >= 2 * K - 2;
+    mbar_arrive_expect_tx(bar, 2 * Tl::U_BYTES + (with_p ? 2 * Tl::P_BYTES : 0u));
+    TE* du = uring + unsigned(j) % unsigned(SU) * (2 * VPL);
+    tma_load_4d(du, tmap_uvw, bar, org.x - HX, org.y - HY, plane_of(2 * j), 1);
+    tma_load_4d(du + VPL, tmap_uvw, bar, org.x - HX, org.y - HY, plane_of(2 * j + 1), 1);
+    if (with_p) {
+      const int m = 2 * (j - K + 1);
+      TE* dp = pring + unsigned(j - K + 1) % unsigned(SP) * (2 * PPL);
+      tma_load_4d(dp, tmap_p, bar, org.x - HX, org.y - 1, plane_of(m), 0);
+      tma_load_4d(dp + PPL, tmap_p, bar, org.x - HX, org.y - 1, plane_of(m + 1), 0);
+    }
+  };
+  if (tid == 0) {                      // the whole window up front, before the wall tables are read
+    prefetch_tensormap(tmap_p);
+    prefetch_tensormap(tmap_uvw);
+    if (chained) grid_dependency_wait();
+    for (int j = 0; j < SU && j < nstage; ++j) issue(j);
+  }
   // Warps that compute (some fluid) and warps over fluid away from walls (no wall sums). With a
   // mask per plane (MP) g.near holds every cell's wall sums; one more plane holds kSolidCell for
   // the columns without any fluid.
@@ -307,16 +345,8 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   const bool warp_on = __any_sync(0xffffffffu, some);
   const bool plain_column = __all_sync(0xffffffffu, every);
 
-  __syncthreads();   // a previous item (persistent grids) is fully consumed
-  if (tid == 0) {
-    for (int s = 0; s < SU; ++s) {
-      if (reinit) mbar_inval(&full[s]);
-      mbar_init(&full[s], 1);
-      released[s] = 0u;
-    }
-    mbar_init_fence();
-  }
   // FP16 storage: the tile's base of w (zero outside the cross-section), read by the predictor
+  if (chained) grid_dependency_wait();
   constexpr bool kBase = std::is_same<TE, __half>::value;
   float* wbs = reinterpret_cast<float*>(smem + Tl::BASE_OFFSET);
   if (kBase && g.wb)
@@ -326,32 +356,6 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
     }
   __syncthreads();
 
-  // stage j: u,v,w of the plane pair j (march planes 2j, 2j + 1) and p of the pair j - K + 1, which
-  // the predictor reads in the iteration that waits for this stage
-  auto plane_of = [&](int m) {
-    int zz = start + dir * m;
-    if (zz < 0 || zz >= g.L) zz %= g.L;
-    return zz < 0 ? zz + g.L : zz;
-  };
-  auto issue = [&](int j) {
-    uint64_t* bar = &full[unsigned(j) % unsigned(SU)];
-    const bool with_p = j >= 2 * K - 2;
-    mbar_arrive_expect_tx(bar, 2 * Tl::U_BYTES + (with_p ? 2 * Tl::P_BYTES : 0u));
-    TE* du = uring + unsigned(j) % unsigned(SU) * (2 * VPL);
-    tma_load_4d(du, tmap_uvw, bar, org.x - HX, org.y - HY, plane_of(2 * j), 1);
-    tma_load_4d(du + VPL, tmap_uvw, bar, org.x - HX, org.y - HY, plane_of(2 * j + 1), 1);
-    if (with_p) {
-      const int m = 2 * (j - K + 1);
-      TE* dp = pring + unsigned(j - K + 1) % unsigned(SP) * (2 * PPL);
-      tma_load_4d(dp, tmap_p, bar, org.x - HX, org.y - 1, plane_of(m), 0);
-      tma_load_4d(dp + PPL, tmap_p, bar, org.x - HX, org.y - 1, plane_of(m + 1), 0);
-    }
-  };
-  if (tid == 0) {                      // the whole window up front
-    prefetch_tensormap(tmap_p);
-    prefetch_tensormap(tmap_uvw);
-    for (int j = 0; j < SU && j < nstage; ++j) issue(j);
-  }
   // Wait for stage j; false after flagging a failure (the caller returns). Then any warp may have
   // issued loads up to SU stages ahead: let them land (bounded).
   auto arrive_wait = [&](int j) -> bool {
@@ -743,13 +747,13 @@ __global__ void __launch_bounds__(Step2Tile<TY, TE, K, ROWS>::THREADS, Step2Tile
   extern __shared__ __align__(128) unsigned char smem[];
   uint32_t* tm_base = reinterpret_cast<uint32_t*>(smem + Tl::REL_OFFSET) + Tl::SU;
   if (threadIdx.x < 32) tm_alloc<Tl::TM_COLS>(tm_base);
-  grid_dependency_wait();
-  if (threadIdx.x == 0 && blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
+  if (!g.early) grid_dependency_wait();
   __syncthreads();
   const uint32_t tmem = *tm_base;
-  step2_march<TY, TE, K, MP, ROWS>(&tmap_p, &tmap_uvw, &tmap_out, tmem, g, k, blockIdx.x % g.ntiles, blockIdx.x / g.ntiles, smem,
-                      false, 0);
+  step2_march<TY, TE, K, MP, ROWS>(&tmap_p, &tmap_uvw, &tmap_out, tmem, g, k, blockIdx.x % g.ntiles, blockIdx.x / g.ntiles,
+                                   smem, false, 0, true);
   grid_launch_dependents();   // not earlier: waiting CTAs of the next step would share this one's SMs
+  if (threadIdx.x == 0 && blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
   __syncthreads();
   if (threadIdx.x < 32) tm_free<Tl::TM_COLS>(tmem);
 }

@@ -84,13 +84,6 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
   const int x = org.x + tx, y = org.y + ty;
   const bool inside = x < g.lxp && y < g.ly;
 
-  double ws0 = 0, wsx = 0, wsy = 0, fl = 0;
-  if (inside) {
-    const ColCoef<double> c = reinterpret_cast<const ColCoef<double>*>(g.colcoef)[size_t(y) * g.lxp + x];
-    ws0 = c.ws0; wsx = c.wsx; wsy = c.wsy; fl = c.fluid;
-  }
-  const bool warp_on = __any_sync(0xffffffffu, fl != 0.0);
-
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(&full[s], 1);
@@ -98,7 +91,6 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
     }
     mbar_init_fence();
   }
-  __syncthreads();
 
   auto issue = [&](int m) {            // load march plane m into its slot
     const int slot = slot_of(m);
@@ -112,8 +104,18 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
   if (tid == 0) {                      // the whole ring up front
     prefetch_tensormap(tmap_p);
     prefetch_tensormap(tmap_uvw);
+    grid_dependency_wait();
     for (int m = 0; m < S && m < niter; ++m) issue(m);
   }
+  double ws0 = 0, wsx = 0, wsy = 0, fl = 0;
+  if (inside) {
+    const ColCoef<double> c = reinterpret_cast<const ColCoef<double>*>(g.colcoef)[size_t(y) * g.lxp + x];
+    ws0 = c.ws0; wsx = c.wsx; wsy = c.wsy; fl = c.fluid;
+  }
+  const bool warp_on = __any_sync(0xffffffffu, fl != 0.0);
+
+  grid_dependency_wait();
+  __syncthreads();
   auto drain = [&](int from) {         // failure path: let this CTA's loads land (bounded)
     if (lane == 0)
       for (int q = from; q < niter && q < from + S; ++q)
@@ -335,9 +337,8 @@ __global__ void __launch_bounds__(ColTile<D1, TY>::THREADS, 1)
                      const __grid_constant__ CUtensorMap tmap_uvw, const Step2Geom g,
                      const StepConst<double> k) {
   extern __shared__ __align__(128) unsigned char smem[];
-  grid_dependency_wait();
-  if (threadIdx.x == 0 && blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
   col_march<D1, TY>(&tmap_p, &tmap_uvw, g, k, blockIdx.x % g.ntiles, blockIdx.x / g.ntiles, smem);
+  if (threadIdx.x == 0 && blockIdx.x == 0 && g.step_counter) *g.step_counter += 1;
   grid_launch_dependents();
 }
 
