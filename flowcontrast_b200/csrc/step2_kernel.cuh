@@ -672,7 +672,7 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
       // own columns of pairs q, q - 1, ...: with kAhead the next field's arrive while a field is
       // computed (-1 % on the FP32 32 x 32 tile, -2 % with FP16 storage; in the FP32 batched
       // kernel the registers spill, +5 %)
-      constexpr bool kAhead = N == 4 || kBase;
+      constexpr bool kAhead = N == 4 || kBase || TY < 32;
       float2 rings[kAhead ? 2 : 1][K + 2][N];
       auto load_ring = [&](int f) {
 #pragma unroll
