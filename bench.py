@@ -34,9 +34,9 @@ E2E_INNER = 200                   # time steps per end-to-end solve request
 METRIC = "MLUPS (plain FSLBM step, all box cells)"
 # plain workload's storage types (--dtype): library type, bytes per value, step kernel, the
 # line's dtype (the arithmetic type; FP16 storage computes in FP32)
-STORAGE = {"f32": ("F32", 4, "fslbm_step2_kernel<2,32,packed>", "f32"),
+STORAGE = {"f32": ("F32", 4, "fslbm_step2_kernel<32,float>", "f32"),
            "f64": ("F64", 8, "fslbm_col_kernel<2,16>", "f64"),
-           "f16": ("F16", 2, "fslbm_step2_kernel<2,32,packed,__half>", "f16 storage, f32 arithmetic")}
+           "f16": ("F16", 2, "fslbm_step2_kernel<32,__half>", "f16 storage, f32 arithmetic")}
 
 
 def physics():
@@ -435,12 +435,10 @@ def _member_start(fb, s, sp):
 
 
 def batch_kernel_name(storage):
-    """The batched kernel the library launches: 32 x 16 tiles unless FSLBM_BATCH_TILE_Y=32,
-    packed pair arithmetic unless FSLBM_BATCH_PACKED=0."""
-    ty = 32 if os.environ.get("FSLBM_BATCH_TILE_Y") == "32" else 16
-    form = "scalar" if os.environ.get("FSLBM_BATCH_PACKED") == "0" else "packed"
+    """The batched kernel the library launches: 32 x 32 tiles unless FSLBM_BATCH_TILE_Y=16."""
+    ty = 16 if os.environ.get("FSLBM_BATCH_TILE_Y") == "16" else 32
     te = "__half" if storage == "f16" else "float"
-    return f"fslbm_step2_batch_kernel<2,{ty},{form},{te}> (chained steps)"
+    return f"fslbm_step2_batch_kernel<{ty},{te}> (chained steps)"
 
 
 def ensemble_line(args):

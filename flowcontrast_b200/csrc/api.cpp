@@ -203,7 +203,7 @@ struct fslbm_solve {
   int2* d_tiles = nullptr;
   int ntiles = 0, chunk = 0, nchunks = 0;
   CUtensorMap maps[2];
-  // FP32 column-pair kernel (even d1): tile height, persistent grid, two maps per buffer
+  // pair kernel or FP64 column kernel (d1 = 2): tile height, grid, maps per buffer
   bool use2 = false;
   int ty2 = 32, grid2 = 0;
   CUtensorMap maps2p[2], maps2u[2], maps2o[2];
@@ -268,7 +268,7 @@ static int validate_params(const fslbm_params* p, int dtype) {
   return FSLBM_OK;
 }
 
-// Tensor maps of the column-pair kernel with tile height ty over the solve's two state buffers:
+// Tensor maps of the pair kernel with tile height ty over the solve's two state buffers:
 // the p box (one-cell halo) and the u,v,w box (the corrector's halo) of the loads.
 static int encode_pair_maps(const fslbm_solve* s, int ty, CUtensorMap mp[2], CUtensorMap mu[2]) {
   EncodeTiledFn enc = encode_fn();
@@ -374,7 +374,7 @@ static std::vector<int2> fluid_tiles(const fslbm_solve* s, int th) {
   return out;
 }
 
-// Warps of each column-pair tile (32 x ty cells) that hold fluid, for the three warp shapes:
+// Warps of each pair-kernel tile (32 x ty cells) that hold fluid, for the three warp shapes:
 // warps[0] 32 x 2 cells, warps[1] 16 x 4 cells, warps[2] 8 x 8 cells (the kernel's lane maps).
 static void tile_warp_counts(const fslbm_solve* s, const std::vector<int2>& tiles, int ty,
                              std::vector<int> (&warps)[3]) {
@@ -445,7 +445,7 @@ static Split choose_split(const fslbm_solve* s, int only_ty) {
 
 // Selects the step kernel for the current dtype and d1, uploads its tile list, builds its
 // tensor maps and sizes its grid. FSLBM_STEP_KERNEL=1 forces the one-column kernel and
-// FSLBM_TILE_Y=8|16|32 picks the column-pair kernel's tile height (for comparisons).
+// FSLBM_TILE_Y=8|16|32 picks the pair kernel's tile height (for comparisons).
 static int configure_kernel(fslbm_solve* s) {
   const char* ek = std::getenv("FSLBM_STEP_KERNEL");
   const char* et = std::getenv("FSLBM_TILE_Y");
@@ -1402,10 +1402,11 @@ struct fslbm_batch {
   std::vector<int2> h_items;
   std::vector<int2> item_shape;    // per member: (tiles, chunks) the item table was built for
   int nitems = 0, grid = 0;
-  // the batch's own column-pair tiling of every member (32 x ty tiles, one height for the whole
-  // batch): tile list, fluid warps per tile for the two warp shapes, tensor maps of both buffers.
-  // 32 x 16 tiles, two 256-thread CTAs per SM: on the 64-pipe ensemble (cross-sections 24..96)
-  // +1.0 % against 32 x 32 tiles; the members' own single-pipe tiling is not affected
+  // the batch's own tiling of every member (32 x ty tiles, one height for the whole batch): tile
+  // list, fluid warps per tile for the three warp shapes, tensor maps of both buffers. 32 x 32
+  // tiles, one 512-thread CTA per SM: the pair kernel's window of 32 x 16 tiles (118 KB for FP32)
+  // leaves an SM one such CTA of 8 warps, which is slower on the 64-pipe ensemble (cross-sections
+  // 24..96) at every chunk and warp shape; the members' own single-pipe tiling is not affected
   int ty = 32;
   struct Tiling {
     int ntiles = 0;
@@ -1441,7 +1442,7 @@ static void free_batch(fslbm_batch* b) {
   ctx_release(c);
 }
 
-// Work of one (tile, chunk) item of the column-pair kernel, for ordering the items: planes
+// Work of one (tile, chunk) item of the pair kernel, for ordering the items: planes
 // marched (the chunk plus the 2R pipeline planes) times the tile's warps that compute plus two
 // for the pipeline's fixed cost.
 static int64_t item_cost(const fslbm_solve* s, const std::vector<int> (&warps)[3], int tile, int nout,
@@ -1455,7 +1456,7 @@ static bool batchable(const fslbm_solve* s) {
   return s->use2 && s->K == 2 && s->planes == 1 && s->dtype != FSLBM_F64 && s->nghost == 0;
 }
 
-// Resident CTAs of the batched kernel: one per SM for 32 x 32 tiles, two for 32 x 16 tiles.
+// Resident CTAs of the batched kernel: one per SM, two for 32 x 16 tiles of FP16 storage.
 static int batch_slots(const fslbm_batch* b) {
   return b->ctx->sm_count * step2_occupancy(b->members[0]->dtype, 2, b->ty);
 }

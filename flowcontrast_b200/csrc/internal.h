@@ -97,7 +97,7 @@ cudaError_t launch_monitor(const MonitorLaunch& a, cudaStream_t st);
 cudaError_t launch_wait_selftest(const unsigned* counter, unsigned long long limit_ns, unsigned* err,
                                  cudaStream_t st);
 
-// ---- batched ensemble (column-pair kernel, d1 = 2, tile height 16 or 32 for the whole batch)
+// ---- batched ensemble (pair kernel, d1 = 2, tile height 16 or 32 for the whole batch)
 struct BatchMon {
   MonitorLaunch mon;           // state is chosen per launch from `state`
   const void* state[2];

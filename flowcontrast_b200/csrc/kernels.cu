@@ -86,7 +86,7 @@ bool step_supported(int dtype, int d1, int K) {
 #define X(DT, TS, D, KK) if (dtype == DT && d1 == D && K == KK) return true;
   FSLBM_STEP_COMBOS(X)
 #undef X
-  if (dtype == FSLBM_F16) return d1 == 2 && K == 2;   // column-pair kernel only
+  if (dtype == FSLBM_F16) return d1 == 2 && K == 2;   // pair kernel only
   return false;
 }
 
@@ -121,7 +121,7 @@ cudaError_t launch_step(const StepLaunch& a, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------------------------------
-// column-pair kernel (FP32 / FP16 storage) and FP64 column kernel dispatch
+// pair kernel (FP32 / FP16 storage) and FP64 column kernel dispatch
 // ------------------------------------------------------------------------------------------
 bool step2_supported(int dtype, int d1, int K, bool mp) {
   if (d1 != 2) return false;

@@ -21,7 +21,7 @@ using namespace fslbm;
 
 constexpr int kNoallocMaxCells = 65536;   // lx_pitch * ly of the cross-section
 constexpr int kNoallocMaxTiles = 2048;
-constexpr int kNoallocTY = 32;            // tile height of the FP32 column-pair kernel used here
+constexpr int kNoallocTY = 32;            // tile height of the FP32 pair kernel used here
 constexpr size_t kCoefBytes = size_t(kNoallocMaxCells) * sizeof(ColCoef<float>);
 constexpr size_t kTileBytes = size_t(kNoallocMaxTiles) * sizeof(int2);
 constexpr size_t kGaugeOffset = kCoefBytes + kTileBytes;

@@ -1,13 +1,13 @@
 // FSLBM time step, FP64 column kernel for sm_100a (d1 = 2, the reference's order 2<->4 corrector).
 //
-// The column-pair kernel's pipeline (step2_kernel.cuh) with one FP64 column per thread:
+// Planes marched one at a time, one FP64 column per thread:
 //  - a 32 x 16 tile per CTA, 512 threads, one warp per tile row: a warp's 64-bit shared loads
 //    read 32 consecutive doubles (two wavefronts, no bank conflict); 16 warps per SM;
 //  - p is staged with a one-cell halo and u,v,w with the corrector's 2*d1 halo, as two TMA boxes
 //    per plane (no multicast) into a window of 7 planes (201 KB);
 //  - no block-wide barrier in the march and no producer thread: per-slot "full" mbarriers count
 //    TMA completion, planes leave the window in pairs and the last warp to release a pair
-//    refills both slots (the protocol of step2_march, same bounded waits and failure path);
+//    refills both slots (the bounded waits and failure path of step2_march);
 //  - the predictor is row-factored per column, the streamwise corrector taps behind the output
 //    plane come from a register history of the thread's own column, the taps ahead from the
 //    window; the update is folded as in the FP32 kernel;

@@ -61,10 +61,10 @@ typedef struct {
   int buffer_depth;      /* d2 of the reference layout used by plane dumps and statistics */
   int mask_planes;       /* 0 or 1: `mask` is one cross-section extruded along z; lz: `mask`
                             holds lx*ly*lz values, one cross-section per plane (geometry that
-                            varies along the pipe, such as wall roughness; run on the one-column
-                            kernel, FP32/FP64). The monitor's l1, the reference's buffer-cell
-                            count over 2*d2 planes (FSLBM.cu:589-591), is then the mean fluid
-                            count of the buffer_depth planes at each end of the core. */
+                            varies along the pipe, such as wall roughness; FP32/FP64). The
+                            monitor's l1, the reference's buffer-cell count over 2*d2 planes
+                            (FSLBM.cu:589-591), is then the mean fluid count of the
+                            buffer_depth planes at each end of the core. */
   int periodic_xy;       /* addition: G > 0 makes the cross-section periodic in x and y with
                             period (lx - 2G, ly - 2G): a G-wide band at the box rim holds the
                             periodic images of the interior (mask value 2; refilled after every
@@ -87,8 +87,8 @@ typedef struct {
                            4<->2 blend; 6 = 6<->4 and 8 = 8<->6 blends (blend weights the higher
                            order; the paper's pipes used 6 with blend 0.4); 10, 12, 14 = fixed
                            sets (blend unused). Orders above 4 reach K*d1 cells (K = 3, 4, 5, 6,
-                           8) and run on the one-column kernel: FP32 with K*d1 <= 8, FP64 with
-                           K*d1 <= 4; FP16 storage supports orders 0/4 only. Not in param.txt. */
+                           8): FP32 with K*d1 <= 8, FP64 with K*d1 <= 4; FP16 storage supports
+                           orders 0/4 only. Not in param.txt. */
 } fslbm_params;
 
 /* One monitor record (FSLBM.cu:632-666): means over the first fluid plane (q1, p1) and over the
