@@ -408,7 +408,7 @@ struct Split {
 // resident per SM: each wave of CTAs costs a launch and pipeline fill and then a time per march
 // iteration, measured on B200 (circular pipes from 32 x 24 x 24 to 512 x 128 x 128, every split).
 // FP32 and FP16 storage march two planes per iteration, two iterations before the first output;
-// FP64 one plane, and its eight planes of fill cost as much as 4.8 output planes. An SM's time per
+// FP64 one plane, and its eight planes of fill cost as much as 4.3 output planes. An SM's time per
 // iteration grows with its resident rows of cells:
 // 1.35 us for one 32 x 8 tile of FP32 against 2.7 us for a 32 x 32 tile, so few cells per SM want
 // small tiles (latency) and many cells the large one (fewer halo cells, more warps).
@@ -417,7 +417,7 @@ static double split_us(int dtype, int K, int ty, int per_sm, int sms, int L, int
   static const double f16[3][3] = {{1.93, 2.37, 3.2}, {2.45, 4.05, 0}, {3.94, 0, 0}};
   const int planes = (L + nch - 1) / nch;
   const int64_t ctas = int64_t(ntiles) * nch, waves = (ctas + int64_t(sms) * per_sm - 1) / (int64_t(sms) * per_sm);
-  if (dtype == FSLBM_F64) return double(waves) * 1.3 * (planes + 4.8);
+  if (dtype == FSLBM_F64) return double(waves) * 1.28 * (planes + 4.3);
   const double tau = (dtype == FSLBM_F16 ? f16 : f32)[ty == 8 ? 0 : (ty == 16 ? 1 : 2)][per_sm - 1];
   return double(waves) * (2.0 + tau * ((planes + 1) / 2 + K));
 }

@@ -142,44 +142,54 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// x sums of one row at one column (two planes). With weights {4,1,1} over cx = 0, +1, -1 (R) or
-// the difference +1 minus -1 (D), of the terms of the brackets as polynomials of cy:
+template <class V> __device__ __forceinline__ V cst(float a);
+template <> __device__ __forceinline__ float2 cst<float2>(float a) { return f2(a); }
+template <> __device__ __forceinline__ double cst<double>(float a) { return double(a); }
+__device__ __forceinline__ double add2(double a, double b) { return __dadd_rn(a, b); }   // FP64: one plane
+__device__ __forceinline__ double neg2(double a) { return -a; }
+__device__ __forceinline__ double sub2(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double mul2(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double fma2(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// x sums of one row at one column (V = float2: two planes; double: one plane, the FP64 kernel). With
+// weights {4,1,1} over cx = 0, +1, -1 (R) or the difference +1 minus -1 (D), of the terms of the
+// brackets as polynomials of cy:
 //   0: q + 3 cx u + 4.5 cx^2 u^2        (P0 at cy = 0)
 //   1: v (1 + 3 cx u)                   (P0 = 0 + 3 cy 1 + 4.5 cy^2 2)
 //   2: v^2
 //   z: w (1 + 3 cx u)                   (P1/3 = z + 3 cy m)
 //   m: v w
 //   w: w^2                              (P2/4.5)
-struct RowSums {
-  float2 R0, D0, R1, D1, R2, D2, Rz, Dz, Rm, Dm, Rw, Dw;
+template <class V> struct RowSums {
+  V R0, D0, R1, D1, R2, D2, Rz, Dz, Rm, Dm, Rw, Dw;
 };
-__device__ __forceinline__ float2 rsum(float2 l, float2 c, float2 r) { return fma2(f2(4.0f), c, add2(l, r)); }
+template <class V> __device__ __forceinline__ V rsum(V l, V c, V r) { return fma2(cst<V>(4.0f), c, add2(l, r)); }
 
-__device__ __forceinline__ RowSums row_sums(const float2 (&p)[3], const float2 (&u)[3], const float2 (&v)[3],
-                                            const float2 (&w)[3]) {
-  float2 P[3], V[3], V2[3], W[3], M[3], W2[3];
+template <class V>
+__device__ __forceinline__ RowSums<V> row_sums(const V (&p)[3], const V (&u)[3], const V (&v)[3], const V (&w)[3]) {
+  V P[3], V1[3], V2[3], W[3], M[3], W2[3];
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     V2[j] = mul2(v[j], v[j]);
     W2[j] = mul2(w[j], w[j]);
     M[j] = mul2(v[j], w[j]);
-    const float2 s = add2(V2[j], W2[j]);
+    const V s = add2(V2[j], W2[j]);
     if (j == 1) {
-      P[j] = fma2(neg2(fma2(u[j], u[j], s)), f2(1.5f), p[j]);
-      V[j] = v[j];
+      P[j] = fma2(neg2(fma2(u[j], u[j], s)), cst<V>(1.5f), p[j]);
+      V1[j] = v[j];
       W[j] = w[j];
     } else {
-      const float2 cu = j == 2 ? u[j] : neg2(u[j]);          // cx u
-      const float2 a = fma2(cu, f2(3.0f), f2(1.0f));
+      const V cu = j == 2 ? u[j] : neg2(u[j]);               // cx u
+      const V a = fma2(cu, cst<V>(3.0f), cst<V>(1.0f));
       // q + 3 cx u + 4.5 u^2 = p - 1.5 (v^2 + w^2) + cx u (3 cx u + 3)
-      P[j] = fma2(cu, fma2(cu, f2(3.0f), f2(3.0f)), fma2(neg2(s), f2(1.5f), p[j]));
-      V[j] = mul2(v[j], a);
+      P[j] = fma2(cu, fma2(cu, cst<V>(3.0f), cst<V>(3.0f)), fma2(neg2(s), cst<V>(1.5f), p[j]));
+      V1[j] = mul2(v[j], a);
       W[j] = mul2(w[j], a);
     }
   }
-  RowSums o;
+  RowSums<V> o;
   o.R0 = rsum(P[0], P[1], P[2]);   o.D0 = sub2(P[2], P[0]);
-  o.R1 = rsum(V[0], V[1], V[2]);   o.D1 = sub2(V[2], V[0]);
+  o.R1 = rsum(V1[0], V1[1], V1[2]); o.D1 = sub2(V1[2], V1[0]);
   o.R2 = rsum(V2[0], V2[1], V2[2]); o.D2 = sub2(V2[2], V2[0]);
   o.Rz = rsum(W[0], W[1], W[2]);   o.Dz = sub2(W[2], W[0]);
   o.Rm = rsum(M[0], M[1], M[2]);   o.Dm = sub2(M[2], M[0]);
@@ -188,16 +198,16 @@ __device__ __forceinline__ RowSums row_sums(const float2 (&p)[3], const float2 (
 }
 
 // A row's contribution to the output row one above (cy = -1) or below (cy = +1) it.
-struct RowSide {
-  float2 R0, D0, Rz, Dz, Rw, Dw;
+template <class V> struct RowSide {
+  V R0, D0, Rz, Dz, Rw, Dw;
 };
-template <int CY> __device__ __forceinline__ RowSide row_side(const RowSums& o) {
-  auto cy = [](float2 a) { return CY > 0 ? a : neg2(a); };
-  RowSide s;
-  s.R0 = fma2(cy(o.R1), f2(3.0f), fma2(f2(4.5f), o.R2, o.R0));
-  s.D0 = fma2(cy(o.D1), f2(3.0f), fma2(f2(4.5f), o.D2, o.D0));
-  s.Rz = fma2(cy(o.Rm), f2(3.0f), o.Rz);
-  s.Dz = fma2(cy(o.Dm), f2(3.0f), o.Dz);
+template <int CY, class V> __device__ __forceinline__ RowSide<V> row_side(const RowSums<V>& o) {
+  auto cy = [](V a) { return CY > 0 ? a : neg2(a); };
+  RowSide<V> s;
+  s.R0 = fma2(cy(o.R1), cst<V>(3.0f), fma2(cst<V>(4.5f), o.R2, o.R0));
+  s.D0 = fma2(cy(o.D1), cst<V>(3.0f), fma2(cst<V>(4.5f), o.D2, o.D0));
+  s.Rz = fma2(cy(o.Rm), cst<V>(3.0f), o.Rz);
+  s.Dz = fma2(cy(o.Dm), cst<V>(3.0f), o.Dz);
   s.Rw = o.Rw;
   s.Dw = o.Dw;
   return s;
@@ -492,8 +502,8 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
     float nfirst[N][4];                  // finished sums of pair q's first plane
     float2 pcen[N];
     {
-      RowSide above, here;               // rows r - 1 and r as their lower neighbours see them
-      RowSums mid;
+      RowSide<float2> above, here;       // rows r - 1 and r as their lower neighbours see them
+      RowSums<float2> mid;
 #pragma unroll
       for (int j = -1; j <= N; ++j) {
         float2 p3[3], u3[3], v3[3], w3[3];
@@ -516,10 +526,10 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
         if (kBase && g.wb)               // w = stored deviation + the column's base
 #pragma unroll
           for (int c = 0; c < 3; ++c) w3[c] = add2(w3[c], f2(wbs[(ty + 1 + j) * Tl::BW + tx + c]));
-        const RowSums row = row_sums(p3, u3, v3, w3);
+        const RowSums<float2> row = row_sums(p3, u3, v3, w3);
         if (j >= 1) {
           const int r = j - 1;
-          const RowSide below = row_side<1>(row);
+          const RowSide<float2> below = row_side<1>(row);
           // row-factored weights w(cx)w(cy) = {4,1,1}x{4,1,1}/36: A, X (cx moment), Y (cy moment)
           float2 A[3], X[3], Y[3];
           A[0] = fma2(f2(4.0f), mid.R0, add2(above.R0, below.R0));

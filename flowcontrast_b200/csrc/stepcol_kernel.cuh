@@ -1,22 +1,26 @@
 // FSLBM time step, FP64 column kernel for sm_100a (d1 = 2, the reference's order 2<->4 corrector).
 //
-// Planes marched one at a time, one FP64 column per thread:
-//  - a 32 x 16 tile per CTA, 512 threads, one warp per tile row: a warp's 64-bit shared loads
-//    read 32 consecutive doubles (two wavefronts, no bank conflict); 16 warps per SM;
+// Planes marched one at a time, two FP64 rows of one column per thread:
+//  - a 32 x 16 tile per CTA, 256 threads, two tile rows per warp: a warp's 64-bit shared loads
+//    read 32 consecutive doubles (two wavefronts, no bank conflict);
 //  - p is staged with a one-cell halo and u,v,w with the corrector's 2*d1 halo, as two TMA boxes
 //    per plane (no multicast) into a window of 7 planes (201 KB);
 //  - no block-wide barrier in the march and no producer thread: per-slot "full" mbarriers count
 //    TMA completion, planes leave the window in pairs and the last warp to release a pair
 //    refills both slots (the bounded waits and failure path of step2_march);
-//  - the predictor is row-factored per column, the streamwise corrector taps behind the output
-//    plane come from a register history of the thread's own column, the taps ahead from the
-//    window; the update is folded as in the FP32 kernel;
+//  - the predictor is step2_march's (x sums per row, carried times 216), the streamwise corrector
+//    taps behind the output plane come from a register history of the thread's own column, the
+//    taps ahead from the window, the output plane's centre from the predictor one plane earlier;
 //  - grid = tiles x streamwise chunks in chunk-major order, odd chunks marching downwards, and a
 //    cell's predictor adds its two neighbour planes' shares before its own plane's, so results do
 //    not depend on the chunking.
-// It replaces the one-column kernel of step_kernel.cuh (one block barrier per plane, a single
-// 4-field box with the corrector halo on p too, 8 warps per SM) for FP64 solves with d1 = 2 and
-// the 2-tap corrector; other orders, strides and per-plane masks keep that kernel.
+// The shared-memory path bounds it (64 % of its wavefront slots; FP64 pipe 45 %). Two rows per
+// thread share the predictor's rows: 54 shared loads per cell against 70 with one row and 512
+// threads, 166 against 177 us a step at 512 x 128 x 128; the predictor's arithmetic per cell stays
+// the same and 8 warps instead of 16 are enough (64 x 32 x 32: 6.8 us either way). Measured and not
+// used: the plane two ahead carried into the predictor (51 loads, 1 % slower), the predictor
+// instantiated apart for the seam planes (2 % slower).
+// FP64 solves with other corrector orders, strides or masks per plane keep step_kernel.cuh.
 #pragma once
 #include <cstdint>
 #include <cuda.h>
@@ -31,7 +35,8 @@ namespace fslbm {
 template <int D1, int TY> struct ColTile {
   static constexpr int ES = int(sizeof(double));
   static constexpr int TX = 32;
-  static constexpr int THREADS = TX * TY;
+  static constexpr int N = 2;                           // rows per thread
+  static constexpr int THREADS = TX * TY / N;
   static constexpr int WARPS = THREADS / 32;
   static constexpr int R = 2 * D1;                      // farthest corrector tap
   static constexpr int HX = (R * ES + 15) / 16 * 16 / ES;   // x halo, TMA-aligned (16 bytes)
@@ -62,7 +67,7 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
                                           int chunk, unsigned char* smem) {
   using Tl = ColTile<D1, TY>;
   static_assert(D1 == 2, "the march prologue below is written for d1 = 2 (R = 4)");
-  constexpr int R = Tl::R, HX = Tl::HX, HY = Tl::HY, SW = Tl::SW, S = Tl::S;
+  constexpr int N = Tl::N, R = Tl::R, HX = Tl::HX, HY = Tl::HY, SW = Tl::SW, S = Tl::S;
   constexpr int PPL = Tl::PPLANE, UPL = Tl::UPLANE, SLOT = Tl::SLOT;
 
   auto slot_of = [](int m) { return int(unsigned(m) % unsigned(S)); };
@@ -72,7 +77,7 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
   unsigned* released = reinterpret_cast<unsigned*>(full + S);
 
   const int tid = threadIdx.x, lane = tid & 31;
-  const int tx = lane, ty = tid >> 5;                  // one warp per tile row
+  const int tx = lane, ty = (tid >> 5) * N;            // N tile rows per warp
 
   // ---- work: one (tile, chunk); odd chunks march towards -z
   const int zb = int((long long)g.L * chunk / g.nchunks);
@@ -81,8 +86,7 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
   const int nout = ze - zb, niter = nout + 2 * R;
   const int start = dir > 0 ? zb - R : ze - 1 + R;      // real plane of march index 0
   const int2 org = g.tiles[tile];
-  const int x = org.x + tx, y = org.y + ty;
-  const bool inside = x < g.lxp && y < g.ly;
+  const int x = org.x + tx, y0 = org.y + ty;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -107,12 +111,20 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
     grid_dependency_wait();
     for (int m = 0; m < S && m < niter; ++m) issue(m);
   }
-  double ws0 = 0, wsx = 0, wsy = 0, fl = 0;
-  if (inside) {
-    const ColCoef<double> c = reinterpret_cast<const ColCoef<double>*>(g.colcoef)[size_t(y) * g.lxp + x];
-    ws0 = c.ws0; wsx = c.wsx; wsy = c.wsy; fl = c.fluid;
+  // wall sums of the predictor (times 216, see the march) and fluid flag; nothing outside the box
+  double ws0[N], wsx[N], wsy[N], fl[N];
+  bool inside[N], some = false;
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    inside[r] = x < g.lxp && y0 + r < g.ly;
+    ws0[r] = wsx[r] = wsy[r] = fl[r] = 0;
+    if (inside[r]) {
+      const ColCoef<double> c = reinterpret_cast<const ColCoef<double>*>(g.colcoef)[size_t(y0 + r) * g.lxp + x];
+      ws0[r] = 216.0 * c.ws0; wsx[r] = 216.0 * c.wsx; wsy[r] = 216.0 * c.wsy; fl[r] = c.fluid;
+    }
+    some |= fl[r] != 0.0;
   }
-  const bool warp_on = __any_sync(0xffffffffu, fl != 0.0);
+  const bool warp_on = __any_sync(0xffffffffu, some);
 
   grid_dependency_wait();
   __syncthreads();
@@ -152,161 +164,168 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
 
   const double gauge = g.gauge ? __ldcg(g.gauge) : 0.0;
   const size_t FS = size_t(g.lxp) * g.ly * g.L;
-  double* outp = reinterpret_cast<double*>(g.out) + (size_t(start + dir * R) * g.ly + y) * g.lxp + x;
+  double* outp = reinterpret_cast<double*>(g.out) + (size_t(start + dir * R) * g.ly + y0) * g.lxp + x;
   const long long ostep = (long long)dir * g.ly * g.lxp;     // output pointer step per plane
   const int po = (ty + 1) * SW + HX + tx;                     // p box
   const int uo = PPL + (ty + HY) * SW + HX + tx;              // u box (v, w at +UPL, +2 UPL)
-  // seam pressure jump: off times the non-wall weight sums (raw units, x36) on A0, X0, Y0
-  const double n0 = 36.0 - 36.0 * ws0, nx = -36.0 * wsx, ny = -36.0 * wsy;
-  const double h6 = double(dir) / 72.0;
+  const double dir3 = 3.0 * double(dir);
   // folded update: u_new = K1 t1 + K2 t2 + K0 u + tb (u* + F)
   const double kam = __dmul_rn(__dmul_rn(k.tb, k.dtddy), k.m);
   const double kK0 = __fma_rn(kam, k.c0, k.cc), kK1 = __dmul_rn(kam, k.c1), kK2 = __dmul_rn(kam, k.c2);
-  const double ktz = double(dir) * k.tb;
+  // the predictor's moments come times 216; the z-moment carries the march direction's sign
+  const double ktb = __ddiv_rn(k.tb, 216.0), ktz = double(dir) * ktb;
 
-  double hu[4], hv[4], hw[4];          // own column of planes jo-4..jo-1
-  // b2: the march-previous plane's share of the output being completed, b1: the same for the
-  // next output, s1: the self-plane moments of the next output (see step2_march)
-  double b2[4], b1[4], s1[3];
+  // own column of the four planes before the output plane: [field][plane parity][older, newer][row]
+  double h[3][2][2][N];
+  // per row: d2 / d1 = the shares that the two planes before the next predictor plane give to their
+  // march-next planes (d2 to the output being completed), s1 = the self-plane moments of the newer
+  double d2[N][3], d1[N][3], s1[N][3], comp[N][4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    hu[j] = hv[j] = hw[j] = 0.0;
-    b2[j] = b1[j] = 0.0;
-    if (j < 3) s1[j] = 0.0;
-  }
-  double comp0 = 0, comp1 = 0, comp2 = 0, comp3 = 0;
+  for (int r = 0; r < N; ++r)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      comp[r][j] = 0.0;
+      if (j < 3) d2[r][j] = d1[r][j] = s1[r][j] = h[j][0][0][r] = h[j][0][1][r] = h[j][1][0][r] = h[j][1][1][r] = 0.0;
+    }
 
-  // predictor contribution of march plane ma (factorisation: step_kernel.cuh, step2_march)
+  double cen[N][4], nxt[N][4];         // p, u, v, w of the output plane and of the one after it
+
+  // predictor contribution of march plane ma (factorisation and scaling: step2_march)
   auto predictor = [&](int ma) {
     const double* ss = ring + slot_of(ma) * SLOT;
     const int sp = start + dir * ma;
-    double A[3], X[3], Y[3];
+    RowSide<double> above, here;         // rows r - 1 and r as their lower neighbours see them
+    RowSums<double> mid;
 #pragma unroll
-    for (int cy = -1; cy <= 1; ++cy) {
-      const double* rp = ss + po + cy * SW;
-      const double* rq = ss + uo + cy * SW;
-      double q3[3], u3[3], v3[3], w3[3], w23[3];
+    for (int j = -1; j <= N; ++j) {
+      double p3[3], u3[3], v3[3], w3[3];
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const double pv = rp[j - 1];
-        u3[j] = rq[j - 1];
-        v3[j] = rq[UPL + j - 1];
-        w3[j] = rq[2 * UPL + j - 1];
-        w23[j] = __dmul_rn(w3[j], w3[j]);
-        q3[j] = __fma_rn(-1.5, __fma_rn(u3[j], u3[j], __fma_rn(v3[j], v3[j], w23[j])), pv);
+      for (int c = 0; c < 3; ++c) {
+        const double* rq = ss + uo + j * SW + c - 1;
+        p3[c] = ss[po + j * SW + c - 1];
+        u3[c] = rq[0];
+        v3[c] = rq[UPL];
+        w3[c] = rq[2 * UPL];
       }
-      double P[3][3];   // [cx+1][k]
-#pragma unroll
-      for (int cx = -1; cx <= 1; ++cx) {
-        const int j = cx + 1;
-        const double u = u3[j], v = v3[j], w = w3[j];
-        double P0, P1;
-        if (cx == 0 && cy == 0) {
-          P0 = q3[j];
-          P1 = w;
-        } else if (cx == 0 || cy == 0) {
-          const double Bv = cy == 0 ? u : v;
-          const double s3 = 3.0 * double(cx + cy);
-          P0 = __fma_rn(Bv, __fma_rn(Bv, 4.5, s3), q3[j]);
-          P1 = __dmul_rn(w, __fma_rn(Bv, s3, 1.0));
-        } else {
-          const double a1 = __fma_rn(v, double(cx * cy), u);
-          const double s3 = 3.0 * double(cx);
-          P0 = __fma_rn(a1, __fma_rn(a1, 4.5, s3), q3[j]);
-          P1 = __dmul_rn(w, __fma_rn(a1, s3, 1.0));
+      if (j >= 0 && j < N) {
+        cen[j][0] = nxt[j][0]; cen[j][1] = nxt[j][1]; cen[j][2] = nxt[j][2]; cen[j][3] = nxt[j][3];
+        nxt[j][0] = p3[1]; nxt[j][1] = u3[1]; nxt[j][2] = v3[1]; nxt[j][3] = w3[1];
+      }
+      const RowSums<double> row = row_sums(p3, u3, v3, w3);
+      if (j >= 1) {
+        const int r = j - 1;
+        const RowSide<double> below = row_side<1>(row);
+        double A[3], X[3], Y[3];
+        A[0] = fma2(4.0, mid.R0, add2(above.R0, below.R0));
+        A[1] = fma2(4.0, mid.Rz, add2(above.Rz, below.Rz));
+        A[2] = fma2(4.0, mid.Rw, add2(above.Rw, below.Rw));
+        X[0] = fma2(4.0, mid.D0, add2(above.D0, below.D0));
+        X[1] = fma2(4.0, mid.Dz, add2(above.Dz, below.Dz));
+        X[2] = fma2(4.0, mid.Dw, add2(above.Dw, below.Dw));
+        Y[0] = sub2(below.R0, above.R0);
+        Y[1] = sub2(below.Rz, above.Rz);
+        Y[2] = sub2(below.Rw, above.Rw);
+        if (sp < 0 || sp >= g.L) {       // seam plane (CTA-uniform): the jump times the non-wall weight sums (x36)
+          const double off = sp < 0 ? k.pin : -k.pin;
+          A[0] = fma2(off, fma2(-1.0 / 6.0, ws0[r], 36.0), A[0]);
+          X[0] = fma2(off, wsx[r] * (-1.0 / 6.0), X[0]);
+          Y[0] = fma2(off, wsy[r] * (-1.0 / 6.0), Y[0]);
         }
-        P[j][0] = P0; P[j][1] = P1; P[j][2] = w23[j];
-      }
+        double s[3], d[3];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const double Rq = __fma_rn(4.0, P[1][q], __dadd_rn(P[0][q], P[2][q]));
-        const double Dq = __dsub_rn(P[2][q], P[0][q]);
-        if (cy == -1) { A[q] = Rq; X[q] = Dq; Y[q] = Rq; }
-        else if (cy == 0) { A[q] = __fma_rn(4.0, Rq, A[q]); X[q] = __fma_rn(4.0, Dq, X[q]); }
-        else { A[q] = __dadd_rn(A[q], Rq); X[q] = __dadd_rn(X[q], Dq); Y[q] = __dsub_rn(Rq, Y[q]); }
-      }
-    }
-    if (sp < 0 || sp >= g.L) {         // seam plane (CTA-uniform): the pressure jump's share
-      const double off = sp < 0 ? k.pin : -k.pin;
-      A[0] = __fma_rn(off, n0, A[0]);
-      X[0] = __fma_rn(off, nx, X[0]);
-      Y[0] = __fma_rn(off, ny, Y[0]);
-    }
-    // true sums are A0/36, dir A1/12, A2/8; shares e + h (next), (2/3) A0 (self), e - h (previous)
-    const double eA = __fma_rn(A[2], 1.0 / 48.0, __dmul_rn(A[0], 1.0 / 216.0));
-    const double eX = __fma_rn(X[2], 1.0 / 48.0, __dmul_rn(X[0], 1.0 / 216.0));
-    const double eY = __fma_rn(Y[2], 1.0 / 48.0, __dmul_rn(Y[0], 1.0 / 216.0));
-    const double sA = __fma_rn(A[1], h6, eA), dA = __fma_rn(A[1], -h6, eA);
-    const double sX = __fma_rn(X[1], h6, eX), dX = __fma_rn(X[1], -h6, eX);
-    const double sY = __fma_rn(Y[1], h6, eY), dY = __fma_rn(Y[1], -h6, eY);
-    comp0 = __fma_rn(s1[0], 1.0 / 54.0, __dadd_rn(b2[0], sA));
-    comp1 = __fma_rn(s1[1], 1.0 / 54.0, __dadd_rn(b2[1], sX));
-    comp2 = __fma_rn(s1[2], 1.0 / 54.0, __dadd_rn(b2[2], sY));
-    comp3 = __dadd_rn(b2[3], sA);
+        for (int i = 0; i < 3; ++i) {
+          const double(&m)[3] = i == 0 ? A : (i == 1 ? X : Y);
+          const double e = fma2(m[2], 4.5, m[0]);
+          s[i] = fma2(m[1], dir3, e);
+          d[i] = fma2(-m[1], dir3, e);
+        }
+        // a cell adds its two neighbour planes' shares first, then its own plane's
 #pragma unroll
-    for (int q = 0; q < 4; ++q) b2[q] = b1[q];
-    b1[0] = dA; b1[1] = dX; b1[2] = dY; b1[3] = -dA;
-    s1[0] = A[0]; s1[1] = X[0]; s1[2] = Y[0];
+        for (int i = 0; i < 3; ++i) comp[r][i] = fma2(s1[r][i], 4.0, add2(d2[r][i], s[i]));
+        comp[r][3] = sub2(s[0], d2[r][0]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          d2[r][i] = d1[r][i];
+          d1[r][i] = d[i];
+          s1[r][i] = i == 0 ? A[0] : (i == 1 ? X[0] : Y[0]);
+        }
+      }
+      if (j >= 0) above = here;
+      mid = row;
+      here = row_side<-1>(row);
+    }
   };
 
-  // corrector and update of output march plane jo; history slot ROT holds plane jo-4 and is then
-  // overwritten with plane jo
-  auto output = [&](int jo, auto rot_c) {
-    constexpr int ROT = decltype(rot_c)::value;
+  // corrector and update of output march plane jo of parity PAR
+  auto output = [&](int jo, auto par_c) {
+    constexpr int PAR = decltype(par_c)::value;
     const double* so = ring + slot_of(jo) * SLOT;
-    const double* sa1 = ring + slot_of(jo + D1) * SLOT;   // march planes ahead
-    const double* sa2 = ring + slot_of(jo + 2 * D1) * SLOT;
-    const double pc = so[po];
-    const double uc = so[uo], vc = so[uo + UPL], wc = so[uo + 2 * UPL];
-    auto update = [&](int f, double c, double zb1, double zb2, double mom, double tm, double tf) {
-      const double* q = so + uo + f * UPL;
-      const double za1 = sa1[uo + f * UPL], za2 = sa2[uo + f * UPL];
-      const double t1 = __dadd_rn(__dadd_rn(__dadd_rn(q[-D1], q[D1]), __dadd_rn(q[-D1 * SW], q[D1 * SW])),
-                                  __dadd_rn(zb1, za1));
-      const double t2 = __dadd_rn(__dadd_rn(__dadd_rn(q[-2 * D1], q[2 * D1]),
-                                            __dadd_rn(q[-2 * D1 * SW], q[2 * D1 * SW])),
-                                  __dadd_rn(zb2, za2));
-      return __fma_rn(kK1, t1, __fma_rn(kK2, t2, __fma_rn(kK0, c, __fma_rn(tm, mom, tf))));
-    };
-    constexpr int H2 = (ROT + 2) & 3;                         // plane jo-2
-    const double rho = __dadd_rn(__fma_rn(pc, ws0, comp0), -gauge);
-    const double us = __fma_rn(pc, wsx, comp1), vs = __fma_rn(pc, wsy, comp2);
-    const double un = update(0, uc, hu[H2], hu[ROT], us, k.tb, __dmul_rn(k.tb, k.fx));
-    const double vn = update(1, vc, hv[H2], hv[ROT], vs, k.tb, __dmul_rn(k.tb, k.fy));
-    const double wn = update(2, wc, hw[H2], hw[ROT], comp3, ktz, __dmul_rn(k.tb, k.fz));
-    hu[ROT] = uc; hv[ROT] = vc; hw[ROT] = wc;
-    if (inside) {   // wall columns get zero (fl = 0)
-      outp[0] = rho * fl;
-      outp[FS] = un * fl;
-      outp[2 * FS] = vn * fl;
-      outp[3 * FS] = wn * fl;
+    const double* sa1 = ring + slot_of(jo + D1) * SLOT + uo;   // march planes ahead
+    const double* sa2 = ring + slot_of(jo + 2 * D1) * SLOT + uo;
+    double pc[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+      pc[r] = cen[r][0];
+      if (inside[r]) outp[r * g.lxp] = fma2(fma2(pc[r], ws0[r], comp[r][0]), 1.0 / 216.0, -gauge) * fl[r];   // walls get zero
+    }
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      const double* b = so + uo + f * UPL;
+#pragma unroll
+      for (int r = 0; r < N; ++r) {
+        const double* q = b + r * SW;
+        const double c = cen[r][1 + f];
+        const double za1 = sa1[f * UPL + r * SW], za2 = sa2[f * UPL + r * SW];
+        const double t1 = add2(add2(add2(q[-D1], q[D1]), add2(q[-D1 * SW], q[D1 * SW])), add2(h[f][PAR][1][r], za1));
+        const double t2 = add2(add2(add2(q[-2 * D1], q[2 * D1]), add2(q[-2 * D1 * SW], q[2 * D1 * SW])),
+                               add2(h[f][PAR][0][r], za2));
+        const double mom = f == 2 ? comp[r][3] : fma2(pc[r], f == 0 ? wsx[r] : wsy[r], comp[r][1 + f]);
+        // the small terms first: only the last operation rounds at the size of u
+        double un = fma2(f == 2 ? ktz : ktb, mom, __dmul_rn(k.tb, f == 0 ? k.fx : (f == 1 ? k.fy : k.fz)));
+        un = fma2(kK1, t1, fma2(kK2, t2, un));
+        un = fma2(kK0, c, un);
+        h[f][PAR][0][r] = h[f][PAR][1][r];
+        h[f][PAR][1][r] = c;
+        if (inside[r]) outp[(1 + f) * FS + r * g.lxp] = un * fl[r];
+      }
     }
     outp += ostep;
   };
 
   using I0 = std::integral_constant<int, 0>;
   using I1 = std::integral_constant<int, 1>;
-  using I2 = std::integral_constant<int, 2>;
-  using I3 = std::integral_constant<int, 3>;
-  // ---- prologue (R = 4): planes 0..3 arrive; 4..5 enter the history; 6..7 also start the
-  // predictor sums of the first output
-#pragma unroll
+  // ---- prologue (R = 4): planes 0..3 enter the history when plane 4..7 arrive; planes 6..7 also
+  // start the predictor sums of the first output
+#pragma unroll 1
   for (int m = 0; m < 2 * R; ++m) {
     if (!arrive_wait(m)) return false;
     if (m >= 2 * R - 2) predictor(m - R + 1);
     if (m >= R) {
-      const double* so = ring + slot_of(m - R) * SLOT;
-      const double uc = so[uo], vc = so[uo + UPL], wc = so[uo + 2 * UPL];
-      const int h = (m - R) & 3;
-      if (h == 0) { hu[0] = uc; hv[0] = vc; hw[0] = wc; }
-      else if (h == 1) { hu[1] = uc; hv[1] = vc; hw[1] = wc; }
-      else if (h == 2) { hu[2] = uc; hv[2] = vc; hw[2] = wc; }
-      else { hu[3] = uc; hv[3] = vc; hw[3] = wc; }
+      const double* so = ring + slot_of(m - R) * SLOT + uo;
+#pragma unroll
+      for (int f = 0; f < 3; ++f)
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+          h[f][0][0][r] = h[f][0][1][r];
+          h[f][0][1][r] = h[f][1][0][r];
+          h[f][1][0][r] = h[f][1][1][r];
+          h[f][1][1][r] = so[f * UPL + r * SW];
+        }
     }
     release_produce(m);
   }
-  // ---- steady state, four planes per pass (the history period)
-  for (int m = 2 * R; m < niter; m += 4) {
+  // in march order the planes are now [0][0], [0][1], [1][0], [1][1]: swap the middle two
+#pragma unroll
+  for (int f = 0; f < 3; ++f)
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+      const double t = h[f][0][1][r];
+      h[f][0][1][r] = h[f][1][0][r];
+      h[f][1][0][r] = t;
+    }
+  // ---- steady state, two planes per pass (the history's parity)
+#pragma unroll 1
+  for (int m = 2 * R; m < niter; m += 2) {
     if (!arrive_wait(m)) return false;
     predictor(m - R + 1);
     output(m - R, I0{});
@@ -316,16 +335,6 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
     predictor(m - R + 2);
     output(m - R + 1, I1{});
     release_produce(m + 1);
-    if (m + 2 >= niter) break;
-    if (!arrive_wait(m + 2)) return false;
-    predictor(m - R + 3);
-    output(m - R + 2, I2{});
-    release_produce(m + 2);
-    if (m + 3 >= niter) break;
-    if (!arrive_wait(m + 3)) return false;
-    predictor(m - R + 4);
-    output(m - R + 3, I3{});
-    release_produce(m + 3);
   }
   return true;
 }
