@@ -14,7 +14,7 @@
 //  - grid = tiles x streamwise chunks in chunk-major order, odd chunks marching downwards, and a
 //    cell's predictor adds its two neighbour planes' shares before its own plane's, so results do
 //    not depend on the chunking.
-// The shared-memory path bounds it (64 % of its wavefront slots; FP64 pipe 45 %). Two rows per
+// The shared-memory path (60 % of its wavefront slots) and the FP64 pipe (54 %) bound it. Two rows per
 // thread share the predictor's rows: 54 shared loads per cell against 70 with one row and 512
 // threads, 166 against 177 us a step at 512 x 128 x 128; the predictor's arithmetic per cell stays
 // the same and 8 warps instead of 16 are enough (64 x 32 x 32: 6.8 us either way). Measured and not
