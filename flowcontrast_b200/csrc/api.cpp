@@ -1612,6 +1612,8 @@ static std::string class_key(const fslbm_solve* s) {
   return buf;
 }
 
+// Default: items of 256 planes fill the pipeline half as often as 128 (64 pipes, 32 steps: 13.50 against
+// 13.83 ms); 16 x 4 warps skip more wall than 32 x 2 and, unlike 8 x 8, read shared memory without conflicts.
 struct Tiling { int chunk = 256, shape = 1; double ms = 0; };
 using TilingTable = std::map<std::string, Tiling>;
 
