@@ -408,7 +408,8 @@ struct Split {
 // resident per SM: each wave of CTAs costs a launch and pipeline fill and then a time per march
 // iteration, measured on B200 (circular pipes from 32 x 24 x 24 to 512 x 128 x 128, every split).
 // FP32 and FP16 storage march two planes per iteration, two iterations before the first output;
-// FP64 one plane, and its eight planes of fill cost as much as 4.3 output planes. An SM's time per
+// FP64 one plane, with eight planes of fill: 32 x 8 tiles fill faster than their share (64 x 32 x 32
+// 6.7 us on 32 x 16 tiles against 7.0, 32 x 24 x 24 6.3 against 5.6). An SM's time per
 // iteration grows with its resident rows of cells:
 // 1.35 us for one 32 x 8 tile of FP32 against 2.7 us for a 32 x 32 tile, so few cells per SM want
 // small tiles (latency) and many cells the large one (fewer halo cells, more warps).
@@ -417,7 +418,7 @@ static double split_us(int dtype, int K, int ty, int per_sm, int sms, int L, int
   static const double f16[3][3] = {{1.93, 2.37, 3.2}, {2.45, 4.05, 0}, {3.94, 0, 0}};
   const int planes = (L + nch - 1) / nch;
   const int64_t ctas = int64_t(ntiles) * nch, waves = (ctas + int64_t(sms) * per_sm - 1) / (int64_t(sms) * per_sm);
-  if (dtype == FSLBM_F64) return double(waves) * 1.28 * (planes + 4.3);
+  if (dtype == FSLBM_F64) return double(waves) * (ty == 8 ? 5.2 + 0.8 * planes : 5.0 + 1.225 * planes);
   const double tau = (dtype == FSLBM_F16 ? f16 : f32)[ty == 8 ? 0 : (ty == 16 ? 1 : 2)][per_sm - 1];
   return double(waves) * (2.0 + tau * ((planes + 1) / 2 + K));
 }
@@ -445,7 +446,7 @@ static Split choose_split(const fslbm_solve* s, int only_ty) {
 
 // Selects the step kernel for the current dtype and d1, uploads its tile list, builds its
 // tensor maps and sizes its grid. FSLBM_STEP_KERNEL=1 forces the one-column kernel and
-// FSLBM_TILE_Y=8|16|32 picks the pair kernel's tile height (for comparisons).
+// FSLBM_TILE_Y=8|16|32 picks the tile height of the others where they have it (for comparisons).
 static int configure_kernel(fslbm_solve* s) {
   const char* ek = std::getenv("FSLBM_STEP_KERNEL");
   const char* et = std::getenv("FSLBM_TILE_Y");
@@ -454,9 +455,10 @@ static int configure_kernel(fslbm_solve* s) {
   // FP16 storage exists only in the pair kernel
   s->use2 = step2_supported(s->dtype, s->prm.d1, s->K, s->planes > 1) &&
             (s->dtype == FSLBM_F16 || !(ek && std::atoi(ek) == 1));
-  const int ety = et && s->dtype != FSLBM_F64 ? std::atoi(et) : 0;
+  int ety = et ? std::atoi(et) : 0, box[5];
+  if (!step2_box(s->dtype, s->K, ety, box, box + 1, box + 2, box + 3, box + 4)) ety = 0;   // the kernel has no such tile
   Split split;
-  if (s->use2) split = choose_split(s, ety == 8 || ety == 16 || ety == 32 ? ety : 0);
+  if (s->use2) split = choose_split(s, ety);
   else split.tiles = fluid_tiles(s, kTY);
   const std::vector<int2>& tiles = split.tiles;
   s->ty2 = split.ty;

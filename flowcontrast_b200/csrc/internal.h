@@ -61,7 +61,7 @@ cudaError_t step_prepare(int dtype, int d1, int K);   // sets the dynamic shared
 cudaError_t launch_step(const StepLaunch& a, cudaStream_t st);
 
 // Pair kernel (d1 = 2; FP32 with 2 or 3 corrector taps, one cross-section or one per plane; FP16
-// storage with 2 taps) and FP64 column kernel (d1 = 2, 2 taps, 32 x 16 tiles): two tensor maps per
+// storage with 2 taps) and FP64 column kernel (d1 = 2, 2 taps, 32 x 16 or 32 x 8 tiles): two tensor maps per
 // input state (p box with a one-cell halo, u,v,w box with the corrector halo).
 struct Step2Launch {
   int ty;                    // tile height (8, 16 or 32)

@@ -158,13 +158,20 @@ template <class F> static cudaError_t with_step2(int dtype, int K, bool mp, int 
   return cudaErrorInvalidValue;
 }
 
+// Calls fn.template operator()<TY>() for the FP64 column kernel with tile height ty.
+template <class F> static cudaError_t with_col(int ty, F&& fn) {
+  if (ty == 16) return fn.template operator()<16>();
+  if (ty == 8) return fn.template operator()<8>();
+  return cudaErrorInvalidValue;
+}
+
 bool step2_box(int dtype, int K, int ty, int* sw, int* ph, int* uh, int* hx, int* hy) {
-  if (dtype == FSLBM_F64) {          // the FP64 column kernel: 32 x 16 tiles only
-    using Tl = ColTile<2, 16>;
-    if (ty != 16) return false;
-    *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
-    return true;
-  }
+  if (dtype == FSLBM_F64)
+    return with_col(ty, [&]<int TY>() {
+             using Tl = ColTile<2, TY>;
+             *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
+             return cudaSuccess;
+           }) == cudaSuccess;
   return with_step2(dtype, K, false, ty, [&]<int TY, class TE, int KK, bool MP, int ROWS>() {
            using Tl = Step2Tile<TY, TE, KK, ROWS>;
            *sw = Tl::SW; *ph = Tl::PH; *uh = Tl::UH; *hx = Tl::HX; *hy = Tl::HY;
@@ -192,9 +199,10 @@ int step2_rows(int dtype, int K, bool mp, int ty) {
 
 cudaError_t step2_prepare(int dtype, int K, bool mp, int ty) {
   if (dtype == FSLBM_F64)
-    return ty != 16 ? cudaErrorInvalidValue
-                    : cudaFuncSetAttribute(fslbm_col_kernel<2, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           int(ColTile<2, 16>::SMEM_BYTES));
+    return with_col(ty, [&]<int TY>() {
+      return cudaFuncSetAttribute(fslbm_col_kernel<2, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(ColTile<2, TY>::SMEM_BYTES));
+    });
   return with_step2(dtype, K, mp, ty, [&]<int TY, class TE, int KK, bool MP, int ROWS>() {
     return cudaFuncSetAttribute(fslbm_step2_kernel<TY, TE, KK, MP, ROWS>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -217,12 +225,13 @@ cudaError_t launch_step2(const StepLaunch& a, const Step2Launch& b, cudaStream_t
   k.fx = float(a.fx); k.fy = float(a.fy); k.fz = float(a.fz);
   if (a.d1 != 2) return cudaErrorInvalidValue;
   if (a.dtype == FSLBM_F64) {
-    if (b.ty != 16) return cudaErrorInvalidValue;
     StepConst<double> kd{};
     kd.tb = a.tb; kd.cc = a.cc; kd.pin = a.pin; kd.dtddy = a.dtddy; kd.m = a.m;
     kd.c0 = a.c0; kd.c1 = a.c1; kd.c2 = a.c2; kd.fx = a.fx; kd.fy = a.fy; kd.fz = a.fz;
-    return launch_chained(fslbm_col_kernel<2, 16>, b.grid, ColTile<2, 16>::THREADS,
-                          ColTile<2, 16>::SMEM_BYTES, st, *b.map_p, *b.map_uvw, g, kd);
+    return with_col(b.ty, [&]<int TY>() {
+      return launch_chained(fslbm_col_kernel<2, TY>, b.grid, ColTile<2, TY>::THREADS, ColTile<2, TY>::SMEM_BYTES, st,
+                            *b.map_p, *b.map_uvw, g, kd);
+    });
   }
   return with_step2(a.dtype, a.K, a.mask_planes > 1, b.ty, [&]<int TY, class TE, int KK, bool MP, int ROWS>() {
     using Tl = Step2Tile<TY, TE, KK, ROWS>;

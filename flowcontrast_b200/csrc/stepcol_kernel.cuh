@@ -1,7 +1,7 @@
 // FSLBM time step, FP64 column kernel for sm_100a (d1 = 2, the reference's order 2<->4 corrector).
 //
 // Planes marched one at a time, two FP64 rows of one column per thread:
-//  - a 32 x 16 tile per CTA, 256 threads, two tile rows per warp: a warp's 64-bit shared loads
+//  - a 32 x 16 tile per CTA (32 x 8 for the smallest pipes), two tile rows per warp: a warp's 64-bit shared loads
 //    read 32 consecutive doubles (two wavefronts, no bank conflict);
 //  - p is staged with a one-cell halo and u,v,w with the corrector's 2*d1 halo, as two TMA boxes
 //    per plane (no multicast) into a window of 7 planes (201 KB);

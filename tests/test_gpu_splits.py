@@ -44,9 +44,13 @@ def test_tile_heights_match_oracle_and_each_other(built, ctx, monkeypatch, L, lx
         if dtype == built.F32:
             _, eu, eps = errors(outs[0], ref, m2)
             assert eu <= 1e-5 and eps <= 1e-5, (eu, eps)
-    monkeypatch.delenv("FSLBM_TILE_Y")
-    got, _ = run_gpu(built, ctx, dom, prm, built.F64, f, steps, monitor_every=3)
-    _, eu, eps = errors(got, ref, m2)
+    outs = []
+    for ty in ("0", "8", "16"):
+        monkeypatch.setenv("FSLBM_TILE_Y", ty)
+        outs.append(run_gpu(built, ctx, dom, prm, built.F64, f, steps, monitor_every=3)[0])
+    for o in outs[1:]:
+        assert np.array_equal(outs[0], o)
+    _, eu, eps = errors(outs[0], ref, m2)
     assert eu <= 1e-12 and eps <= 1e-12, (eu, eps)
 
 
