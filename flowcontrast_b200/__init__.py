@@ -143,6 +143,7 @@ def lib():
             "fslbm_ctx_create": ([_i, ctypes.POINTER(_vp)], _i),
             "fslbm_ctx_destroy": ([_vp], _i),
             "fslbm_selftest_waits": ([_vp, ctypes.c_double, ctypes.POINTER(ctypes.c_uint)], _i),
+            "fslbm_selftest_warp_wait": ([_vp, ctypes.c_double, ctypes.POINTER(ctypes.c_uint)], _i),
             "fslbm_solve_create": ([_vp, ctypes.POINTER(Domain), ctypes.POINTER(Params), _i,
                                     ctypes.POINTER(_vp)], _i),
             "fslbm_solve_destroy": ([_vp], _i),
@@ -322,6 +323,13 @@ class Context:
         bits = ctypes.c_uint(0)
         rc = lib().fslbm_selftest_waits(self.handle, float(limit_ms), ctypes.byref(bits))
         return rc, bits.value
+
+    def selftest_warp_wait(self, limit_ms=160.0):
+        """Lanes of a warp that see a phase which completes between their limits, each by itself
+        and with the warp's one verdict (fslbm_selftest_warp_wait)."""
+        lanes = (ctypes.c_uint * 2)()
+        _check(lib().fslbm_selftest_warp_wait(self.handle, float(limit_ms), lanes))
+        return lanes[0], lanes[1]
 
     def __enter__(self):
         return self

@@ -152,6 +152,22 @@ extern "C" int fslbm_selftest_waits(fslbm_ctx* c, double limit_ms, unsigned* gav
   return FSLBM_OK;
 }
 
+// Self-test of the warp-wide wait (no reference counterpart): lanes[0] = the lanes that saw a phase
+// which completes between their limits, lanes[1] = the same with the warp's one verdict.
+extern "C" int fslbm_selftest_warp_wait(fslbm_ctx* c, double limit_ms, unsigned* lanes) {
+  if (!c || !lanes || !(limit_ms > 0.0) || limit_ms > 1000.0)
+    return fslbm_set_error(FSLBM_ERR_ARG, "selftest_warp_wait: bad argument");
+  CUDA_TRY(cudaSetDevice(c->device));
+  unsigned* d = nullptr;
+  CUDA_TRY(ctx_alloc(c, reinterpret_cast<void**>(&d), 2 * sizeof(unsigned)));
+  cudaError_t e = launch_warp_wait_selftest(static_cast<unsigned long long>(limit_ms * 1e6), d, c->stream);
+  if (!e) e = cudaMemcpyAsync(lanes, d, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream);
+  ctx_free(c, d);
+  if (!e) e = cudaStreamSynchronize(c->stream);
+  if (e) return fslbm_set_error(FSLBM_ERR_CUDA, "selftest_warp_wait: %s", cudaGetErrorString(e));
+  return FSLBM_OK;
+}
+
 // ------------------------------------------------------------------------------------------
 // tensor-map encoding through the driver entry point (no link-time libcuda dependency)
 // ------------------------------------------------------------------------------------------

@@ -96,6 +96,9 @@ cudaError_t launch_monitor(const MonitorLaunch& a, cudaStream_t st);
 // counter wait gave up, bit 1 = the mbarrier wait gave up.
 cudaError_t launch_wait_selftest(const unsigned* counter, unsigned long long limit_ns, unsigned* err,
                                  cudaStream_t st);
+// Warp-wide wait whose phase completes between the limits of its lanes: the lanes that saw it, lane
+// by lane (out[0]) and as a warp (out[1]).
+cudaError_t launch_warp_wait_selftest(unsigned long long limit_ns, unsigned* out, cudaStream_t st);
 
 // ---- batched ensemble (pair kernel, d1 = 2, tile height 16 or 32 for the whole batch)
 struct BatchMon {

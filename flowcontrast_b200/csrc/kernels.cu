@@ -1013,6 +1013,41 @@ __global__ void wait_selftest_kernel(const unsigned* counter, unsigned long long
   mbar_inval(&bar);
 }
 
+// Warp 0 waits on a phase that warp 1 completes between the limits of its even and its odd lanes,
+// once lane by lane and once as a warp: out[0], out[1] = the lanes that saw it.
+__global__ void warp_wait_selftest_kernel(unsigned long long limit_ns, unsigned* out) {
+  __shared__ __align__(8) uint64_t bar[2];
+  const int lane = threadIdx.x & 31;
+  const uint64_t limit = lane & 1 ? limit_ns : limit_ns / 16;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_init_fence();
+  }
+  for (int i = 0; i < 2; ++i) {
+    __syncthreads();
+    if (threadIdx.x >= 32) {
+      if (lane == 0) {
+        const uint64_t t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < limit_ns / 4) __nanosleep(1000);
+        mbar_arrive_expect_tx(&bar[i], 0u);      // no bytes expected: completes the phase
+      }
+    } else {
+      const bool ok = i == 0 ? mbar_wait_bounded(&bar[0], 0u, limit) : mbar_wait_warp(&bar[1], 0u, limit);
+      __syncwarp();
+      const unsigned seen = __ballot_sync(0xffffffffu, ok);
+      if (lane == 0) out[i] = seen;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) mbar_inval(&bar[threadIdx.x]);
+}
+
+cudaError_t launch_warp_wait_selftest(unsigned long long limit_ns, unsigned* out, cudaStream_t st) {
+  warp_wait_selftest_kernel<<<1, 64, 0, st>>>(limit_ns, out);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_wait_selftest(const unsigned* counter, unsigned long long limit_ns, unsigned* err,
                                  cudaStream_t st) {
   wait_selftest_kernel<<<1, 32, 0, st>>>(counter, limit_ns, err);

@@ -58,6 +58,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
+// The same for a whole warp (converged on entry), with one verdict: false in every lane when the
+// limit passed in any. Lanes poll the barrier and the clock apart, so around the limit some would
+// see the phase and others give up, and the warp-wide instructions that follow (.aligned
+// tensor-memory accesses, __syncwarp) need them all. The vote also reconverges the warp for those.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, limit_ns));
+}
+
 // Generic-proxy shared-memory accesses before this point are ordered before later async-proxy
 // (TMA) accesses of the same thread.
 __device__ __forceinline__ void fence_proxy_async_smem() {

@@ -378,17 +378,17 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
     }
   __syncthreads();
 
-  // Wait for stage j; false after flagging a failure (the caller returns). Then any warp may have
-  // issued loads up to SU stages ahead: let them land (bounded).
+  // Wait for stage j, one verdict per warp; false after flagging a failure (the whole warp
+  // returns). Then any warp may have issued loads up to SU stages ahead: let them land (bounded).
   auto arrive_wait = [&](int j) -> bool {
-    auto wait = [&](int q, uint64_t limit) {
-      return mbar_wait_bounded(&full[unsigned(q) % unsigned(SU)], (unsigned(q) / unsigned(SU)) & 1u, limit);
-    };
-    if (wait(j, kWaitLimitNs)) return true;
+    auto bar_of = [&](int q) { return &full[unsigned(q) % unsigned(SU)]; };
+    auto parity = [](int q) { return (unsigned(q) / unsigned(SU)) & 1u; };
+    if (mbar_wait_warp(bar_of(j), parity(j), kWaitLimitNs)) return true;
     if (lane == 0) {
       atomicOr(g.err, 1u);
-      for (int q = j + 1; q < nstage && q <= j + SU; ++q) wait(q, kWaitLimitNs / 8);
+      for (int q = j + 1; q < nstage && q <= j + SU; ++q) mbar_wait_bounded(bar_of(q), parity(q), kWaitLimitNs / 8);
     }
+    __syncwarp();
     return false;
   };
   // Pair j leaves the window (u,v,w after it was the output pair, p of pair j + 1 after the
@@ -491,6 +491,7 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
     if (!arrive_wait(q + K - 1)) {
       tm_wait_stores();
       if (lane == 0) bulk_wait_all();
+      __syncwarp();
       return false;
     }
     const TE* sp0 = pring + unsigned(q) % unsigned(SP) * (2 * PPL) + po;

@@ -128,15 +128,16 @@ __device__ __forceinline__ bool col_march(const CUtensorMap* tmap_p, const CUten
 
   grid_dependency_wait();
   __syncthreads();
-  auto drain = [&](int from) {         // failure path: let this CTA's loads land (bounded)
-    if (lane == 0)
-      for (int q = from; q < niter && q < from + S; ++q)
-        mbar_wait_bounded(&full[slot_of(q)], phase_of(q), kWaitLimitNs / 8);
-  };
+  // wait for march plane m, one verdict per warp; false after flagging a failure and letting this
+  // CTA's loads land (bounded)
   auto arrive_wait = [&](int m) -> bool {
-    if (mbar_wait_bounded(&full[slot_of(m)], phase_of(m), kWaitLimitNs)) return true;
-    if (lane == 0) atomicOr(g.err, 1u);
-    drain(m + 1);
+    if (mbar_wait_warp(&full[slot_of(m)], phase_of(m), kWaitLimitNs)) return true;
+    if (lane == 0) {
+      atomicOr(g.err, 1u);
+      for (int q = m + 1; q < niter && q < m + 1 + S; ++q)
+        mbar_wait_bounded(&full[slot_of(q)], phase_of(q), kWaitLimitNs / 8);
+    }
+    __syncwarp();
     return false;
   };
   // planes p - 1 and p (p = m - R odd) leave the window; see step2_march for the ordering

@@ -127,6 +127,11 @@ int fslbm_ctx_destroy(fslbm_ctx* ctx);
    per wait (3 = both) and the call returns FSLBM_ERR_TIMEOUT, the code a kernel's gave-up wait
    produces. The context stays usable. */
 int fslbm_selftest_waits(fslbm_ctx* ctx, double limit_ms, unsigned* gave_up);
+/* Self-test of the warp-wide form of the mbarrier wait: the phase completes after the limit of a
+   warp's even lanes (limit_ms / 16) and before that of its odd ones (limit_ms, at most 1000).
+   lanes[0] gets the lanes that saw it, each by itself; lanes[1] the same with the wait's one
+   verdict for the warp (0 or all). */
+int fslbm_selftest_warp_wait(fslbm_ctx* ctx, double limit_ms, unsigned lanes[2]);
 
 /* ---- solve (replaces main's set-up and time loop, FSLBM.cu:489-905) ---- */
 int fslbm_solve_create(fslbm_ctx* ctx, const fslbm_domain* dom, const fslbm_params* prm,
