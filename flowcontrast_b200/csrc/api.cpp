@@ -214,8 +214,10 @@ struct fslbm_solve {
   void* state[2] = {nullptr, nullptr};
   int cur = 0;
   uint8_t* d_mask = nullptr;
+  // wall sums the step kernel reads: per column, or with masks per plane one of two tables per cell
+  // (load_cell_table), in one buffer that holds either
   void* d_colcoef = nullptr;
-  uint32_t* d_near = nullptr;      // masks per plane, FP32: packed wall sums per cell, then per column (step2_march)
+  enum class CellTable { none, coefs, packed } cell_table = CellTable::none;
   int2* d_tiles = nullptr;
   int ntiles = 0, chunk = 0, nchunks = 0;
   CUtensorMap maps[2];
@@ -412,6 +414,7 @@ static void tile_warp_counts(const fslbm_solve* s, const std::vector<int2>& tile
 }
 
 static void choose_chunks(fslbm_solve* s);
+static int load_cell_table(fslbm_solve* s);
 
 // How a solve's step is split over the SMs: tile height and streamwise chunks.
 struct Split {
@@ -471,6 +474,8 @@ static int configure_kernel(fslbm_solve* s) {
   // FP16 storage exists only in the pair kernel
   s->use2 = step2_supported(s->dtype, s->prm.d1, s->K, s->planes > 1) &&
             (s->dtype == FSLBM_F16 || !(ek && std::atoi(ek) == 1));
+  if (s->planes > 1)
+    if (int r = load_cell_table(s)) return r;
   int ety = et ? std::atoi(et) : 0, box[5];
   if (!step2_box(s->dtype, s->K, ety, box, box + 1, box + 2, box + 3, box + 4)) ety = 0;   // the kernel has no such tile
   Split split;
@@ -593,6 +598,34 @@ static std::vector<CellCoef<TC>> cell_coefs(const fslbm_solve* s, const std::vec
   return cc;
 }
 
+// Device bytes of the table below: the larger of the two, so a change of parameters that moves the
+// solve to the other kernel needs no memory.
+static size_t cell_table_bytes(size_t plane, size_t L, bool f64) {
+  return plane * L * (f64 ? sizeof(CellCoef<double>) : sizeof(CellCoef<float>));
+}
+
+// Masks per plane: the wall sums that the configured step kernel reads, built and uploaded when the
+// kernel changes (192 x 96 x 96 cells, FP32: 7 MB of packed words instead of 28 MB of coefficients).
+// Pair kernel: pack_wall_sums words per cell, then per column. One-column kernel: CellCoef.
+static int load_cell_table(fslbm_solve* s) {
+  using Table = fslbm_solve::CellTable;
+  const Table want = s->use2 ? Table::packed : Table::coefs;
+  if (s->cell_table == want) return FSLBM_OK;
+  const std::vector<uint32_t> near = packed_cell_sums(s);
+  auto upload = [&](const auto& table) {           // pageable: staged before the copy returns
+    return cudaMemcpyAsync(s->d_colcoef, table.data(), table.size() * sizeof(table[0]), cudaMemcpyHostToDevice,
+                           s->ctx->stream);
+  };
+  s->cell_table = Table::none;
+  cudaError_t e = want == Table::packed        ? upload(near)
+                  : s->dtype == FSLBM_F64      ? upload(cell_coefs<double>(s, near))
+                                               : upload(cell_coefs<float>(s, near));
+  if (!e) e = cudaStreamSynchronize(s->ctx->stream);
+  CUDA_TRY(e);
+  s->cell_table = want;
+  return FSLBM_OK;
+}
+
 // Picks the streamwise chunking: minimises waves * (chunk + 2R) over chunk counts.
 static void choose_chunks(fslbm_solve* s) {
   int occ = 1;
@@ -619,7 +652,7 @@ static void choose_chunks(fslbm_solve* s) {
 static void free_solve(fslbm_solve* s) {
   if (!s) return;
   cudaSetDevice(s->ctx->device);
-  void* ptrs[] = {s->state[0], s->state[1], s->d_mask, s->d_colcoef, s->d_near, s->d_tiles, s->d_ghosts, s->d_counters,
+  void* ptrs[] = {s->state[0], s->state[1], s->d_mask, s->d_colcoef, s->d_tiles, s->d_ghosts, s->d_counters,
                   s->d_log, s->d_gauge, s->d_err, s->d_scratch, s->d_stats, s->d_prof,
                   s->d_stage, s->d_plane, s->d_wbase, s->d_wgt};
   for (void* p : ptrs) ctx_free(s->ctx, p);
@@ -784,19 +817,8 @@ extern "C" int fslbm_solve_create(fslbm_ctx* ctx, const fslbm_domain* dom, const
     free_solve(s);
     return r;
   }
-  if (s->planes > 1 && dtype == FSLBM_F64) {
-    auto cc = cell_coefs<double>(s, packed_cell_sums(s));
-    if ((e = dalloc(s, &s->d_colcoef, cc.size() * sizeof(cc[0])))) return fail("colcoef");
-    e = cudaMemcpyAsync(s->d_colcoef, cc.data(), cc.size() * sizeof(cc[0]), cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaStreamSynchronize(st);       // the table is a local vector
-  } else if (s->planes > 1) {
-    const std::vector<uint32_t> near = packed_cell_sums(s);
-    auto cc = cell_coefs<float>(s, near);
-    if ((e = dalloc(s, &s->d_colcoef, cc.size() * sizeof(cc[0])))) return fail("colcoef");
-    e = cudaMemcpyAsync(s->d_colcoef, cc.data(), cc.size() * sizeof(cc[0]), cudaMemcpyHostToDevice, st);
-    if (!e) e = dalloc(s, &s->d_near, near.size() * sizeof(near[0]));
-    if (!e) e = cudaMemcpyAsync(s->d_near, near.data(), near.size() * sizeof(near[0]), cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaStreamSynchronize(st);
+  if (s->planes > 1) {                           // filled by configure_kernel
+    e = dalloc(s, &s->d_colcoef, cell_table_bytes(plane, size_t(s->L), dtype == FSLBM_F64));
   } else if (dtype == FSLBM_F64) {
     auto cc = column_coefs<double>(s);
     if ((e = dalloc(s, &s->d_colcoef, cc.size() * sizeof(cc[0])))) return fail("colcoef");
@@ -979,8 +1001,7 @@ extern "C" int fslbm_solve_footprint(const fslbm_domain* dom, fslbm_dtype dtype,
   const int64_t cc = dtype == FSLBM_F64 ? int64_t(sizeof(ColCoef<double>)) : int64_t(sizeof(ColCoef<float>));
   const int64_t tiles = ((lxp + kTX - 1) / kTX) * ((dom->ly + kTY - 1) / kTY) * int64_t(sizeof(int2));
   const int64_t masks = dom->mask_planes > 1
-                            ? 4 * cs + cs * dom->lz * (1 + int64_t(dtype == FSLBM_F64 ? sizeof(CellCoef<double>)
-                                                                                : sizeof(CellCoef<float>) + 4))
+                            ? cs * dom->lz + int64_t(cell_table_bytes(size_t(cs), size_t(dom->lz), dtype == FSLBM_F64))
                             : cs + cs * cc;
   const int64_t wtabs = dtype == FSLBM_F16 ? 2 * cs * int64_t(sizeof(float)) : 0;
   *bytes = 2 * 4 * fs * es + masks + tiles + wtabs + int64_t(sizeof(DevCounters)) +
@@ -1052,7 +1073,8 @@ static int enqueue_steps(fslbm_solve* s, int64_t nsteps) {
   a.ntiles = s->ntiles; a.chunk = s->chunk; a.nchunks = s->nchunks;
   a.tiles = s->d_tiles; a.mask = s->d_mask; a.colcoef = s->d_colcoef;
   a.err = s->d_err; a.counters = s->d_counters; a.mask_planes = s->planes;
-  a.wb = s->d_wbase; a.wgt = s->d_wgt; a.near = s->d_near;
+  a.wb = s->d_wbase; a.wgt = s->d_wgt;
+  a.near = s->cell_table == fslbm_solve::CellTable::packed ? static_cast<const uint32_t*>(s->d_colcoef) : nullptr;
   fill_constants(s, a);
   MonitorLaunch m{};
   m.dtype = s->dtype; m.mask = s->d_mask;
