@@ -483,9 +483,10 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   // iteration q: predictor of pair q, which completes the sums of pair q - 1, and from q = K + 1 on
   // corrector and update of the output pair q - 1
   // Two iterations per pass rename the carried registers instead of moving them (FP32, two rows
-  // per thread, one cross-section: -3 %); the other forms would spill or outgrow the instruction
-  // cache (four rows: 4718 against 4415 us per 50 steps at 512 x 128 x 128).
-  constexpr int kPass = !MP && !kBase && N == 2 ? 2 : 1;
+  // per thread, one cross-section, tiles of 16 or 8 rows: -3 %); the other forms would spill (the
+  // batched kernel's 32 x 32 tile: 14.55 against 13.21 ms per 32 steps of 64 pipes) or outgrow the
+  // instruction cache (four rows: 4718 against 4415 us per 50 steps at 512 x 128 x 128).
+  constexpr int kPass = !MP && !kBase && N == 2 && TY < 32 ? 2 : 1;
 #pragma unroll kPass
   for (int q = K - 1; q <= nstage - K; ++q) {
     if (!arrive_wait(q + K - 1)) {
