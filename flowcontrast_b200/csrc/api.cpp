@@ -1360,18 +1360,46 @@ extern "C" int fslbm_stats_sample(fslbm_solve* s) {
   return FSLBM_OK;
 }
 
+// Device buffer of n values for a read-out combined on the device. Null, without an error, when the
+// device's memory is used up: the accumulators are then copied and combined on the host, which
+// needs none (and takes longer: 1.02 ms instead of 0.17 for the plane statistics of 256 x 96 x 96).
+static cudaError_t readout_buffer(fslbm_solve* s, size_t n, double** p) {
+  *p = nullptr;
+  const cudaError_t e = ctx_alloc(s->ctx, reinterpret_cast<void**>(p), n * sizeof(double));
+  if (e != cudaErrorMemoryAllocation) return e;
+  (void)cudaGetLastError();                         // not left for a later launch check
+  *p = nullptr;
+  return cudaSuccess;
+}
+
+// Copies n accumulators from device memory into acc and waits for them.
+static cudaError_t readout_host(fslbm_solve* s, const double* src, std::vector<double>& acc, size_t n) {
+  acc.resize(n);
+  const cudaError_t e = cudaMemcpyAsync(acc.data(), src, n * sizeof(double), cudaMemcpyDeviceToHost, s->ctx->stream);
+  return e ? e : cudaStreamSynchronize(s->ctx->stream);
+}
+
 extern "C" int fslbm_stats_get(fslbm_solve* s, double* out, int* cnt, int* cnt2) {
   if (!s || !out) return fslbm_set_error(FSLBM_ERR_ARG, "stats_get: null argument");
   CUDA_TRY(cudaSetDevice(s->ctx->device));
   if (int r = ensure_stats(s)) return r;
   const size_t n = size_t(s->ly) * (s->L + 2 * s->d2);
   double* val = nullptr;                            // compensated sums / counts
-  CUDA_TRY(ctx_alloc(s->ctx, reinterpret_cast<void**>(&val), 11 * n * sizeof(double)));
-  cudaError_t e = launch_stats_value(s->d_stats, n, s->cnt, s->cnt2, val, s->ctx->stream);
-  if (!e) e = cudaMemcpyAsync(out, val, 11 * n * sizeof(double), cudaMemcpyDeviceToHost, s->ctx->stream);
-  ctx_free(s->ctx, val);
-  CUDA_TRY(e);
-  CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
+  CUDA_TRY(readout_buffer(s, 11 * n, &val));
+  if (val) {
+    cudaError_t e = launch_stats_value(s->d_stats, n, s->cnt, s->cnt2, val, s->ctx->stream);
+    if (!e) e = cudaMemcpyAsync(out, val, 11 * n * sizeof(double), cudaMemcpyDeviceToHost, s->ctx->stream);
+    ctx_free(s->ctx, val);
+    CUDA_TRY(e);
+    CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
+  } else {
+    std::vector<double> acc;
+    CUDA_TRY(readout_host(s, s->d_stats, acc, 22 * n));
+    for (size_t k = 0; k < 11 * n; ++k) {
+      const int c = k < 4 * n ? s->cnt : s->cnt2;
+      out[k] = c ? (acc[k] + acc[11 * n + k]) / double(c) : 0.0;
+    }
+  }
   if (cnt) *cnt = s->cnt;
   if (cnt2) *cnt2 = s->cnt2;
   return FSLBM_OK;
@@ -1412,12 +1440,22 @@ extern "C" int fslbm_profile_get(fslbm_solve* s, double* sums, int64_t* nsamples
   const size_t n = size_t(s->lx) * s->ly;
   if (s->d_prof) {
     double* val = nullptr;                          // compensated sums, dense rows
-    CUDA_TRY(ctx_alloc(s->ctx, reinterpret_cast<void**>(&val), 10 * n * sizeof(double)));
-    cudaError_t e = launch_profile_value(s->d_prof, s->lx, s->lxp, s->ly, val, s->ctx->stream);
-    if (!e) e = cudaMemcpyAsync(sums, val, 10 * n * sizeof(double), cudaMemcpyDeviceToHost, s->ctx->stream);
-    ctx_free(s->ctx, val);
-    CUDA_TRY(e);
-    CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
+    CUDA_TRY(readout_buffer(s, 10 * n, &val));
+    if (val) {
+      cudaError_t e = launch_profile_value(s->d_prof, s->lx, s->lxp, s->ly, val, s->ctx->stream);
+      if (!e) e = cudaMemcpyAsync(sums, val, 10 * n * sizeof(double), cudaMemcpyDeviceToHost, s->ctx->stream);
+      ctx_free(s->ctx, val);
+      CUDA_TRY(e);
+      CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
+    } else {
+      const size_t np = size_t(s->lxp) * s->ly;
+      std::vector<double> acc;
+      CUDA_TRY(readout_host(s, s->d_prof, acc, 20 * np));
+      for (size_t i = 0; i < 10 * n; ++i) {
+        const size_t src = i / s->lx * s->lxp + i % s->lx;
+        sums[i] = acc[src] + acc[10 * np + src];
+      }
+    }
   } else {
     std::fill(sums, sums + 10 * n, 0.0);
   }
