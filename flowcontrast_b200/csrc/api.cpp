@@ -202,6 +202,7 @@ struct fslbm_solve {
   size_t es = 4;
   fslbm_params prm{};
   std::vector<uint8_t> mask;   // lxp*ly, padded columns are wall
+  std::vector<uint8_t> fluid_rows;   // find_fluid_rows
   int64_t fluid2d = 0;             // fluid cells of the (first) cross-section
   double l1 = 0;                   // the monitor's l1 (FSLBM.cu:589-591)
   int64_t fluid_total = 0;         // fluid cells of the core
@@ -366,24 +367,33 @@ static int build_tensor_maps(fslbm_solve* s) {
   return FSLBM_OK;
 }
 
+// Which rows of each 32-wide column of tiles hold fluid, in any plane: column by column. Formed once per
+// solve, because choosing a split lists the tiles of every height (a search of the whole mask for
+// each took a tenth of the time to create a 256 x 96 x 96 solve).
+static std::vector<uint8_t> find_fluid_rows(const fslbm_solve* s) {
+  std::vector<uint8_t> rows(size_t((s->lxp + kTX - 1) / kTX) * s->ly, 0);
+  for (int z = 0; z < s->planes; ++z)
+    for (int y = 0; y < s->ly; ++y)
+      for (int x0 = 0; x0 < s->lxp; x0 += kTX) {
+        uint8_t& r = rows[size_t(x0 / kTX) * s->ly + y];
+        if (!r)
+          r = std::memchr(&s->mask[(size_t(z) * s->ly + y) * s->lxp + x0], 0, std::min(kTX, s->lxp - x0)) != nullptr;
+      }
+  return rows;
+}
+
 // Tile list (tiles holding fluid) for a tile of kTX x th cells, by rows of tiles. Every 32-wide
 // column of tiles starts at its own first fluid row (TMA boxes may start at any row), which saves
 // a tile where the fluid rows fit fewer: 30 instead of 32 tiles of 32 x 16 over the 128 x 128
 // pipe, 4 % of the march over the mixed-size ensemble.
 static std::vector<int2> fluid_tiles(const fslbm_solve* s, int th) {
   std::vector<std::pair<int, int2>> tiles;            // (row of tiles, origin)
-  std::vector<uint8_t> row(s->ly);
   for (int x0 = 0; x0 < s->lxp; x0 += kTX) {
-    for (int y = 0; y < s->ly; ++y) {
-      row[y] = 0;
-      for (int z = 0; z < s->planes && !row[y]; ++z)
-        for (int x = x0; x < std::min(x0 + kTX, s->lxp); ++x)
-          if (s->mask[(size_t(z) * s->ly + y) * s->lxp + x] == 0) { row[y] = 1; break; }
-    }
+    const uint8_t* row = s->fluid_rows.data() + size_t(x0 / kTX) * s->ly;
     int y0 = 0, k = 0;
     while (y0 < s->ly && !row[y0]) ++y0;
     for (; y0 < s->ly; y0 += th, ++k)
-      if (std::any_of(row.begin() + y0, row.begin() + std::min(y0 + th, s->ly), [](uint8_t r) { return r; }))
+      if (std::any_of(row + y0, row + std::min(y0 + th, s->ly), [](uint8_t r) { return r; }))
         tiles.push_back({k, make_int2(x0, y0)});
   }
   std::stable_sort(tiles.begin(), tiles.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
@@ -451,14 +461,18 @@ static Split choose_split(const fslbm_solve* s, int only_ty) {
     int box[5];
     if ((only_ty && ty != only_ty) || !step2_box(s->dtype, s->K, ty, box, box + 1, box + 2, box + 3, box + 4))
       continue;
-    const std::vector<int2> tiles = fluid_tiles(s, ty);
+    std::vector<int2> tiles = fluid_tiles(s, ty);
     const int nt = int(tiles.size());
+    bool better = false;
     for (int per_sm = 1; per_sm <= step2_occupancy(s->dtype, s->K, ty); ++per_sm)
       for (int waves = 1; waves <= 4; ++waves) {
         const int nch = std::max(1, std::min(int(int64_t(sms) * per_sm * waves / nt), max_nch));
         const double us = split_us(s->dtype, s->K, ty, per_sm, sms, s->L, nt, nch);
-        if (us < best.us) best = Split{ty, nch, us, tiles};
+        if (us >= best.us) continue;
+        best.ty = ty; best.nch = nch; best.us = us;
+        better = true;
       }
+    if (better) best.tiles = std::move(tiles);
   }
   return best;
 }
@@ -507,23 +521,27 @@ static int configure_kernel(fslbm_solve* s) {
 // wall cells of the 3x3 cross-section neighbourhood; outside the box counts as wall.
 template <class TC>
 static std::vector<ColCoef<TC>> column_coefs(const fslbm_solve* s) {
-  std::vector<ColCoef<TC>> cc(size_t(s->lxp) * s->ly);
+  const int nx = s->lxp, ny = s->ly, px = nx + 2;
+  const uint8_t* mask = s->mask.data();
+  std::vector<uint8_t> wall(size_t(px) * (ny + 2), 1);          // with a rim of outside cells
+  for (int y = 0; y < ny; ++y)
+    for (int x = 0; x < nx; ++x) wall[size_t(y + 1) * px + x + 1] = mask[size_t(y) * nx + x] == kWall;
+  std::vector<ColCoef<TC>> cc(size_t(nx) * ny);
   const double wv[3] = {1.0 / 6.0, 2.0 / 3.0, 1.0 / 6.0};
-  for (int y = 0; y < s->ly; ++y)
-    for (int x = 0; x < s->lxp; ++x) {
+  for (int y = 0; y < ny; ++y)
+    for (int x = 0; x < nx; ++x) {
+      ColCoef<TC>& c = cc[size_t(y) * nx + x];
+      c.fluid = TC(mask[size_t(y) * nx + x] == 0 ? 1 : 0);
+      const uint8_t *r0 = &wall[size_t(y) * px + x], *r1 = r0 + px, *r2 = r1 + px;
+      if (!(r0[0] | r0[1] | r0[2] | r1[0] | r1[1] | r1[2] | r2[0] | r2[1] | r2[2])) continue;   // away from walls: zero
       double a = 0, bx = 0, by = 0;
       for (int dy = -1; dy <= 1; ++dy)
         for (int dx = -1; dx <= 1; ++dx) {
-          const int gx = x + dx, gy = y + dy;
-          const bool wall = gx < 0 || gy < 0 || gx >= s->lxp || gy >= s->ly ||
-                            s->mask[size_t(gy) * s->lxp + gx] == kWall;
-          if (!wall) continue;
+          if (!r1[dy * px + dx + 1]) continue;
           const double w = wv[dx + 1] * wv[dy + 1];
           a += w; bx += dx * w; by += dy * w;
         }
-      ColCoef<TC>& c = cc[size_t(y) * s->lxp + x];
       c.ws0 = TC(a); c.wsx = TC(bx); c.wsy = TC(by);
-      c.fluid = TC(s->mask[size_t(y) * s->lxp + x] == 0 ? 1 : 0);
     }
   return cc;
 }
@@ -771,6 +789,7 @@ extern "C" int fslbm_solve_create(fslbm_ctx* ctx, const fslbm_domain* dom, const
     free_solve(s);
     return fslbm_set_error(FSLBM_ERR_ARG, "solve_create: no fluid cells");
   }
+  s->fluid_rows = find_fluid_rows(s);
   // l1 of the monitor: the reference counts its buffer cells over 2*d2 planes (FSLBM.cu:589-591),
   // i.e. the mean fluid count of the core planes the buffers copy
   {
