@@ -441,8 +441,9 @@ def _member_start(fb, s, sp):
 
 
 def batch_kernel_name(storage):
-    """The batched kernel the library launches: 32 x 32 tiles unless FSLBM_BATCH_TILE_Y=16."""
-    ty = 16 if os.environ.get("FSLBM_BATCH_TILE_Y") == "16" else 32
+    """The batched kernel the library launches; it chooses the tile height by the members' sizes unless
+    FSLBM_BATCH_TILE_Y gives it."""
+    ty = os.environ.get("FSLBM_BATCH_TILE_Y", "16 or 32")
     te = "__half" if storage == "f16" else "float"
     return f"fslbm_step2_batch_kernel<{ty},{te}> (chained steps)"
 

@@ -318,16 +318,16 @@ static int encode_pair_maps(const fslbm_solve* s, int ty, CUtensorMap mp[2], CUt
   return FSLBM_OK;
 }
 
-// Tensor maps of the pair kernel's stores into the two state buffers: the four fields of one
+// Tensor maps of the pair kernel's stores into the two state buffers: `fields` fields of one
 // warp's cells, 32 >> shape columns and rows << shape rows.
-static int encode_store_maps(const fslbm_solve* s, int rows, int shape, CUtensorMap mo[2]) {
+static int encode_store_maps(const fslbm_solve* s, int rows, int shape, int fields, CUtensorMap mo[2]) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return fslbm_set_error(FSLBM_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
   const CUtensorMapDataType dt = s->dtype == FSLBM_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   cuuint64_t dims[4] = {cuuint64_t(s->lxp), cuuint64_t(s->ly), cuuint64_t(s->L), 4};
   cuuint64_t strides[3] = {cuuint64_t(s->lxp) * s->es, cuuint64_t(s->lxp) * s->ly * s->es,
                            cuuint64_t(field_stride(s)) * s->es};
-  cuuint32_t estr[4] = {1, 1, 1, 1}, box[4] = {cuuint32_t(32 >> shape), cuuint32_t(rows << shape), 1, 4};
+  cuuint32_t estr[4] = {1, 1, 1, 1}, box[4] = {cuuint32_t(32 >> shape), cuuint32_t(rows << shape), 1, cuuint32_t(fields)};
   for (int b = 0; b < 2; ++b) {
     const CUresult r = enc(&mo[b], dt, 4, s->state[b], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -341,7 +341,7 @@ static int encode_store_maps(const fslbm_solve* s, int rows, int shape, CUtensor
 static int build_tensor_maps(fslbm_solve* s) {
   if (s->use2) {
     if (s->dtype != FSLBM_F64)
-      if (int r = encode_store_maps(s, step2_rows(s->dtype, s->K, s->planes > 1, s->ty2), 0, s->maps2o)) return r;
+      if (int r = encode_store_maps(s, step2_rows(s->dtype, s->K, s->planes > 1, s->ty2), 0, 4, s->maps2o)) return r;
     return encode_pair_maps(s, s->ty2, s->maps2p, s->maps2u);
   }
   EncodeTiledFn enc = encode_fn();
@@ -1498,6 +1498,11 @@ extern "C" int fslbm_profile_reset(fslbm_solve* s) {
 // gauges booked there too); the launch is captured once as a CUDA graph and replayed. Members
 // of other kinds step one after another.
 // ------------------------------------------------------------------------------------------
+// Shortest streamwise chunk of a batch member, in planes, as long as every SM has an item.
+constexpr int kMinChunk = 8;
+// Planes of pipeline fill that an item marches besides its own (two pairs, and the set-up's share).
+constexpr int kFillPlanes = 5;
+
 struct fslbm_batch {
   fslbm_ctx* ctx = nullptr;
   std::vector<fslbm_solve*> members;
@@ -1514,12 +1519,10 @@ struct fslbm_batch {
   std::vector<int2> h_items;
   std::vector<int2> item_shape;    // per member: (tiles, chunks) the item table was built for
   int nitems = 0, grid = 0;
-  // the batch's own tiling of every member (32 x ty tiles, one height for the whole batch): tile
-  // list, fluid warps per tile for the three warp shapes, tensor maps of both buffers. 32 x 32
-  // tiles, one 512-thread CTA per SM: the pair kernel's window of 32 x 16 tiles (118 KB for FP32)
-  // leaves an SM one such CTA of 8 warps, which is slower on the 64-pipe ensemble (cross-sections
-  // 24..96) at every chunk and warp shape; the members' own single-pipe tiling is not affected
-  int ty = 32;
+  // the batch's own tiling of every member (32 x ty tiles, one height for the whole batch, see
+  // batch_tile_height): tile list, fluid warps per tile for the three warp shapes, tensor maps of
+  // both buffers; the members' own single-pipe tiling is not affected
+  int ty = 16;
   struct Tiling {
     int ntiles = 0;
     int2* d_tiles = nullptr;
@@ -1531,7 +1534,8 @@ struct fslbm_batch {
   // per member tiling: streamwise planes per work item and warp shape (0: 32 x 2, 1: 16 x 4,
   // 2: 8 x 8), from the tuning table by size class, else 256 (FSLBM_BATCH_CHUNK) and 16 x 4
   std::vector<int> m_chunk, m_shape;
-  int shrink = 1;                  // chunk divisor for batches with fewer than 2 items per SM
+  int shrink = 1;                  // chunk divisor for batches with few items per CTA slot
+  int min_chunk = kMinChunk;       // planes of the shortest item
   cudaGraphExec_t exec2 = nullptr;  // one chained launch of `chain` steps
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double last_ms = 0;
@@ -1568,15 +1572,31 @@ static bool batchable(const fslbm_solve* s) {
   return s->use2 && s->K == 2 && s->planes == 1 && s->dtype != FSLBM_F64 && s->nghost == 0;
 }
 
-// Resident CTAs of the batched kernel: one per SM, two for 32 x 16 tiles of FP16 storage.
-static int batch_slots(const fslbm_batch* b) {
-  return b->ctx->sm_count * step2_occupancy(b->members[0]->dtype, 2, b->ty);
+// Tile height of a batch: 16 unless 32 x 32 tiles march less. Both forms run 16 warps per SM, one CTA of
+// 32 x 32 or two of 32 x 16; a 32 x 16 tile has more halo rows per row of its own but leaves less of
+// itself outside a cross-section that ends in it. Per pair of planes two FP32 32 x 16 tiles
+// take 1.03 to 1.05 of the time of one 32 x 32 tile, two of FP16 storage the same time (measured
+// on batches of 40 and 150 equal pipes). FP32, us a step, 32 x 32 / 32 x 16: 150 pipes of
+// 64 x 44 x 44 348 / 294, of 64 x 96 x 96 922 / 956, the 64-pipe ensemble 413 / 413.
+static int batch_tile_height(fslbm_solve* const* solves, int n) {
+  int64_t planes16 = 0, planes32 = 0;      // planes marched, summed over the tiles
+  for (int i = 0; i < n; ++i) {
+    planes16 += int64_t(fluid_tiles(solves[i], 16).size()) * solves[i]->L;
+    planes32 += int64_t(fluid_tiles(solves[i], 32).size()) * solves[i]->L;
+  }
+  const double ratio = solves[0]->dtype == FSLBM_F32 ? 1.03 : 1.0;
+  return ratio * double(planes16) <= 2.0 * double(planes32) ? 16 : 32;
 }
 
-// Streamwise chunks of a member: about `chunk` planes each, at least 4*d1 planes.
-static int member_chunks(const fslbm_solve* s, int chunk) {
-  int nch = (s->L + chunk - 1) / chunk;
-  return std::max(1, std::min(nch, std::max(1, s->L / (4 * s->prm.d1))));
+// Resident CTAs of the batched kernel: one per SM of 32 x 32 tiles, two of 32 x 16 tiles.
+static int batch_slots(const fslbm_batch* b) { return b->ctx->sm_count * batch_occupancy(b->members[0]->dtype, b->ty); }
+
+// Streamwise chunks of member i in the batch's present split: about m_chunk / shrink planes each, at
+// least min_chunk.
+static int member_chunks(const fslbm_batch* b, int i) {
+  const int L = b->members[i]->L, least = b->min_chunk;
+  const int chunk = least < kMinChunk ? least : std::max(least, b->m_chunk[i] / b->shrink);
+  return std::max(1, std::min((L + chunk - 1) / chunk, L / least));
 }
 
 // Member descriptors for the members' current buffers, step counts and stops, and the work-item
@@ -1597,11 +1617,10 @@ static int batch_upload(fslbm_batch* b) {
       return fslbm_set_error(FSLBM_ERR_STATE, "batch_step: member %d was reconfigured and no longer "
                              "fits the batched kernel; create a new batch", i);
   }
-  auto eff_chunk = [&](int i) { return std::max(4 * b->members[i]->prm.d1, b->m_chunk[i] / b->shrink); };
   if (!b->h_items.empty() && b->item_shape.size() == size_t(n))
     for (int i = 0; i < n; ++i)
       if (b->item_shape[i].x != b->mt[i].ntiles ||
-          b->item_shape[i].y != member_chunks(b->members[i], eff_chunk(i))) {
+          b->item_shape[i].y != member_chunks(b, i)) {
         b->h_items.clear();
         break;
       }
@@ -1609,20 +1628,40 @@ static int batch_upload(fslbm_batch* b) {
   struct Item { int64_t cost; int2 it; };
   std::vector<Item> items;
   if (build_items) {
-    // shorter chunks while there are fewer than two items per SM (few or small members)
-    auto count = [&]() {
-      int64_t c = 0;
-      for (int i = 0; i < n; ++i) c += int64_t(b->mt[i].ntiles) * member_chunks(b->members[i], eff_chunk(i));
-      return c;
+    // Shorter chunks while the longest item is more than 3/4 of a CTA slot's share of the work (few or
+    // small members): the tail of a step costs more than the chunks' pipeline fill (from 0.65 to
+    // 0.85 the choice hardly changes; the 64-pipe ensemble at 0.92 440 us a step, halved 412; FP16
+    // storage, 64 pipes, 0.84 602, halved 555). Where chunks of 8 planes leave SMs without any, chunks
+    // of a pair of planes at the least: what bounds a step then is its longest item (FP32, us a step
+    // with 8 planes and now: 64 x 48 x 48 alone 19.2 and 16.3, 33 x 33 x 33 alone 27.3 and 18.7, 16
+    // pipes of 32 x 24 x 24 22.2 and 17.6).
+    struct Load { int64_t items = 0, planes = 0, longest = 0; };
+    auto load = [&]() {                // planes marched, those of the fill included
+      Load w;
+      for (int i = 0; i < n; ++i) {
+        const int nch = member_chunks(b, i), planes = (b->members[i]->L + nch - 1) / nch + kFillPlanes;
+        w.items += int64_t(b->mt[i].ntiles) * nch;
+        w.planes += int64_t(b->mt[i].ntiles) * nch * planes;
+        w.longest = std::max<int64_t>(w.longest, planes);
+      }
+      return w;
     };
+    const int64_t slots = batch_slots(b);
     b->shrink = 1;
-    while (b->shrink < 64 && count() < 2 * batch_slots(b)) b->shrink *= 2;
+    b->min_chunk = kMinChunk;
+    for (Load w = load(); b->shrink < 64 && 4 * w.longest * slots > 3 * w.planes; w = load()) b->shrink *= 2;
+    while (b->min_chunk > 2) {
+      b->min_chunk /= 2;
+      if (load().items <= slots) continue;
+      b->min_chunk *= 2;
+      break;
+    }
   }
   for (int i = 0; i < n; ++i) {
     fslbm_solve* s = b->members[i];
     fslbm_batch::Tiling& tl = b->mt[i];
     if (tl.mo_shape != b->m_shape[i]) {
-      if (int r = encode_store_maps(s, 2, b->m_shape[i], tl.mo)) return r;
+      if (int r = encode_store_maps(s, 2, b->m_shape[i], batch_staged_fields(b->ty, s->es), tl.mo)) return r;
       tl.mo_shape = b->m_shape[i];
     }
     StepLaunch a{};
@@ -1632,7 +1671,7 @@ static int batch_upload(fslbm_batch* b) {
     a.err = b->d_tickets + 2;        // one flag for the whole batch
     a.wb = s->d_wbase; a.wgt = s->d_wgt;
     fill_constants(s, a);
-    const int nch = member_chunks(s, eff_chunk(i));
+    const int nch = member_chunks(b, i);
     const long long stop_at = b->stop[i] >= 0 ? (long long)b->stop[i] : LLONG_MAX;
     CUDA_TRY(fill_batch_member(b->h_members.data() + mbytes * i, tl.mp, tl.mu, tl.mo, a,
                                s->state[0], s->state[1], s->d_gauge, &s->d_counters->steps,
@@ -1709,8 +1748,8 @@ static std::string class_key(const fslbm_solve* s) {
   return buf;
 }
 
-// Default: items of 256 planes fill the pipeline half as often as 128 (64 pipes, 32 steps: 13.50 against
-// 13.83 ms); 16 x 4 warps skip more wall than 32 x 2 and, unlike 8 x 8, read shared memory without conflicts.
+// Default: items of 256 planes fill the pipeline half as often as 128; batches that they leave with a
+// long tail are split further (batch_upload). 16 x 4 warps skip more wall than 32 x 2 and, unlike 8 x 8, read shared memory without conflicts.
 struct Tiling { int chunk = 256, shape = 1; double ms = 0; };
 using TilingTable = std::map<std::string, Tiling>;
 
@@ -1805,6 +1844,7 @@ extern "C" int fslbm_batch_create(fslbm_ctx* ctx, fslbm_solve* const* solves, in
   cudaError_t e = cudaSetDevice(ctx->device);
   // tile height of the batch's tiles (FSLBM_BATCH_TILE_Y=16|32 overrides the default)
   if (const char* ety = std::getenv("FSLBM_BATCH_TILE_Y")) b->ty = std::atoi(ety) == 16 ? 16 : 32;
+  else if (fast) b->ty = batch_tile_height(solves, n);
   if (!e && fast) e = batch_prepare(solves[0]->dtype, b->ty);
   if (!e && fast) {
     b->mt.resize(n);

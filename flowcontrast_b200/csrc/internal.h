@@ -108,6 +108,11 @@ struct BatchMon {
   int monitor_every;
   int cur0;
 };
+// Fields of a warp's cells that the batched kernel stages for one store (the store maps' box): two with
+// FP32 32 x 16 tiles, so that two CTAs fit an SM (150 pipes of 64 x 44 x 44: 435 us a step with one CTA
+// of 8 warps, 295 with two), else all four.
+constexpr int batch_staged_fields(int ty, size_t element) { return ty == 16 && element == 4 ? 2 : 4; }
+int batch_occupancy(int dtype, int ty);   // CTAs per SM
 cudaError_t batch_prepare(int dtype, int ty);
 size_t batch_member_bytes();
 // Writes one member descriptor (layout private to the kernels) into host memory at dst.

@@ -454,12 +454,13 @@ __device__ __forceinline__ bool batch_item_begin(const BatchMember& mb, int memb
 // Two rows per thread: with four (the single-pipe kernel's form) a warp of the 16 x 4 shape holds 16 x 8
 // cells, whose rows four apart share banks, and skips wall at a coarser grain (64 pipes, 32 steps:
 // 13.62 ms with the best shape against 13.15).
+template <int TY, class TE> using BatchTile = Step2Tile<TY, TE, 2, 2, batch_staged_fields(TY, sizeof(TE))>;
 template <int TY, class TE>
-__global__ void __launch_bounds__(Step2Tile<TY, TE>::THREADS, Step2Tile<TY, TE>::CTAS)
+__global__ void __launch_bounds__(BatchTile<TY, TE>::THREADS, BatchTile<TY, TE>::CTAS)
     fslbm_step2_batch_kernel(const BatchMember* __restrict__ members,
                              const BatchMon* __restrict__ mons, const int2* __restrict__ items,
                              int nitems, int nsteps, unsigned* sync, unsigned* err) {
-  using Tl = Step2Tile<TY, TE>;
+  using Tl = BatchTile<TY, TE>;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ unsigned s_ticket;
   __shared__ long long s_done;
@@ -513,7 +514,7 @@ __global__ void __launch_bounds__(Step2Tile<TY, TE>::THREADS, Step2Tile<TY, TE>:
     if (s_done < mb.stop_at) {
       const int cur = mb.cur0 ^ (step & 1);
       const int ntiles = mb.g.ntiles;
-      ok = step2_march<TY, TE>(&mb.map_p[cur], &mb.map_u[cur], &mb.map_o[1 - cur], tmem, s_g, s_k,
+      ok = step2_march<TY, TE, 2, false, 2, Tl::STAGED>(&mb.map_p[cur], &mb.map_u[cur], &mb.map_o[1 - cur], tmem, s_g, s_k,
                                it.y % ntiles, it.y / ntiles, smem, !first, mb.shape, false);
       first = false;
     }
@@ -527,8 +528,17 @@ cudaError_t batch_prepare(int dtype, int ty) {
     if constexpr (TY == 8 || K != 2 || MP) return cudaErrorInvalidValue;
     else
       return cudaFuncSetAttribute(fslbm_step2_batch_kernel<TY, TE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(Step2Tile<TY, TE>::SMEM_BYTES));
+                                  int(BatchTile<TY, TE>::SMEM_BYTES));
   });
+}
+
+int batch_occupancy(int dtype, int ty) {
+  int n = 1;
+  (void)with_step2(dtype, 2, false, ty, [&]<int TY, class TE, int K, bool MP, int ROWS>() {
+    n = BatchTile<TY, TE>::CTAS;
+    return cudaSuccess;
+  });
+  return n;
 }
 
 size_t batch_member_bytes() { return sizeof(BatchMember); }
@@ -569,7 +579,7 @@ cudaError_t launch_batch_steps(int dtype, int ty, const void* members, const Bat
     if constexpr (TY == 8 || K != 2 || MP) {
       return cudaErrorInvalidValue;
     } else {
-      using Tl = Step2Tile<TY, TE>;
+      using Tl = BatchTile<TY, TE>;
       fslbm_step2_batch_kernel<TY, TE><<<grid, Tl::THREADS, Tl::SMEM_BYTES, st>>>(mb, mons, items, nitems, nsteps,
                                                                                  sync, err);
       return cudaGetLastError();

@@ -52,10 +52,11 @@ namespace fslbm {
 // TE is the storage type of the state (float, or __half for FP16 storage); arithmetic is FP32
 // either way. Halo widths and paddings keep every TMA box start and destination on 16 bytes.
 // K is the number of corrector taps per direction (2: the reference's order 2<->4 blend, 3: its
-// order 4<->6 blend).
-template <int TY, class TE = float, int K = 2, int ROWS = 2> struct Step2Tile {
+// order 4<->6 blend), SF the fields staged for a store at a time (4, or 2).
+template <int TY, class TE = float, int K = 2, int ROWS = 2, int SF = 4> struct Step2Tile {
   static constexpr int D1 = 2;                          // corrective stride
   static constexpr int N = ROWS;                        // rows per thread
+  static constexpr int STAGED = SF;                     // fields staged at a time
   static constexpr int ES = int(sizeof(TE));
   static constexpr int A16 = 16 / ES;                   // elements per 16 bytes
   static constexpr int TX = 32;
@@ -76,7 +77,7 @@ template <int TY, class TE = float, int K = 2, int ROWS = 2> struct Step2Tile {
   static constexpr uint32_t U_BYTES = uint32_t(3 * UPL * ES), P_BYTES = uint32_t(SW * PH * ES);
   static constexpr size_t P_OFFSET = size_t(SU) * 2 * VPL * ES;
   // staging of a warp's output pair: [plane][field][row][column] of the warp's cells
-  static constexpr int STG = 2 * 4 * N * 32;
+  static constexpr int STG = 2 * SF * N * 32;
   static constexpr size_t STG_OFFSET = P_OFFSET + size_t(SP) * 2 * PPL * ES;
   static constexpr size_t BAR_OFFSET = STG_OFFSET + size_t(WARPS) * STG * ES;   // a "full" mbarrier per slot
   static constexpr size_t REL_OFFSET = BAR_OFFSET + SU * sizeof(uint64_t);       // release counters, tensor memory base
@@ -92,13 +93,15 @@ template <int TY, class TE = float, int K = 2, int ROWS = 2> struct Step2Tile {
   static constexpr int TM_SLOT = 6 * N, TM_WARP = TM_RING * TM_SLOT;
   static constexpr int TM_NEED = TM_WARP * ((WARPS + 3) / 4);
   static constexpr int TM_COLS = TM_NEED <= 32 ? 32 : TM_NEED <= 64 ? 64 : TM_NEED <= 128 ? 128 : 256;
-  // CTAs per SM (shared memory; 128 registers a thread at 16 warps per SM)
-  static constexpr int CTAS = K > 2 || TY == 32 ? 1 : TY == 16 ? (ES == 2 ? 2 : 1) : 3;
+  // CTAs per SM (shared memory; 128 registers a thread at 16 warps per SM). FP32 32 x 16: 120 KB with
+  // four fields staged, 112 KB with two, which leaves room for a second CTA.
+  static constexpr int CTAS = K > 2 || TY == 32 ? 1 : TY == 16 ? (ES == 2 || SF == 2 ? 2 : 1) : 3;
   static_assert(TM_NEED <= TM_COLS && TM_COLS * CTAS <= 512, "tensor memory columns");
   static_assert((PPL * ES) % 128 == 0 && (VPL * ES) % 128 == 0 && (STG * ES) % 128 == 0,
                 "TMA addresses must stay aligned");
   static_assert((HX * ES) % 16 == 0, "TMA box x start must be 16-byte aligned");
   static_assert(SMEM_BYTES <= 227 * 1024, "window exceeds a CTA's shared memory");
+  static_assert(SF == 4 || SF == 2, "fields staged at a time");
   static_assert(TY % 8 == 0, "warp shapes within a 32-wide tile");
 };
 
@@ -270,12 +273,13 @@ template <int COLS> __device__ __forceinline__ void tm_free(uint32_t base) {
 // cross-sections. With the 160-byte FP32 row stride the shapes 0 and 1 read shared memory without
 // bank conflicts (rows 2 apart are 16 banks apart), shape 2 two-way. The map changes no thread's
 // arithmetic.
-template <int TY, class TE, int K = 2, bool MP = false, int ROWS = 2>
+// tmap_out's box holds SF fields of the warp's cells.
+template <int TY, class TE, int K = 2, bool MP = false, int ROWS = 2, int SF = 4>
 __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUtensorMap* tmap_uvw,
                                             const CUtensorMap* tmap_out, uint32_t tmem, const Step2Geom& g,
                                             const StepConst<float>& k, int tile, int chunk,
                                             unsigned char* smem, bool reinit, int shape, bool chained) {
-  using Tl = Step2Tile<TY, TE, K, ROWS>;
+  using Tl = Step2Tile<TY, TE, K, ROWS, SF>;
   constexpr int N = Tl::N, R = Tl::R, D1 = Tl::D1, HX = Tl::HX, HY = Tl::HY, SW = Tl::SW, SU = Tl::SU, SP = Tl::SP;
   constexpr int PPL = Tl::PPL, UPL = Tl::UPL, VPL = Tl::VPL;
   TE* uring = reinterpret_cast<TE*>(smem);
@@ -486,7 +490,7 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
   // per thread, one cross-section, tiles of 16 or 8 rows: -3 %); the other forms would spill (the
   // batched kernel's 32 x 32 tile: 14.55 against 13.21 ms per 32 steps of 64 pipes) or outgrow the
   // instruction cache (four rows: 4718 against 4415 us per 50 steps at 512 x 128 x 128).
-  constexpr int kPass = !MP && !kBase && N == 2 && TY < 32 ? 2 : 1;
+  constexpr int kPass = !MP && !kBase && N == 2 && TY < 32 && SF == 4 ? 2 : 1;
 #pragma unroll kPass
   for (int q = K - 1; q <= nstage - K; ++q) {
     if (!arrive_wait(q + K - 1)) {
@@ -674,7 +678,7 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
       __syncwarp();
       auto put = [&](int f, int r, float2 val) {
         val = mul2(val, f2(fluid[r]));                           // walls get zero
-        TE* o = sto + f * N * 32 + r * wcols;
+        TE* o = sto + f % SF * N * 32 + r * wcols;
         if constexpr (kBase) {
           // two cells share a hash word: the even column's lane forms the first plane's, the odd
           // column's the second plane's
@@ -684,10 +688,19 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
           const uint32_t mine = hash32(((cell << 2) | uint32_t(f)) ^ seed);
           const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
           o[0] = sr_half(val.x, odd ? other >> 16 : mine);
-          o[4 * N * 32] = sr_half(val.y, odd ? mine >> 16 : other);
+          o[SF * N * 32] = sr_half(val.y, odd ? mine >> 16 : other);
         } else {
           o[0] = val.x;
-          o[4 * N * 32] = val.y;
+          o[SF * N * 32] = val.y;
+        }
+      };
+      auto flush = [&](int f0) {                                 // fields f0 .. f0 + SF - 1 leave the staging
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_4d(tmap_out, stg, org.x + wx, org.y + wy, zo, f0);
+          if (second) tma_store_4d(tmap_out, stg + SF * N * 32, org.x + wx, org.y + wy, zo + dir, f0);
+          bulk_commit();
         }
       };
 #pragma unroll
@@ -696,7 +709,7 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
       // own columns of pairs q, q - 1, ...: with kAhead the next field's arrive while a field is
       // computed (-1 % on the FP32 32 x 32 tile, -2 % with FP16 storage; in the FP32 batched
       // kernel the registers spill, +5 %)
-      constexpr bool kAhead = N == 4 || kBase || TY < 32;
+      constexpr bool kAhead = N == 4 || kBase || (TY < 32 && SF == 4);
       float2 rings[kAhead ? 2 : 1][K + 2][N];
       auto load_ring = [&](int f) {
 #pragma unroll
@@ -737,16 +750,15 @@ __device__ __forceinline__ bool step2_march(const CUtensorMap* tmap_p, const CUt
 #pragma unroll
           for (int j = K - 1; j >= 0; --j) un = fma2(f2(kKt[j]), taps[j], un);
           un = fma2(f2(kK0), ring[1][r], un);
+          if (SF == 2 && f == 1 && r == 0) {                     // p and u have left the staging
+            if (lane == 0) bulk_wait_read();
+            __syncwarp();
+          }
           put(1 + f, r, un);
         }
+        if (SF == 2 && f == 0) flush(0);
       }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        tma_store_4d(tmap_out, stg, org.x + wx, org.y + wy, zo, 0);
-        if (second) tma_store_4d(tmap_out, stg + 4 * N * 32, org.x + wx, org.y + wy, zo + dir, 0);
-        bulk_commit();
-      }
+      flush(4 - SF);
     }
 #pragma unroll
     for (int r = 0; r < N; ++r) {

@@ -234,9 +234,10 @@ int fslbm_batch_set_stop(fslbm_batch* b, int member, int64_t stop_step);
  * the smaller shapes suit small cross-sections. Members fall in size classes (32-wide tiles
  * across x and y, length rounded up to a power of two); a batch takes its classes' tiling from
  * the table named by the FSLBM_BATCH_TUNING environment variable, else from batch_tiling.json
- * next to the library, else 256 planes and 16 x 4 warps. The batch marches its own 32 x 32
- * tiles (FSLBM_BATCH_TILE_Y=16 selects 32 x 16 tiles), independent of the tiling each member uses
- * when stepped alone. */
+ * next to the library, else 256 planes and 16 x 4 warps; batches with few
+ * or small members use shorter chunks. The batch marches its own 32 x 16 or 32 x 32 tiles, whichever
+ * its members fill better (FSLBM_BATCH_TILE_Y=16|32 overrides), independent of the tiling each member
+ * uses when stepped alone. */
 int fslbm_batch_set_tiling(fslbm_batch* b, int member, int chunk, int warp_shape);
 int fslbm_batch_load_tiling(fslbm_batch* b, const char* path);
 /* Autotuner: times each size class's candidate tilings (chunks 16..256, the three warp shapes) on the
