@@ -1674,7 +1674,7 @@ static int batch_upload(fslbm_batch* b) {
     const int nch = member_chunks(b, i);
     const long long stop_at = b->stop[i] >= 0 ? (long long)b->stop[i] : LLONG_MAX;
     CUDA_TRY(fill_batch_member(b->h_members.data() + mbytes * i, tl.mp, tl.mu, tl.mo, a,
-                               s->state[0], s->state[1], s->d_gauge, &s->d_counters->steps,
+                               s->d_gauge, &s->d_counters->steps,
                                stop_at, s->prm.monitor_every, s->cur, nch, b->m_shape[i]));
     if (build_items) {
       if (i == 0) b->item_shape.assign(n, make_int2(0, 0));

@@ -117,8 +117,7 @@ cudaError_t batch_prepare(int dtype, int ty);
 size_t batch_member_bytes();
 // Writes one member descriptor (layout private to the kernels) into host memory at dst.
 cudaError_t fill_batch_member(void* dst, const CUtensorMap* map_p, const CUtensorMap* map_u, const CUtensorMap* map_o,
-                              const StepLaunch& a, void* state0, void* state1,
-                              const double* gauge_slot, const long long* steps, long long stop_at,
+                              const StepLaunch& a, const double* gauge_slot, const long long* steps, long long stop_at,
                               int monitor_every, int cur0, int nchunks, int shape);
 // Advances every member `nsteps` steps (fewer for members that reach their stop) in one
 // persistent launch, preceded by a reset of the launch's counters. items: nitems (member, item

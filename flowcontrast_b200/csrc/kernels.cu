@@ -375,9 +375,8 @@ __global__ void monitor_kernel(MonitorLaunch a) {
 // and constants, and where its step count stops.
 struct alignas(64) BatchMember {
   CUtensorMap map_p[2], map_u[2], map_o[2];
-  Step2Geom g;                 // g.out is replaced by the buffer the step writes
+  Step2Geom g;                 // step_no and gauge are set per item
   StepConst<float> k;
-  void* state[2];
   const double* gauge_slot;    // the member's monitor p2, applied on the step after a monitor
   const long long* steps;      // the member's device step counter
   long long stop_at;           // the member is not stepped once its counter reaches this
@@ -420,14 +419,13 @@ __device__ __forceinline__ bool batch_item_begin(const BatchMember& mb, int memb
     atomicOr(err, 1u);
     return false;
   }
-  // the member's previous step was written by other CTAs through the generic proxy; this
-  // thread's TMA loads of it follow
+  // The member's previous step was written by other CTAs' TMA stores. Each warp waited for its own
+  // (bulk_wait_all), a barrier, the item's count and the step's release followed, and this thread
+  // acquired that release; the fence orders its TMA loads, of the async proxy, behind it.
   fence_proxy_async_global();
   const long long done = __ldcg(mb.steps);
   *s_done = done;
-  const int cur = mb.cur0 ^ (step & 1);
   Step2Geom g = mb.g;
-  g.out = mb.state[1 - cur];
   g.step_counter = nullptr;
   g.step_no = unsigned(done + 1);
   g.gauge = (mb.monitor_every > 0 && done > 0 && done % mb.monitor_every == 0) ? mb.gauge_slot : nullptr;
@@ -544,8 +542,7 @@ int batch_occupancy(int dtype, int ty) {
 size_t batch_member_bytes() { return sizeof(BatchMember); }
 
 cudaError_t fill_batch_member(void* dst, const CUtensorMap* mp, const CUtensorMap* mu, const CUtensorMap* mo,
-                              const StepLaunch& a, void* state0, void* state1,
-                              const double* gauge_slot, const long long* steps, long long stop_at,
+                              const StepLaunch& a, const double* gauge_slot, const long long* steps, long long stop_at,
                               int monitor_every, int cur0, int nchunks, int shape) {
   BatchMember m;
   std::memset(&m, 0, sizeof m);
@@ -559,7 +556,6 @@ cudaError_t fill_batch_member(void* dst, const CUtensorMap* mp, const CUtensorMa
   m.k.tb = float(a.tb); m.k.cc = float(a.cc); m.k.pin = float(a.pin); m.k.dtddy = float(a.dtddy);
   m.k.m = float(a.m); m.k.c0 = float(a.c0); m.k.c1 = float(a.c1); m.k.c2 = float(a.c2);
   m.k.fx = float(a.fx); m.k.fy = float(a.fy); m.k.fz = float(a.fz);
-  m.state[0] = state0; m.state[1] = state1;
   m.gauge_slot = gauge_slot; m.steps = steps; m.stop_at = stop_at; m.shape = shape;
   m.monitor_every = monitor_every; m.cur0 = cur0;
   std::memcpy(dst, &m, sizeof m);

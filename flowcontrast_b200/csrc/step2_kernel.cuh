@@ -111,7 +111,7 @@ struct Step2Geom {
   const int2* tiles;
   const uint8_t* mask;
   const void* colcoef;     // ColCoef<float>[lxp*ly]
-  void* out;
+  void* out;               // FP64 column kernel (the pair kernel stores through tensor maps)
   const double* gauge;
   unsigned* err;
   long long* step_counter;
