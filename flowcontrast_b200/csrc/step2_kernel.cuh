@@ -26,17 +26,19 @@
 //    chunks share are read by both at the same time;
 //  - warps whose cells are all wall keep the pipeline protocol but skip the arithmetic.
 //
-// What bounds it. FP32: with four rows per thread 8 warps of 219 registers issue on 47 % of the
-// cycles (fixed-latency dependencies), the FMA pipes are busy 46 %, DRAM 29 %; FP16 storage:
+// What bounds it. FP32: with four rows per thread 8 warps of 209 registers issue on 48 % of the
+// cycles (fixed-latency dependencies), the FMA pipes are busy 47 %, DRAM 29 %; FP16 storage:
 // instruction issue, 67 % (conversions, rounding); small pipes: the march's K fill iterations. The
 // form it replaces, two columns per thread with scalar FP32 and a register history, was bound by
-// shared-memory wavefronts (17.3 M a launch, now 11.6 M) and instructions (59.9 M, now 41.3 M).
+// shared-memory wavefronts (17.3 M a launch, now 11.6 M) and instructions (59.9 M, now 41.0 M).
 // Per step, that form against this one, one B200:
-//   512 x 128 x 128   FP32 97.2 -> 85.6 us, FP16 storage 167 -> 127 us
-//   300 x 120 x 120   FP32 61.7 -> 46.9 us
-//   151 x 61 x 61     FP32 20.9 -> 13.3 us
-// and against step_kernel.cuh, 10 steps: order 6 on 256 x 96 x 96 670 -> 366 us, a mask per plane on
-// 192 x 96 x 96 488 -> 318 us.
+//   512 x 128 x 128   FP32 97.2 -> 83.9 us, FP16 storage 167 -> 125 us
+//   300 x 120 x 120   FP32 61.7 -> 46.4 us
+//   151 x 61 x 61     FP32 20.9 -> 13.0 us
+// and against step_kernel.cuh, 10 steps: order 6 on 256 x 96 x 96 670 -> 367 us, a mask per plane on
+// 192 x 96 x 96 488 -> 300 us.
+// At 128 registers some forms spill (bytes stored a thread): 32 x 32 with masks per plane 36, FP16
+// storage on 32 x 32 and 32 x 16 tiles 8, batched FP32 40, batched FP16 16 (32 x 32) and 24 (32 x 16).
 #pragma once
 #include <cstdint>
 #include <type_traits>

@@ -16,7 +16,7 @@
 //    not depend on the chunking.
 // The shared-memory path (60 % of its wavefront slots) and the FP64 pipe (54 %) bound it. Two rows per
 // thread share the predictor's rows: 54 shared loads per cell against 70 with one row and 512
-// threads, 166 against 177 us a step at 512 x 128 x 128; the predictor's arithmetic per cell stays
+// threads, 166 against 177 us a step at 512 x 128 x 128 in 25-step passes (164 over 2000 steps); the predictor's arithmetic per cell stays
 // the same and 8 warps instead of 16 are enough (64 x 32 x 32: 6.8 us either way). Measured and not
 // used: the plane two ahead carried into the predictor (51 loads, 1 % slower), the predictor
 // instantiated apart for the seam planes (2 % slower).
