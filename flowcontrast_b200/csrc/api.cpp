@@ -83,7 +83,12 @@ static void ctx_release(fslbm_ctx* c) {
 }
 
 static cudaError_t ctx_alloc(fslbm_ctx* c, void** p, size_t bytes) {
-  return cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), c->pool, c->stream);
+  const cudaError_t e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), c->pool, c->stream);
+  if (e) {
+    (void)cudaGetLastError();                       // reported by the caller, not by a later launch check
+    *p = nullptr;
+  }
+  return e;
 }
 
 static void ctx_free(fslbm_ctx* c, void* p) {
@@ -222,6 +227,7 @@ struct fslbm_solve {
   int2* d_tiles = nullptr;
   int ntiles = 0, chunk = 0, nchunks = 0;
   CUtensorMap maps[2];
+  bool ready = false;              // tile list, wall table and maps are those of the parameters (configure_kernel)
   // pair kernel or FP64 column kernel (d1 = 2): tile height, grid, maps per buffer
   bool use2 = false;
   int ty2 = 32, grid2 = 0;
@@ -485,7 +491,9 @@ static Split choose_split(const fslbm_solve* s, int only_ty) {
 // Selects the step kernel for the current dtype and d1, uploads its tile list, builds its
 // tensor maps and sizes its grid. FSLBM_STEP_KERNEL=1 forces the one-column kernel and
 // FSLBM_TILE_Y=8|16|32 picks the tile height of the others where they have it (for comparisons).
+// Where it fails (no memory for a longer tile list) the solve is not stepped until it has succeeded.
 static int configure_kernel(fslbm_solve* s) {
+  s->ready = false;
   const char* ek = std::getenv("FSLBM_STEP_KERNEL");
   const char* et = std::getenv("FSLBM_TILE_Y");
   double cf[9];
@@ -519,7 +527,9 @@ static int configure_kernel(fslbm_solve* s) {
     CUDA_TRY(step_prepare(s->dtype, s->prm.d1, s->K));
     choose_chunks(s);
   }
-  return build_tensor_maps(s);
+  if (int r = build_tensor_maps(s)) return r;
+  s->ready = true;
+  return FSLBM_OK;
 }
 
 // Static wall sums per column (see step_kernel.cuh): sums of w(cx)w(cy) cx^a cy^b over the
@@ -915,7 +925,7 @@ extern "C" int fslbm_solve_set_params(fslbm_solve* s, const fslbm_params* prm) {
   if (rc) return rc;
   const bool d1_changed = prm->d1 != s->prm.d1 || prm->fd_order != s->prm.fd_order;
   s->prm = *prm;
-  if (d1_changed) {
+  if (d1_changed || !s->ready) {
     CUDA_TRY(cudaSetDevice(s->ctx->device));
     CUDA_TRY(cudaStreamSynchronize(s->ctx->stream));
     if (int r = configure_kernel(s)) return r;
@@ -1090,6 +1100,8 @@ static void fill_constants(const fslbm_solve* s, StepLaunch& a) {
 }
 
 static int enqueue_steps(fslbm_solve* s, int64_t nsteps) {
+  if (!s->ready)
+    return fslbm_set_error(FSLBM_ERR_STATE, "step: the last set_params failed; set the parameters again");
   cudaStream_t st = s->ctx->stream;
   StepLaunch a{};
   a.dtype = s->dtype; a.d1 = s->prm.d1;
@@ -1390,10 +1402,7 @@ extern "C" int fslbm_stats_sample(fslbm_solve* s) {
 static cudaError_t readout_buffer(fslbm_solve* s, size_t n, double** p) {
   *p = nullptr;
   const cudaError_t e = ctx_alloc(s->ctx, reinterpret_cast<void**>(p), n * sizeof(double));
-  if (e != cudaErrorMemoryAllocation) return e;
-  (void)cudaGetLastError();                         // not left for a later launch check
-  *p = nullptr;
-  return cudaSuccess;
+  return e == cudaErrorMemoryAllocation ? cudaSuccess : e;
 }
 
 // Copies n accumulators from device memory into acc and waits for them.
