@@ -138,7 +138,9 @@ int fslbm_solve_create(fslbm_ctx* ctx, const fslbm_domain* dom, const fslbm_para
                        fslbm_dtype dtype, fslbm_solve** out);
 int fslbm_solve_destroy(fslbm_solve* s);
 /* Live parameter update, as the reference's re-read of param.txt every 500 steps
- * (FSLBM.cu:669-677). d1 may change only to another supported stride. */
+ * (FSLBM.cu:669-677). d1 may change only to another supported stride. After a change of d1 or
+ * fd_order that failed on the device (no memory for its tile list), steps return FSLBM_ERR_STATE
+ * until the parameters are set again. */
 int fslbm_solve_set_params(fslbm_solve* s, const fslbm_params* prm);
 /* Host fields in, lx*ly*lz each, FP64 (host_dtype FSLBM_F64) or FP32 (FSLBM_F32). Wall cells
  * are set to zero, the invariant the reference's bcond restores every step (FSLBM.cu:290).
